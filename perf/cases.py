@@ -164,8 +164,8 @@ def _data(case, seed):
         pos = (rows + at[:, k]).reshape(-1, 1) + j
         x.view(-1).index_put_((pos[live],), (b * (amp[:, k] / rms.sqrt()).reshape(-1, 1))[live], accumulate=True)
     if case["kind"] == "stress":
-        # piecewise-constant envelope over six decades, a new level every minute or so, on a large offset
-        seg = 6000 + int(1000 * float(u[0, 0, 0]))
+        # piecewise-constant envelope over six decades, a new level every 10 to 20 minutes, on a large offset
+        seg = 60000 + int(60000 * float(u[0, 0, 0]))
         lev = 10.0 ** (6.0 * torch.rand(n // seg + 1, generator=g, dtype=torch.float64, device="cuda") - 3.0)
         x = x * lev.repeat_interleave(seg)[:n] + 1e3 * 10.0 ** (2.0 * float(u[1, 0, 0]))
     x = x.to(torch.float32 if case.get("bits", 32) == 32 else torch.float64)
