@@ -2045,20 +2045,20 @@ template <class T> static mfgpu_status mf_launch_fixup(mfgpu_mf *mf)
         f.S0 = mf->S;
     }
     const int nctas = 4 * std::max(1, mf->n_sm);
-    if (mf->fx_on && mf->nblocks > 0 && !mf->test_skip_fixup)
-    {
-        FixParams<T> g = f;
-        g.flist = mf->fxlist.as<int>(); g.fcount = mf->fxcount.as<int>();
-        g.nbmax = mf->fx_nbmax;
-        g.chan_b0 = mf->fx_cb0.as<int>(); g.chan_nb = mf->fx_cnb.as<int>();
-        g.Lmax = mf->fx_lmax;
-        CU(launch_fixup<T>(g, nctas, fixup_warps<T>(g.Lmax, mf->dev_smem), mf->stream));
-        ++mf->launches;
-    }
+    if constexpr (sizeof(T) == 4)
+        if (mf->fx_on && mf->nblocks > 0 && !mf->test_skip_fixup)
+        {
+            FixParams<float> g = f;
+            g.flist = mf->fxlist.as<int>(); g.fcount = mf->fxcount.as<int>();
+            g.nbmax = mf->fx_nbmax;
+            g.chan_b0 = mf->fx_cb0.as<int>(); g.chan_nb = mf->fx_cnb.as<int>();
+            g.Lmax = mf->fx_lmax;
+            CU(launch_fix_list(g, nctas, mf->stream));
+            ++mf->launches;
+        }
     if (mf->n_direct > 0)
     {
         FixParams<T> g = f;
-        g.flist = nullptr;
         g.dir_b0 = mf->dir_b0; g.ndir = mf->dir_nb;
         g.Lmax = mf->dir_lmax;
         CU(launch_fixup<T>(g, nctas, fixup_warps<T>(g.Lmax, mf->dev_smem), mf->stream));

@@ -34,17 +34,17 @@ constexpr float kFixTcC2Bf16 = 0.f;
 
 // Fix-up batches: the templates of a channel sorted by length, kFixBatch per
 // batch; coefficients (demeaned, unit norm, in the sample type) interleaved
-// as [i][kFixBatch] and zero past each template's length.  Two uses of the
-// same kernel: the FP32 fix-up of listed runs (flist), and the direct
-// time-domain correlation of templates too long for any FFT plan (every run
-// of batches dir_b0 .. dir_b0 + ndir - 1, both sample types).
+// as [i][kFixBatch] and zero past each template's length.  Two kernels read
+// them: the FP32 fix-up of listed runs (fix_list_kernel), and the direct
+// time-domain correlation of templates too long for any FFT plan (fixup_kernel,
+// every run of batches dir_b0 .. dir_b0 + ndir - 1, both sample types).
 template <class T> struct FixParams
 {
     const T *x;
     long ldx;
     T *rho;
     long ldr;
-    const int *flist;            // listed runs: c * ldf + r (null: direct mode)
+    const int *flist;            // listed runs: c * ldf + r
     const int *fcount;           // number of listed runs
     long ldf;
     int nruns;                   // runs per channel row

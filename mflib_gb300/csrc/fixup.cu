@@ -70,6 +70,15 @@ template <class T> cudaError_t launch_fixup(const FixParams<T> &p, int nctas, in
     fixup_kernel<T><<<nctas, 32 * warps, bytes, s>>>(p);
     return cudaGetLastError();
 }
+cudaError_t launch_fix_list(const FixParams<float> &p, int nctas, cudaStream_t s)
+{
+    const size_t bytes = fix_list_bytes(p.Lmax);
+    static SmemCap cap;
+    cudaError_t e = raise_smem_cap(fix_list_kernel, bytes, cap);
+    if (e != cudaSuccess) return e;
+    fix_list_kernel<<<nctas, 32 * kFixListWarps, bytes, s>>>(p);
+    return cudaGetLastError();
+}
 template cudaError_t launch_fixup<float>(const FixParams<float> &, int, int, cudaStream_t);
 template cudaError_t launch_fixup<double>(const FixParams<double> &, int, int, cudaStream_t);
 

@@ -28,13 +28,13 @@
 //     hi+lo split and FP32 accumulation err relative to |x - off|, off the
 //     strip's operand offset (chosen here as the level of the strip's
 //     quietest run).  Runs over the bound are flagged.
-//  3. fixup_kernel: every flagged run is recomputed for all templates on its
+//  3. fix_list_kernel: every flagged run is recomputed for all templates on its
 //     channel by a direct two-pass FP32 Pearson correlation about a local
 //     reference, whose error is relative to each window's own variance.  The
 //     fused peak candidates of the touched blocks are recounted
-//     (fix_rescan_kernel) and the tensor-core candidate flags updated.  The
-//     same kernel, in direct mode and in either sample type, correlates the
-//     templates too long for any FFT plan over every lag.
+//     (fix_rescan_kernel) and the tensor-core candidate flags updated.
+//     fixup_kernel, in either sample type, correlates the templates too long
+//     for any FFT plan over every lag the same way.
 #pragma once
 #include "kernels_mf.cuh"
 #include "fix_params.h"
@@ -427,15 +427,205 @@ template <class T> __host__ __device__ constexpr size_t fix_warp_bytes(int Lmax)
     return sizeof(T) * ((size_t) fix_yrow<T>(Lmax) + kFixBatch * kFixChunk);
 }
 
-// One warp per work item, grid-strided (blockDim.x / 32 warps per CTA).
-// List mode: item j is listed run i = j / nbmax with the k-th batch of its
-// channel (k = j % nbmax; items past the channel's batches are skipped), so
-// the runs of one amplitude step (which cluster) spread over every warp.
-// Direct mode: item j is run j / ndir of direct batch j % ndir.  Per item,
-// the 32 lags of each template of the batch: dot products against the
-// window's samples about a local reference (coefficients staged kFixChunk at
-// a time in shared memory), window mean and M2 two-pass per distinct
-// template length.
+// The 32 lags of one template of a recomputed run: store, fused candidate
+// flags (tensor-core path) or the slots to recount (FFT path).  One warp,
+// lane = lag.
+template <class T>
+__device__ __forceinline__ void fix_store(const FixParams<T> &p, int t, long lag0, int lane, T rho)
+{
+    const long lag = lag0 + lane;
+    if (lag < p.nvalid[t])
+    {
+        p.rho[(long) t * p.ldr + lag] = rho;
+        if (p.pk_flags && lag < p.pk_len && rho > p.pk_thr)
+        {
+            const long cc = lag >> 6;
+            atomicOr(p.pk_flags + (long) t * p.pk_words + (cc >> 5), 1u << (cc & 31));
+        }
+    }
+    if (p.pk_dirty && lane == 0)
+    {
+        // candidates at lags lag0 - 1 .. lag0 + 32 depend on these values
+        const long S = p.row_S ? p.row_S[t] : p.S0;
+        const long bl = (lag0 > 0 ? lag0 - 1 : 0) / S, bh = (lag0 + 32) / S;
+        for (long bb = bl; bb <= bh && bb < p.pk_stride; ++bb) p.pk_dirty[(long) t * p.pk_stride + bb] = 1;
+    }
+}
+
+// List mode (FP32): one CTA per (listed run, 16-template batch of its
+// channel), grid-strided; item j is run j / nbmax with batch j % nbmax
+// (items past the channel's batches are skipped), so the runs of one
+// amplitude step (which cluster) spread over every CTA.
+//
+// Few runs are listed in ordinary use (a loud arrival in a quiet block), so
+// the time of one item counts as much as the throughput: the template's
+// samples are split over the CTA's 8 warps in pieces of 32 (each lane one
+// lag, 8 packed FMAs per sample for the 16 templates), and the window
+// statistics come from the pieces' own means and sums of squares instead of
+// two passes over the whole window per distinct length.  One warp per item
+// with serial two-pass statistics took 240 us for 148 runs of a bank of 100
+// templates of up to 3,000 samples and 150 us for 143 runs of 512 templates
+// of 1,000.
+//
+// Window statistics of length L = 32 nc + re at lane's lag: the window's mean
+// from its nc piece means and re last samples, then M2 as the sum of the
+// pieces' own M2, 32 (piece mean - mean)^2 and the last samples' squares
+// about the mean: every term non-negative, nothing cancels (as the two-pass
+// form over samples).
+constexpr int kFixListWarps = 8;
+__host__ __device__ constexpr int fix_list_pieces(int Lmax) { return (Lmax + 31) / 32; }
+__host__ __device__ constexpr size_t fix_list_bytes(int Lmax)
+{
+    // samples | piece statistics (mean, M2 per lane) | staged coefficients, then the warps' partial sums | statistics
+    // per template
+    return sizeof(float) * ((size_t) fix_yrow<float>(Lmax + 32) + 64 * (size_t) fix_list_pieces(Lmax) +
+                            kFixListWarps * kFixBatch * 32 + 2 * kFixBatch * 32);
+}
+
+__global__ void __launch_bounds__(32 * kFixListWarps) fix_list_kernel(FixParams<float> p)
+{
+    extern __shared__ __align__(16) unsigned char smem_fl[];
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    float *ys = reinterpret_cast<float *>(smem_fl);
+    float2 *pst = reinterpret_cast<float2 *>(ys + fix_yrow<float>(p.Lmax + 32));  // [piece][lane]: mean, M2
+    float *csh = reinterpret_cast<float *>(pst + 32 * fix_list_pieces(p.Lmax));   // [warp][32][kFixBatch]
+    float2 *tst = reinterpret_cast<float2 *>(csh + kFixListWarps * kFixBatch * 32);  // [template][lane]: mean, M2
+    const long U = (long) *p.fcount * p.nbmax;
+    for (long j = blockIdx.x; j < U; j += gridDim.x)
+    {
+        const int e = p.flist[j / p.nbmax], k = (int) (j % p.nbmax);
+        const int c = (int) (e / p.ldf), r = (int) (e % p.ldf);
+        if (k >= p.chan_nb[c] || r >= p.nruns) continue;  // uniform across the CTA
+        const int B = p.chan_b0[c] + k;
+        const int Lb = p.bL[B];
+        const int mytid = lane < kFixBatch ? p.btid[B * kFixBatch + lane] : -1;
+        const int myL = mytid >= 0 ? p.tlen[mytid] : 0;
+        const int L0 = __shfl_sync(0xffffffffu, myL, 0);
+        const float *xc = p.x + (long) c * p.ldx;
+        const long lag0 = 32L * r;
+        for (int i = tid; i < Lb + 64; i += 32 * kFixListWarps) ys[i] = i < Lb + 31 ? xc[lag0 + i] : 0.f;
+        const int np = (Lb + 31) / 32;
+        const float4 *co = reinterpret_cast<const float4 *>(p.bco + p.boff[B]);
+        float4 *cw = reinterpret_cast<float4 *>(csh + (size_t) w * kFixBatch * 32);
+        // coefficients of piece q: 128 float4, four per lane; zero past Lb
+        auto fetch = [&](int q, float4 (&f)[4]) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+            {
+                const int v = lane + 32 * u;  // float4 v of the piece: sample v / 4
+                f[u] = 32 * q + v / 4 < Lb ? co[(long) q * 128 + v] : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+        };
+        f2 acc[kFixBatch / 2];
+#pragma unroll
+        for (int q = 0; q < kFixBatch / 2; ++q) acc[q] = f2_make(0.f, 0.f);
+        float4 nx[4];
+        if (w < np) fetch(w, nx);
+        __syncthreads();  // samples staged
+        // each lag's own reference, a sample of its shortest window: a run
+        // that straddles an amplitude step holds loud and quiet windows
+        const float Rl = ys[lane + L0 / 2];
+        for (int q = w; q < np; q += kFixListWarps)
+        {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) cw[lane + 32 * u] = nx[u];
+            __syncwarp();
+            if (q + kFixListWarps < np) fetch(q + kFixListWarps, nx);
+            float v[32], s = 0.f;
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+            {
+                v[i] = ys[lane + 32 * q + i] - Rl;
+                s += v[i];
+            }
+            const float mu = s * (1.f / 32.f);
+            float a = 0.f, b = 0.f;
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+            {
+                const float d = v[i] - mu;
+                a += d;
+                b = fmaf(d, d, b);
+                const ulonglong2 *cf = reinterpret_cast<const ulonglong2 *>(cw + 4 * i);
+                const f2 yy = f2_dup(v[i]);
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                {
+                    const ulonglong2 cc = cf[u];
+                    acc[2 * u] = fma2(f2{cc.x}, yy, acc[2 * u]);
+                    acc[2 * u + 1] = fma2(f2{cc.y}, yy, acc[2 * u + 1]);
+                }
+            }
+            // the rounding of mu moves into the piece's mean; its M2 about it
+            pst[32 * q + lane] = make_float2(fmaf(a, 1.f / 32.f, mu), fmaf(-a, a * (1.f / 32.f), b));
+            __syncwarp();  // the staged coefficients are rewritten next
+        }
+        __syncthreads();  // piece statistics complete, staged coefficients free
+        // the warps' partial sums [warp][template][lane]
+        float *red = csh;
+#pragma unroll
+        for (int q = 0; q < kFixBatch / 2; ++q)
+        {
+            float x0, x1;
+            f2_split(acc[q], x0, x1);
+            red[(w * kFixBatch + 2 * q) * 32 + lane] = x0;
+            red[(w * kFixBatch + 2 * q + 1) * 32 + lane] = x1;
+        }
+        // statistics of each distinct length (the batch is sorted by length:
+        // a template of the length before it shares them)
+        for (int q = w; q < kFixBatch; q += kFixListWarps)
+        {
+            const int L = __shfl_sync(0xffffffffu, myL, q);
+            const int Lp = q > 0 ? __shfl_sync(0xffffffffu, myL, q - 1) : -1;
+            if (L == 0 || L == Lp) continue;
+            const int nc = L >> 5;
+            float sm = 0.f, sp = 0.f;
+#pragma unroll 4
+            for (int i = 0; i < nc; ++i) sm += pst[32 * i + lane].x;
+            for (int i = 32 * nc; i < L; ++i) sp += ys[lane + i] - Rl;
+            const float mean = fmaf(32.f, sm, sp) / (float) L;
+            float a = 0.f, b = 0.f, ap = 0.f;
+#pragma unroll 4
+            for (int i = 0; i < nc; ++i)
+            {
+                const float2 t = pst[32 * i + lane];
+                const float d = t.x - mean;
+                a += d;
+                b += fmaf(32.f * d, d, t.y);
+            }
+            for (int i = 32 * nc; i < L; ++i)
+            {
+                const float d = (ys[lane + i] - Rl) - mean;
+                ap += d;
+                b = fmaf(d, d, b);
+            }
+            a = fmaf(32.f, a, ap);
+            tst[32 * q + lane] = make_float2(mean, fmaf(-a, a / (float) L, b));
+        }
+        __syncthreads();
+        for (int q = w; q < kFixBatch; q += kFixListWarps)
+        {
+            const int t = __shfl_sync(0xffffffffu, mytid, q);
+            if (t < 0) continue;  // empty slots (the batch's last ones)
+            const int L = __shfl_sync(0xffffffffu, myL, q);
+            // first slot of this length
+            const unsigned same = __ballot_sync(0xffffffffu, lane < kFixBatch && myL == L);
+            const float2 st = tst[32 * (__ffs(same) - 1) + lane];
+            float num = 0.f;
+#pragma unroll
+            for (int u = 0; u < kFixListWarps; ++u) num += red[(u * kFixBatch + q) * 32 + lane];
+            fix_store<float>(p, t, lag0, lane, fix_rho<float>(fmaf(-st.x, p.bsum[t], num), st.y, L, p.tol));
+        }
+        __syncthreads();  // shared memory reused by the next item
+    }
+}
+
+// Direct mode (templates longer than any FFT plan): one warp per work item,
+// grid-strided (blockDim.x / 32 warps per CTA); item j is run j / ndir of
+// direct batch j % ndir.  Per item, the 32 lags of each template of the
+// batch: dot products against the window's samples about a local reference
+// (coefficients staged kFixChunk at a time in shared memory), window mean and
+// M2 two-pass per distinct template length.
 template <class T> __global__ void __launch_bounds__(32 * kFixWarps) fixup_kernel(FixParams<T> p)
 {
     extern __shared__ __align__(16) unsigned char smem_fx_raw[];
@@ -445,31 +635,16 @@ template <class T> __global__ void __launch_bounds__(32 * kFixWarps) fixup_kerne
     T *ys = smem_fx + (size_t) wid * (yrow + kFixBatch * kFixChunk);
     T *csh = ys + yrow;
     const long W = (long) gridDim.x * nw;
-    const bool direct = p.flist == nullptr;
-    const long U = direct ? (long) p.nruns * p.ndir : (long) *p.fcount * p.nbmax;
+    const long U = (long) p.nruns * p.ndir;
     for (long j = (long) blockIdx.x * nw + wid; j < U; j += W)
     {
-        int B, c, r;
-        if (direct)
-        {
-            B = p.dir_b0 + (int) (j % p.ndir);
-            r = (int) (j / p.ndir);
-            c = p.bch[B];
-        }
-        else
-        {
-            const int e = p.flist[j / p.nbmax], k = (int) (j % p.nbmax);
-            c = (int) (e / p.ldf);
-            r = (int) (e % p.ldf);
-            if (k >= p.chan_nb[c] || r >= p.nruns) continue;
-            B = p.chan_b0[c] + k;
-        }
+        const int B = p.dir_b0 + (int) (j % p.ndir), r = (int) (j / p.ndir), c = p.bch[B];
         const int Lb = p.bL[B];
         const int mytid = lane < kFixBatch ? p.btid[B * kFixBatch + lane] : -1;
         const int L0 = __shfl_sync(0xffffffffu, mytid >= 0 ? p.tlen[mytid] : 0, 0);
         const T *xc = p.x + (long) c * p.ldx;
         const long lag0 = 32L * r;
-        const bool dead = direct && p.dead[c];
+        const bool dead = p.dead[c];
         T acc[kFixBatch];
 #pragma unroll
         for (int q = 0; q < kFixBatch; ++q) acc[q] = (T) 0;
@@ -496,7 +671,6 @@ template <class T> __global__ void __launch_bounds__(32 * kFixWarps) fixup_kerne
                 }
             }
         }
-        const long lag = lag0 + lane;
         int prevL = -1;
         T mu = 0, M2 = 0;
 #pragma unroll
@@ -520,23 +694,7 @@ template <class T> __global__ void __launch_bounds__(32 * kFixWarps) fixup_kerne
                 M2 = fma(-a, a / (T) Lt, b);
                 prevL = Lt;
             }
-            const T rho = dead ? (T) 0 : fix_rho<T>(fma(-mu, p.bsum[t], acc[q]), M2, Lt, p.tol);
-            if (lag < p.nvalid[t])
-            {
-                p.rho[(long) t * p.ldr + lag] = rho;
-                if (p.pk_flags && lag < p.pk_len && rho > p.pk_thr)
-                {
-                    const long cc = lag >> 6;
-                    atomicOr(p.pk_flags + (long) t * p.pk_words + (cc >> 5), 1u << (cc & 31));
-                }
-            }
-            if (p.pk_dirty && lane == 0)
-            {
-                // candidates at lags lag0 - 1 .. lag0 + 32 depend on these values
-                const long S = p.row_S ? p.row_S[t] : p.S0;
-                const long bl = (lag0 > 0 ? lag0 - 1 : 0) / S, bh = (lag0 + 32) / S;
-                for (long bb = bl; bb <= bh && bb < p.pk_stride; ++bb) p.pk_dirty[(long) t * p.pk_stride + bb] = 1;
-            }
+            fix_store<T>(p, t, lag0, lane, dead ? (T) 0 : fix_rho<T>(fma(-mu, p.bsum[t], acc[q]), M2, Lt, p.tol));
         }
         __syncwarp();  // ys reused by the next item
     }

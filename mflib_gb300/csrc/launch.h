@@ -72,6 +72,7 @@ template <class T>
 cudaError_t launch_fix_prep(const double *tmpl, const long *toff, const int *tlen, const int *btid, const long *boff,
                             const int *bL, int nbatch, T *bco, T *bsum, cudaStream_t s);
 template <class T> cudaError_t launch_fixup(const FixParams<T> &p, int nctas, int warps, cudaStream_t s);
+cudaError_t launch_fix_list(const FixParams<float> &p, int nctas, cudaStream_t s);
 template <class T>
 cudaError_t launch_fix_rescan(const T *rho, long ldr, int nt, int pk_stride, const unsigned char *dirty,
                               const int *row_S, const int *row_nblk, int S0, int nblk0, const int *nvalid, int pk_len,
