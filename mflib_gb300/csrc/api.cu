@@ -2485,9 +2485,10 @@ try
         return fail(MFGPU_EINVAL, "Threshold = " + std::to_string(threshold) + " must be in the range [0,1]");
     int len = trace_length > 0 ? trace_length : mf->n - mf->maxLen + 1;
     if (len > mf->maxvalid) return fail(MFGPU_EINVAL, "trace_length exceeds the valid lags");
-    mfgpu_status st = mf_sync(mf);
-    if (st != MFGPU_OK) return st;
+    // the search is enqueued behind the apply and waits once, at its end,
+    // where it also reads the status word
     mf->have_peaks = false;
+    int dev_err = 0;
     std::vector<int> rows(mf->nt);
     for (int t = 0; t < mf->nt; ++t) rows[t] = t;
     mf->pk_off.assign(mf->nt + 1, 0);
@@ -2505,11 +2506,16 @@ try
     int rc = mf->prec == 4
                  ? run_peaks<float>(mf->rho.as<float>(), mf->ldr, rows.data(), mf->nt, len, threshold, min_distance,
                                     mf->pk, mf->stream, &mf->launches, mf->pk_off.data(), err, fused ? &ff : nullptr,
-                                    flags, mf->pk_words)
+                                    flags, mf->pk_words, mf->err.as<int>(), &dev_err)
                  : run_peaks<double>(mf->rho.as<double>(), mf->ldr, rows.data(), mf->nt, len, threshold,
                                      min_distance, mf->pk, mf->stream, &mf->launches, mf->pk_off.data(), err,
-                                     fused ? &fd : nullptr);
+                                     fused ? &fd : nullptr, nullptr, 0, mf->err.as<int>(), &dev_err);
     if (rc != 0) return fail(MFGPU_ECUDA, err);
+    if (dev_err != 0 || mf->pk.dense)
+    {
+        mfgpu_status st = mf_sync(mf);
+        if (st != MFGPU_OK) return st;
+    }
     mf->have_peaks = true;
     return MFGPU_OK;
 }

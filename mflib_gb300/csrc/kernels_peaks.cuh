@@ -446,4 +446,269 @@ static __global__ void __launch_bounds__(kPkThreads)
     }
 }
 
+// ----------------------------------------------------------------------------
+// Pruning per trace.  Traces are independent, so one CTA takes a trace's
+// candidates into shared memory, runs the rounds above until none is
+// undecided and compacts the accepted ones: three launches (totals, prune,
+// emit) instead of two launches and a clear per round over a grid sized for
+// the candidate capacity, three scans and a compaction (25 launches, about
+// 130 us of mostly empty grids for the banks measured; now 15 us).  A trace
+// with more than kPkTraceCap candidates, or a chunk with more than its slot
+// holds, raises flags[0] and the host takes the launches above, which have no
+// such limit.
+constexpr int kPkTraceCap = 4096;
+constexpr int kPkTotThreads = 128;
+template <class T> constexpr size_t pk_prune_bytes() { return (sizeof(int) + sizeof(T) + 1) * (size_t) kPkTraceCap; }
+
+// Exclusive prefix of n ints by one CTA: out[0..n]; sh holds 32 values.
+static __device__ __forceinline__ void cta_prefix(const int *in, int n, long long *out, long long *sh)
+{
+    long long base = 0;
+    for (int i0 = 0; i0 < n; i0 += blockDim.x)
+    {
+        const int i = i0 + threadIdx.x;
+        long long tot;
+        const long long e = block_excl_scan((long long) (i < n ? __ldcg(in + i) : 0), sh, &tot);
+        if (i < n) out[i] = base + e;
+        base += tot;
+    }
+    if (threadIdx.x == 0) out[n] = base;
+}
+
+// True in every thread of the last CTA of the grid to get here (whose other
+// CTAs' global stores before the call are then visible); the ticket is left
+// at 0 for the next launch.
+static __device__ __forceinline__ bool last_cta(int *ticket, int *sh)
+{
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0)
+    {
+        *sh = atomicAdd(ticket, 1) == (int) gridDim.x - 1;
+        if (*sh) *ticket = 0;
+    }
+    __syncthreads();
+    const bool last = *sh != 0;
+    if (last) __threadfence();
+    return last;
+}
+
+// Candidates per trace (FUSED: with the block-edge lags decided here, as
+// peak_seam_kernel), and by the last CTA the traces' offsets.
+template <class T, bool FUSED>
+static __global__ void __launch_bounds__(kPkTotThreads)
+    peak_totals_kernel(PeakTraces<T> tr, FusedSlots<T> fs, int nchunks, int *counts, unsigned char *ht, int *totals,
+                       long long *trace_beg, int *ticket, int *flags)
+{
+    __shared__ long long sh[32];
+    __shared__ int lsh;
+    const int trace = blockIdx.x, row = tr.row[trace];
+    const long n = tr.len;
+    const T *x = tr.x + (long) row * tr.ldx;
+    const int nb = FUSED && fs.row_nblk ? fs.row_nblk[row] : nchunks;
+    const long S = FUSED && fs.row_S ? fs.row_S[row] : fs.S;
+    long long mine = 0;
+    for (int b = threadIdx.x; b < nchunks; b += kPkTotThreads)
+    {
+        const long g = (long) trace * nchunks + b;
+        int cnt;
+        if constexpr (FUSED)
+        {
+            const long i0 = (long) b * S, i1 = i0 + S - 1;
+            int h = 0, tl = 0;
+            cnt = 0;
+            if (b < nb)
+            {
+                h = (i0 < n && is_candidate<T>(x, (int) i0, (int) n, tr.thr)) ? 1 : 0;
+                tl = (i1 < n && is_candidate<T>(x, (int) i1, (int) n, tr.thr)) ? 1 : 0;
+                cnt = h + fs.cnt[(long) row * fs.nblk + b] + tl;
+            }
+            counts[g] = cnt;
+            ht[g] = (unsigned char) (h | (tl << 1));
+        }
+        else
+            cnt = counts[g];
+        mine += cnt;
+    }
+    long long tot;
+    block_excl_scan(mine, sh, &tot);
+    if (threadIdx.x == 0) totals[trace] = (int) tot;
+    if (last_cta(ticket, &lsh))
+    {
+        cta_prefix(totals, gridDim.x, trace_beg, sh);
+        if (threadIdx.x == 0) flags[0] = 0;
+    }
+}
+
+// One CTA per trace: gather, prune, compact into raw[trace_beg[t]...], the
+// accepted count in nacc; the last CTA forms the traces' peak offsets.
+template <class T, bool FUSED>
+static __global__ void __launch_bounds__(kPkThreads)
+    peak_prune_kernel(PeakTraces<T> tr, FusedSlots<T> fs, int nchunks, const int *counts, const unsigned char *ht,
+                      const int *slot_idx, const T *slot_val, int dist, const long long *trace_beg, long long cap,
+                      int *raw, int *nacc, long long *peak_off, int *ticket, int *flags)
+{
+    extern __shared__ __align__(16) unsigned char smem_pk[];
+    __shared__ long long sh[32];
+    __shared__ int lsh;
+    T *val = reinterpret_cast<T *>(smem_pk);
+    int *idx = reinterpret_cast<int *>(val + kPkTraceCap);
+    unsigned char *state = reinterpret_cast<unsigned char *>(idx + kPkTraceCap);
+    const int tid = threadIdx.x, trace = blockIdx.x, row = tr.row[trace];
+    const long long tb = trace_beg[trace];
+    const long long total = trace_beg[trace + 1] - tb;
+    const T *x = tr.x + (long) row * tr.ldx;
+    bool ok = total <= kPkTraceCap && trace_beg[gridDim.x] <= cap;
+    int accepted = 0;
+    if (ok && total > 0)
+    {
+        const int nc = (int) total;
+        // ---- candidates in index order; a thread packs one chunk
+        long long base = 0;
+        bool over = false;
+        for (int b0 = 0; b0 < nchunks; b0 += kPkThreads)
+        {
+            const int b = b0 + tid;
+            const long g = (long) trace * nchunks + b;
+            const int cnt = b < nchunks ? counts[g] : 0;
+            long long tot;
+            int o = (int) (base + block_excl_scan((long long) cnt, sh, &tot));
+            base += tot;
+            if (cnt == 0) continue;
+            if constexpr (FUSED)
+            {
+                const int hv = ht[g];
+                const long S = fs.row_S ? fs.row_S[row] : fs.S;
+                const long i0 = (long) b * S, bs = (long) row * fs.nblk + b;
+                const int bc = cnt - (hv & 1) - (hv >> 1);
+                if (bc > kPkCap)
+                {
+                    over = true;
+                    continue;
+                }
+                if (hv & 1)
+                {
+                    idx[o] = (int) i0;
+                    val[o++] = x[i0];
+                }
+                for (int q = 0; q < bc; ++q)
+                {
+                    // insertion by index: the slot's entries are unordered
+                    const int ir = fs.idx[bs * kPkCap + q];
+                    const T vr = fs.val[bs * kPkCap + q];
+                    int k = o + q;
+                    for (; k > o && idx[k - 1] > ir; --k)
+                    {
+                        idx[k] = idx[k - 1];
+                        val[k] = val[k - 1];
+                    }
+                    idx[k] = ir;
+                    val[k] = vr;
+                }
+                o += bc;
+                if (hv & 2)
+                {
+                    idx[o] = (int) (i0 + S - 1);
+                    val[o] = x[i0 + S - 1];
+                }
+            }
+            else
+            {
+                if (cnt > kPkCap)
+                {
+                    over = true;
+                    continue;
+                }
+                for (int q = 0; q < cnt; ++q)
+                {
+                    idx[o + q] = slot_idx[g * kPkCap + q];
+                    val[o + q] = slot_val[g * kPkCap + q];
+                }
+            }
+        }
+        ok = !__syncthreads_or(over);
+        if (ok)
+        {
+            for (int i = tid; i < nc; i += kPkThreads) state[i] = dist > 0 ? PK_UNDECIDED : PK_ACCEPTED;
+            __syncthreads();
+            // ---- rounds: each accepts at least the best undecided candidate
+            bool left = dist > 0;
+            while (left)
+            {
+                bool mine = false;
+                for (int g = tid; g < nc; g += kPkThreads)
+                {
+                    if (state[g] != PK_UNDECIDED) continue;
+                    const int ig = idx[g];
+                    const T vg = val[g];
+                    bool best = true;
+                    for (int k = g - 1; k >= 0 && ig - idx[k] <= dist; --k)
+                        if (state[k] <= PK_NEW && state[k] != PK_ACCEPTED && higher<T>(val[k], idx[k], vg, ig))
+                        {
+                            best = false;
+                            break;
+                        }
+                    if (best)
+                        for (int k = g + 1; k < nc && idx[k] - ig <= dist; ++k)
+                            if (state[k] <= PK_NEW && state[k] != PK_ACCEPTED && higher<T>(val[k], idx[k], vg, ig))
+                            {
+                                best = false;
+                                break;
+                            }
+                    if (best) state[g] = PK_NEW;
+                    else mine = true;
+                }
+                left = __syncthreads_or(mine);
+                for (int g = tid; g < nc; g += kPkThreads)
+                {
+                    if (state[g] != PK_NEW) continue;
+                    const int ig = idx[g];
+                    for (int k = g - 1; k >= 0 && ig - idx[k] <= dist; --k)
+                        if (state[k] == PK_UNDECIDED) state[k] = PK_REJECTED;
+                    for (int k = g + 1; k < nc && idx[k] - ig <= dist; ++k)
+                        if (state[k] == PK_UNDECIDED) state[k] = PK_REJECTED;
+                    state[g] = PK_ACCEPTED;
+                }
+                __syncthreads();
+            }
+            // ---- accepted lags, ascending
+            for (int g0 = 0; g0 < nc; g0 += kPkThreads)
+            {
+                const int g = g0 + tid;
+                const bool a = g < nc && state[g] == PK_ACCEPTED;
+                long long tot;
+                const long long o = block_excl_scan((long long) (a ? 1 : 0), sh, &tot);
+                if (a) raw[tb + accepted + o] = idx[g];
+                accepted += (int) tot;
+            }
+        }
+    }
+    if (tid == 0)
+    {
+        nacc[trace] = accepted;
+        if (!ok) flags[0] = 1;
+    }
+    if (last_cta(ticket, &lsh)) cta_prefix(nacc, gridDim.x, peak_off, sh);
+}
+
+// The traces' accepted lags side by side; res[ntr + 1 ..]: candidates, bail
+// flag, the object's device status word.
+static __global__ void __launch_bounds__(64) peak_emit_kernel(int ntr, const int *raw, const long long *trace_beg,
+                                                              const int *flags, const int *err, long long *res,
+                                                              int *peaks)
+{
+    const int t = blockIdx.x;
+    const bool bail = flags[0] != 0;
+    if (t == 0 && threadIdx.x == 0)
+    {
+        res[ntr + 1] = trace_beg[ntr];
+        res[ntr + 2] = bail ? 1 : 0;
+        res[ntr + 3] = err ? *err : 0;
+    }
+    if (bail) return;
+    const long long o = res[t], b = trace_beg[t];
+    const int n = (int) (res[t + 1] - o);
+    for (int i = threadIdx.x; i < n; i += 64) peaks[o + i] = raw[b + i];
+}
+
 }  // namespace mfgpu

@@ -144,18 +144,32 @@ struct DevBuf
     template <class U> U *as() const { return static_cast<U *>(p); }
 };
 
+// what a peak search looks at, for the choice between its two forms
+struct PeakSearch
+{
+    double thr = 0;
+    int ntr = 0, len = 0, dist = 0;
+    bool fused = false;
+    bool operator==(const PeakSearch &o) const
+    {
+        return thr == o.thr && ntr == o.ntr && len == o.len && dist == o.dist && fused == o.fused;
+    }
+};
+
 // peak finder pipeline over ntr traces (rows of a matrix)
 struct PeakWS
 {
     DevBuf counts, offs, slot_idx, slot_val, cidx, cval, ctr, state, flags, pos, tiles, trace_beg, peak_off, peaks,
-        counter, row, ht;
+        counter, row, ht, totals, nacc, ticket;
+    bool dense = false;        // dense_search had a trace with more candidates than one CTA prunes
+    PeakSearch dense_search;
     long long npeaks = 0;
     long long cand_cap = 1 << 16;  // capacity of the packed candidate arrays
     std::vector<int> rows_on_device;  // the trace rows last uploaded to `row`
     template <class F> void each_buf(F &&f)
     {
         DevBuf *all[] = {&counts, &offs, &slot_idx, &slot_val, &cidx, &cval, &ctr, &state, &flags,
-                         &pos, &tiles, &trace_beg, &peak_off, &peaks, &counter, &row, &ht};
+                         &pos, &tiles, &trace_beg, &peak_off, &peaks, &counter, &row, &ht, &totals, &nacc, &ticket};
         for (DevBuf *d : all) f(*d);
     }
     void release()
@@ -163,6 +177,7 @@ struct PeakWS
         each_buf([](DevBuf &d) { d.release(); });
         npeaks = 0;
         cand_cap = 1 << 16;
+        dense = false;
         rows_on_device.clear();
     }
 };
@@ -173,10 +188,13 @@ struct PeakWS
 // trace length) replace the scan over the traces.  Otherwise `flags` (bit
 // per 64 lags of each row, fwords words per row; see PeakTraces), when given,
 // lets the scan skip the lags no value above the threshold lies in.
+// host_err (optional) receives the device status word dev_err as of the end
+// of the search (0 when not read).
 template <class T>
 int run_peaks(const T *x, long ldx, const int *host_rows, int ntr, int len, double thr, int dist, PeakWS &ws,
               cudaStream_t s, long long *launches, long long *host_peak_off, std::string &err,
-              const FusedSlots<T> *fused = nullptr, const unsigned *flags = nullptr, int fwords = 0);
+              const FusedSlots<T> *fused = nullptr, const unsigned *flags = nullptr, int fwords = 0,
+              const int *dev_err = nullptr, int *host_err = nullptr);
 
 // ---------------------------------------------------------------------------
 // DBSCAN over segments

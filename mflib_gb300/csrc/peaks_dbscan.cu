@@ -36,9 +36,10 @@ cudaError_t device_excl_scan(const int *in, long n, long long *out, long long *t
 template <class T>
 int run_peaks(const T *x, long ldx, const int *host_rows, int ntr, int len, double thr, int dist, PeakWS &ws,
               cudaStream_t s, long long *launches, long long *host_peak_off, std::string &err,
-              const FusedSlots<T> *fused, const unsigned *flags, int fwords)
+              const FusedSlots<T> *fused, const unsigned *flags, int fwords, const int *dev_err, int *host_err)
 {
     ws.npeaks = 0;
+    if (host_err) *host_err = 0;
     if (ntr <= 0) return 0;
     if (len <= 0)
     {
@@ -55,16 +56,14 @@ int run_peaks(const T *x, long ldx, const int *host_rows, int ntr, int len, doub
         if (ws.row.p != old) ws.rows_on_device.clear();  // a new buffer holds no rows
     }
     MF_TRY(ws.trace_beg.ensure(sizeof(long long) * (ntr + 1)));
-    MF_TRY(ws.peak_off.ensure(sizeof(long long) * (ntr + 1)));
+    MF_TRY(ws.peak_off.ensure(sizeof(long long) * (ntr + 4)));
     MF_TRY(ws.counts.ensure(sizeof(int) * nslots));
-    MF_TRY(ws.offs.ensure(sizeof(long long) * (nslots + 1)));
     if (fused) MF_TRY(ws.ht.ensure(nslots));
     else
     {
         MF_TRY(ws.slot_idx.ensure(sizeof(int) * nslots * kPkCap));
         MF_TRY(ws.slot_val.ensure(sizeof(T) * nslots * kPkCap));
     }
-    MF_TRY(ws.counter.ensure(4 * sizeof(int)));  // [0] undecided after the last round, [1] overflow
     // the rows rarely change between calls: upload only when they do (an
     // upload queues behind any large host-to-device copy in flight)
     if (ws.rows_on_device.size() != (size_t) ntr ||
@@ -74,14 +73,79 @@ int run_peaks(const T *x, long ldx, const int *host_rows, int ntr, int len, doub
         MF_TRY(cudaStreamSynchronize(s));  // host_rows may be a temporary
         ws.rows_on_device.assign(host_rows, host_rows + ntr);
     }
-    int *undecided = ws.counter.as<int>(), *overflow = ws.counter.as<int>() + 1;
-    const long long *ncand_dev = ws.offs.as<long long>() + nslots;
-
     PeakTraces<T> tr;
     tr.x = x; tr.ldx = ldx; tr.row = ws.row.as<int>(); tr.len = len; tr.thr = (T) thr;
     tr.flags = fused ? nullptr : flags; tr.fwords = fwords;
     const dim3 grid(nchunks, ntr);
     const bool prune = dist > 0;
+
+    // One CTA per trace, unless this search's candidates did not fit it the
+    // last time (the same traces are then as dense again)
+    const PeakSearch search{thr, ntr, len, dist, fused != nullptr};
+    if (!(ws.dense && ws.dense_search == search))
+    {
+        const long long cap = ws.cand_cap;
+        MF_TRY(ws.totals.ensure(sizeof(int) * ntr));
+        MF_TRY(ws.nacc.ensure(sizeof(int) * ntr));
+        MF_TRY(ws.cidx.ensure(sizeof(int) * cap));
+        MF_TRY(ws.peaks.ensure(sizeof(int) * cap));
+        if (!ws.ticket.p)
+        {
+            MF_TRY(ws.ticket.ensure(4 * sizeof(int)));  // [0], [1] tickets, [2] the bail flag
+            MF_TRY(cudaMemsetAsync(ws.ticket.p, 0, 4 * sizeof(int), s));
+        }
+        int *tick = ws.ticket.as<int>();
+        long long *res = ws.peak_off.as<long long>();
+        const size_t bytes = pk_prune_bytes<T>();
+        static SmemCap capf, caps;
+        FusedSlots<T> none{};
+        if (fused)
+        {
+            peak_totals_kernel<T, true><<<ntr, kPkTotThreads, 0, s>>>(tr, *fused, nchunks, ws.counts.as<int>(),
+                                                                     ws.ht.as<unsigned char>(), ws.totals.as<int>(),
+                                                                     ws.trace_beg.as<long long>(), tick, tick + 2);
+            MF_TRY(raise_smem_cap(peak_prune_kernel<T, true>, bytes, capf));
+            peak_prune_kernel<T, true><<<ntr, kPkThreads, bytes, s>>>(
+                tr, *fused, nchunks, ws.counts.as<int>(), ws.ht.as<unsigned char>(), nullptr, nullptr, dist,
+                ws.trace_beg.as<long long>(), cap, ws.cidx.as<int>(), ws.nacc.as<int>(), res, tick + 1, tick + 2);
+            *launches += 3;
+        }
+        else
+        {
+            peak_cand_kernel<T><<<grid, kPkThreads, 0, s>>>(tr, nchunks, ws.counts.as<int>(), ws.slot_idx.as<int>(),
+                                                            ws.slot_val.as<T>());
+            peak_totals_kernel<T, false><<<ntr, kPkTotThreads, 0, s>>>(tr, none, nchunks, ws.counts.as<int>(), nullptr,
+                                                                      ws.totals.as<int>(),
+                                                                      ws.trace_beg.as<long long>(), tick, tick + 2);
+            MF_TRY(raise_smem_cap(peak_prune_kernel<T, false>, bytes, caps));
+            peak_prune_kernel<T, false><<<ntr, kPkThreads, bytes, s>>>(
+                tr, none, nchunks, ws.counts.as<int>(), nullptr, ws.slot_idx.as<int>(), ws.slot_val.as<T>(), dist,
+                ws.trace_beg.as<long long>(), cap, ws.cidx.as<int>(), ws.nacc.as<int>(), res, tick + 1, tick + 2);
+            *launches += 4;
+        }
+        peak_emit_kernel<<<ntr, 64, 0, s>>>(ntr, ws.cidx.as<int>(), ws.trace_beg.as<long long>(), tick + 2, dev_err, res,
+                                            ws.peaks.as<int>());
+        MF_TRY(cudaGetLastError());
+        std::vector<long long> got(ntr + 4);
+        MF_TRY(cudaMemcpyAsync(got.data(), res, sizeof(long long) * (ntr + 4), cudaMemcpyDeviceToHost, s));
+        MF_TRY(cudaStreamSynchronize(s));
+        if (host_err) *host_err = (int) got[ntr + 3];
+        if (got[ntr + 2] == 0)
+        {
+            std::copy(got.begin(), got.begin() + ntr + 1, host_peak_off);
+            ws.npeaks = host_peak_off[ntr];
+            ws.dense = false;
+            return 0;
+        }
+        ws.dense = true;
+        ws.dense_search = search;
+    }
+
+    // Any number of candidates: rounds over all traces' packed candidates
+    MF_TRY(ws.offs.ensure(sizeof(long long) * (nslots + 1)));
+    MF_TRY(ws.counter.ensure(4 * sizeof(int)));  // [0] undecided after the last round, [1] overflow
+    int *undecided = ws.counter.as<int>(), *overflow = ws.counter.as<int>() + 1;
+    const long long *ncand_dev = ws.offs.as<long long>() + nslots;
     for (int attempt = 0; attempt < 4; ++attempt)
     {
         const long long cap = ws.cand_cap;
@@ -188,10 +252,10 @@ int run_peaks(const T *x, long ldx, const int *host_rows, int ntr, int len, doub
 }
 template int run_peaks<float>(const float *, long, const int *, int, int, double, int, PeakWS &, cudaStream_t,
                               long long *, long long *, std::string &, const FusedSlots<float> *,
-                              const unsigned *, int);
+                              const unsigned *, int, const int *, int *);
 template int run_peaks<double>(const double *, long, const int *, int, int, double, int, PeakWS &, cudaStream_t,
                                long long *, long long *, std::string &, const FusedSlots<double> *,
-                               const unsigned *, int);
+                               const unsigned *, int, const int *, int *);
 
 int run_dbscan(int n, int nf, const double *X, const double *w, double eps, int min_obs, int nseg,
                const int *seg_off_host, int *labels_host, int *nclusters_host, DbWS &ws, cudaStream_t s,

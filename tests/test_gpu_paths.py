@@ -46,3 +46,27 @@ def test_listed_runs(gpu, oracle, rng, lens):
     f.apply()
     assert f.get_fixup_runs() > 0
     assert _worst(f, oracle, tps, [x] * len(lens)) < FP32_TOL
+
+
+# pruning per trace: traces without a candidate, with more than one CTA
+# prunes (the general rounds take over) and with more candidates in a chunk
+# than its slot holds; separations from none to the trace's length.  Indices
+# are compared exactly, on the coefficients the search ran on.
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("thr,dist", [(0.0625, 0), (0.0625, 1), (0.03125, 7), (0.3125, 40), (0.3125, 50_000), (0.984375, 3)])
+@pytest.mark.parametrize("fused", [False, True])
+def test_prune_per_trace(gpu, oracle, rng, dtype, thr, dist, fused):
+    n, lens = 41_007, (60, 300, 200, 300, 60)
+    x = rng.standard_normal((2, n))
+    x[1, 1000:9000] = 0.0
+    tps = [x[t % 2, 20_000 + 500 * t:20_000 + 500 * t + L].copy() for t, L in enumerate(lens)]
+    f = _filter(gpu, tps, [t % 2 for t in range(len(lens))], 2, n, dtype)
+    f.set_channel_signals(x.astype(dtype))
+    if fused:
+        f.set_peak_threshold(thr)
+    f.apply()
+    for _ in range(2):
+        f.find_peaks(thr, dist)
+        for t in range(len(lens)):
+            ref = oracle.peaks(f.get_matched_filtered_signal(t).astype(np.float64), thr, dist)
+            np.testing.assert_array_equal(f.get_peaks(t), ref)
