@@ -221,8 +221,9 @@ mfgpu_status mfgpu_mf_get_device_signal(mfgpu_mf *mf, int it, const void **dptr,
 /* Overlap-save plan chosen at initialize. */
 mfgpu_status mfgpu_mf_get_plan(const mfgpu_mf *mf, int *fft_length, int *lags_per_block, int *n_blocks);
 /* Correlator organisation chosen at initialize, numbered like
- * correlator_variant (1-3, 5 and 6 FFT organisations, 4 tensor cores); for the
- * tensor-core path also the templates per group and the padded K, else 0.
+ * correlator_variant (1-3, 5 and 6 FFT organisations, 4 tensor cores), or 7 for
+ * the integer transforms that FP64 data take unless an FFT length, an
+ * organisation or several buckets are asked for; for the tensor-core path also the templates per group and the padded K, else 0.
  * Extension: the reference has one CPU correlator and no such query. */
 mfgpu_status mfgpu_mf_get_correlator(const mfgpu_mf *mf, int *variant, int *tc_group, int *tc_k);
 /* Length buckets chosen at initialize: their number, and for each (up to
@@ -232,7 +233,7 @@ mfgpu_status mfgpu_mf_get_correlator(const mfgpu_mf *mf, int *variant, int *tc_g
 mfgpu_status mfgpu_mf_get_buckets(const mfgpu_mf *mf, int max, int *fft_lengths, int *n_templates, int *count);
 /* Per length bucket (same order, up to max): lags per block and the FFT
  * organisation numbered like correlator_variant (4 for the tensor-core
- * correlator, which has one bucket).  Extension. */
+ * correlator, 7 for the integer one, which have one bucket).  Extension. */
 mfgpu_status mfgpu_mf_get_bucket_plans(const mfgpu_mf *mf, int max, int *lags_per_block, int *variants, int *count);
 /* Request-window upload for a serving loop.  Extension: the reference sets
  * whole-length signals one template at a time (setSignal,

@@ -295,6 +295,11 @@ struct mfgpu_mf
     float last_xcorr_ms = 0, last_apply_ms = 0;
     bool test_wait_timeout = false;  // mfgpu_mf_test_wait_timeout: the next apply only
     int dev_smem = 0;                // opt-in shared memory per block of the device
+    // FP64 data correlated in integer arithmetic (kernels_int.cuh): template
+    // table, twiddles, lags and number of the normalisation tiles
+    bool intx = false;
+    DevBuf int_B, int_tw;
+    int int_lags = 0, int_tiles = 0;
     bool persistent = false;         // FFT correlator as a persistent work-queue launch (option)
     bool tc_bf16 = false;            // tensor-core operands split into BF16 instead of FP16 (option)
     float tc_maxb = 0.f;             // largest coefficient of the unit-norm templates (tensor-core path)
@@ -309,7 +314,7 @@ struct mfgpu_mf
                          &xrange,   &tc_B,   &tc_bscale, &tc_grp_chan, &tc_grp_tid, &pk_flags,
                          &rstat,    &cst,    &fxbits, &fxlist, &fxcount, &tc_off, &fx_btid, &fx_boff,
                          &fx_bL,    &fx_cb0, &fx_cnb, &fx_bch, &dlags,
-                         &fx_bco,   &fx_bsum, &pk_dirty, &tws, &tickets};
+                         &fx_bco,   &fx_bsum, &pk_dirty, &tws, &tickets, &int_B, &int_tw};
         for (DevBuf *d : all) f(*d);
         pk.each_buf(f);
         f(row_S);
@@ -350,6 +355,7 @@ struct mfgpu_mf
         can_stack = false;
         nfft = log2p = S = nblocks = ngroups = maxvalid = 0;
         ldx = ldr = 0;
+        intx = false;
         fx_on = false;
         fx_L = fx_nden = fx_nruns = fx_nbatch = 0;
         fx_nbmax = fx_lmax = n_direct = dir_b0 = dir_nb = dir_lmax = fLen = fMin = 0;
@@ -802,7 +808,10 @@ try
     std::vector<int> cuts{0, ntf};
     const int maxb = p->length_buckets > 0 ? p->length_buckets : 3;
     if (p->length_buckets < 0) return fail(MFGPU_EINVAL, "length_buckets must be >= 0");
-    if (!all_equal && p->fft_length == 0 && (forced_mode <= 1 || forced_mode == 4) && maxb > 1)
+    // FP64 data take the integer correlator unless the caller asks for an FFT
+    // plan (a length, an organisation, several buckets)
+    mf->intx = mf->prec == 8 && ntf > 0 && v == 0 && p->fft_length == 0 && !bucket_forced && p->length_buckets <= 1;
+    if (!mf->intx && !all_equal && p->fft_length == 0 && (forced_mode <= 1 || forced_mode == 4) && maxb > 1)
     {
         std::vector<int> pos{0};
         for (int q = 1; q < 64; ++q)
@@ -855,7 +864,8 @@ try
         if (is_direct[t]) bucket_of[t] = -1;  // in no FFT plan
     const int mv0 = ntf > 0 ? n - mf->lens[order[cuts[nbk - 1]]] + 1 : 0;
     const PlanPick best =
-        plan_for(maxLen, nbk > 1 ? mv0 : maxvalid_f, all_equal, bucket_nfft(nbk - 1), bucket_mode(nbk - 1));
+        mf->intx ? PlanPick{11, ((kIntN - maxLen + 1) / 32) * 32, 0, 0.0}
+                 : plan_for(maxLen, nbk > 1 ? mv0 : maxvalid_f, all_equal, bucket_nfft(nbk - 1), bucket_mode(nbk - 1));
     if (best.l2p < 0 && (bucket_nfft(nbk - 1) > 0 || bucket_mode(nbk - 1) >= 0))
         return fail(MFGPU_EINVAL, "the plan override of bucket " + std::to_string(nbk - 1) + " does not fit");
     const int best_l2p = best.l2p, best_S = best.S, best_mode = best.mode;
@@ -1030,7 +1040,10 @@ try
             for (int c = 0; c < nch; ++c) ng += (pc[c] + gsz - 1) / gsz;
             return ng;
         };
-        while (G > 1 && ((long) nblocks * count_groups(G) < 4L * 152 * 2 || count_groups(G) > 65535)) G = (G + 1) / 2;
+        // (the integer correlator holds one CTA per SM, whose start costs
+        // about as much as two templates: two CTAs per SM are enough)
+        const long want = mf->intx ? 2L * 152 : 4L * 152 * 2;
+        while (G > 1 && ((long) nblocks * count_groups(G) < want || count_groups(G) > 65535)) G = (G + 1) / 2;
         if (count_groups(G) > 65535) return false;
         for (int c = 0; c < nch; ++c)
         {
@@ -1096,9 +1109,23 @@ try
     CU(cudaMemcpyAsync(mf->tchan_d.p, mf->tchan.data(), sizeof(int) * nt, cudaMemcpyHostToDevice, mf->stream));
     CU(mf->xrange.ensure(sizeof(float) * nch));
     CU(cudaMemsetAsync(mf->xrange.p, 0, sizeof(float) * nch, mf->stream));
-    mfgpu_status s2 = mf->prec == 4 ? mf_upload_tables<float>(mf, mf->log2p, mf->tw, mf->Bc,
-                                                              mf->mode_x == 4 ? &mf->tws : nullptr)
-                                    : mf_upload_tables<double>(mf, mf->log2p, mf->tw, mf->Bc);
+    mfgpu_status s2 = MFGPU_OK;
+    if (mf->intx)
+    {
+        const std::vector<int> &tw = int_twiddles();
+        CU(mf->int_tw.ensure(sizeof(int) * tw.size()));
+        CU(cudaMemcpyAsync(mf->int_tw.p, tw.data(), sizeof(int) * tw.size(), cudaMemcpyHostToDevice, mf->stream));
+        CU(mf->int_B.ensure(sizeof(int) * (size_t) nt * kIntPrimes * kIntN));
+        mf->int_lags = ((kIntTile - maxLen) / 32) * 32;
+        mf->int_tiles = (std::max(1, maxvalid_f) + mf->int_lags - 1) / mf->int_lags;
+        CU(launch_int_bank(mf->tmpl_d.as<double>(), mf->toff_d.as<long>(), mf->tlen_d.as<int>(), nt,
+                           mf->int_tw.as<int>(), mf->int_B.as<int>(), mf->stream));
+        ++mf->launches;
+    }
+    else
+        s2 = mf->prec == 4 ? mf_upload_tables<float>(mf, mf->log2p, mf->tw, mf->Bc,
+                                                    mf->mode_x == 4 ? &mf->tws : nullptr)
+                           : mf_upload_tables<double>(mf, mf->log2p, mf->tw, mf->Bc);
     if (s2 != MFGPU_OK) return s2;
     for (size_t b = 0; b < mf->xb.size(); ++b)
     {
@@ -1326,7 +1353,7 @@ mfgpu_status mfgpu_mf_get_correlator(const mfgpu_mf *mf, int *variant, int *tc_g
 try
 {
     MF_CHECK_INIT(mf);
-    if (variant) *variant = mf->tc ? 4 : mf->mode_x == 3 ? 5 : mf->mode_x == 4 ? 6 : mf->mode_x + 1;
+    if (variant) *variant = mf->tc ? 4 : mf->intx ? 7 : mf->mode_x == 3 ? 5 : mf->mode_x == 4 ? 6 : mf->mode_x + 1;
     if (tc_group) *tc_group = mf->tc ? mf->tc_Gp : 0;
     if (tc_k) *tc_k = mf->tc ? mf->tc_Kp : 0;
     return MFGPU_OK;
@@ -1366,7 +1393,7 @@ try
     {
         const bool prim = b == nb - 1;
         if (lags_per_block) lags_per_block[b] = prim ? mf->S : mf->xb[b]->S;
-        if (variants) variants[b] = prim ? (mf->tc ? 4 : variant_of(mf->mode_x)) : variant_of(mf->xb[b]->mode);
+        if (variants) variants[b] = prim ? (mf->tc ? 4 : mf->intx ? 7 : variant_of(mf->mode_x)) : variant_of(mf->xb[b]->mode);
     }
     return MFGPU_OK;
 }
@@ -1905,7 +1932,18 @@ template <class T> static mfgpu_status mf_launch_xcorr(mfgpu_mf *mf)
             }
         }
     }
-    if (mf->shared_den && !(sizeof(T) == 4 && mf->fx_on))
+    if constexpr (sizeof(T) == 8)
+        if (mf->intx)
+        {
+            IntDenParams d{};
+            d.x = p.x; d.ldx = p.ldx; d.n = mf->n; d.dead = p.dead; d.tol = p.tol; d.lags = mf->int_lags;
+            d.L = mf->fLen; d.nv = mf->n - mf->fLen + 1; d.den = mf->den.as<double>(); d.ldd = p.ldd;
+            d.grp_chan = p.grp_chan; d.grp_tb = p.grp_tb; d.grp_te = p.grp_te; d.tids = p.tids;
+            d.tlen = p.tlen; d.nvalid = p.nvalid; d.rho = p.rho; d.ldr = p.ldr;
+            CU(launch_int_den(d, !mf->shared_den, mf->int_tiles, mf->shared_den ? mf->nch : mf->ngroups, mf->stream));
+            ++mf->launches;
+        }
+    if (mf->shared_den && !mf->intx && !(sizeof(T) == 4 && mf->fx_on))
     {
         CU(launch_den<T>(mf->x.as<T>(), mf->ldx, mf->fLen, mf->den.as<T>(), mf->ldd, p.tol, mf->nden, mf->nch,
                          mf->stream));
@@ -1981,7 +2019,14 @@ template <class T> static mfgpu_status mf_launch_xcorr(mfgpu_mf *mf)
     p.ticket = persist(mf->mode_x, mf->log2p) ? mf->tickets.as<int>() : nullptr;
     p.nblk = mf->nblocks;
     p.ntiles = mf->nblocks * mf->ngroups;
-    CU(launch_xcorr<T>(mf->log2p, mf->shared_den, mf->mode_x, p, mf->nblocks, mf->ngroups, mf->stream));
+    if constexpr (sizeof(T) == 8)
+    {
+        if (mf->intx)
+            CU(launch_int_xcorr(p, mf->shared_den, mf->int_B.as<int>(), mf->int_tw.as<int>(), mf->fLen, mf->n, mf->nblocks,
+                                mf->ngroups, mf->stream));
+    }
+    if (!mf->intx)
+        CU(launch_xcorr<T>(mf->log2p, mf->shared_den, mf->mode_x, p, mf->nblocks, mf->ngroups, mf->stream));
     ++mf->launches;
     // the other length buckets, one launch each
     for (auto &xb : mf->xb)

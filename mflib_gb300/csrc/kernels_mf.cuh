@@ -766,6 +766,47 @@ __device__ __forceinline__ bool xcorr_wait(uint64_t *bar, uint32_t parity, int *
     return true;
 }
 
+// Fused peak candidates of block bx (first lag k0) of template t: NTT threads
+// (ttid) read back the 64-lag chunks flagged in mk (MW words) from L2 and apply
+// the candidate rule to the lags whose neighbours both lie in the block.
+template <class T, int NTT, int MW>
+__device__ __forceinline__ void pk_scan(const XcorrParams<T> &p, const unsigned *mk, int t, int ttid, int bx, long k0)
+{
+    const int S = p.S;
+    const long pk_n = p.pk_len;
+    const T pk_thr = p.pk_thr;
+    const T *Rt = p.rho + (long) t * p.ldr + k0;
+    const long nv = p.nvalid[t];
+    const int kmax = (int) (nv - k0 < (long) S ? nv - k0 : (long) S);
+#pragma unroll 1
+    for (int w = 0; w < MW; ++w)
+    {
+        unsigned m = mk[w];
+        while (m)
+        {
+            const int c = 32 * w + __ffs(m) - 1;
+            m &= m - 1;
+            for (int l = 64 * c + ttid; l < 64 * c + 64; l += NTT)
+            {
+                if (l < 1 || l > S - 2 || k0 + l >= pk_n) continue;  // then also l < kmax
+                const T xi = __ldcg(Rt + l);
+                if (!(xi > pk_thr)) continue;
+                const T xr = l + 1 < kmax ? __ldcg(Rt + l + 1) : (T) 0;  // unused at the trace's last lag
+                if (cand_rule<T>(__ldcg(Rt + l - 1), xi, xr, k0 + l, pk_n, pk_thr))
+                {
+                    const long slot = (long) t * p.pk_stride + bx;
+                    const int pos = atomicAdd(p.pk_cnt + slot, 1);
+                    if (pos < kPkCap)
+                    {
+                        p.pk_idx[slot * kPkCap + pos] = (int) (k0 + l);
+                        p.pk_val[slot * kPkCap + pos] = xi;
+                    }
+                }
+            }
+        }
+    }
+}
+
 // ----------------------------------------------------------------------------
 // Fused overlap-save correlator: one CTA per (block, template group).
 // SHARED_DEN: every template has the same length, so the normalisation was
@@ -949,42 +990,8 @@ __device__ __forceinline__ int xcorr_tile(const XcorrParams<T> &p, const int bx,
     // in this block.  The block's first and last lags are decided from the
     // stored trace after the launch.
     const bool pk = p.pk_on != 0;
-    const long pk_n = p.pk_len;
     const T pk_thr = p.pk_thr;
     constexpr int MW = LY::mask_words;
-    auto pk_scan = [&](auto nt_tag, const unsigned *mk, int t, int ttid) {
-        constexpr int NTT = decltype(nt_tag)::value;
-        const T *Rt = p.rho + (long) t * p.ldr + k0;
-        const long nv = p.nvalid[t];
-        const int kmax = (int) (nv - k0 < (long) S ? nv - k0 : (long) S);
-#pragma unroll 1
-        for (int w = 0; w < MW; ++w)
-        {
-            unsigned m = mk[w];
-            while (m)
-            {
-                const int c = 32 * w + __ffs(m) - 1;
-                m &= m - 1;
-                for (int l = 64 * c + ttid; l < 64 * c + 64; l += NTT)
-                {
-                    if (l < 1 || l > S - 2 || k0 + l >= pk_n) continue;  // then also l < kmax
-                    const T xi = __ldcg(Rt + l);
-                    if (!(xi > pk_thr)) continue;
-                    const T xr = l + 1 < kmax ? __ldcg(Rt + l + 1) : (T) 0;  // unused at the trace's last lag
-                    if (cand_rule<T>(__ldcg(Rt + l - 1), xi, xr, k0 + l, pk_n, pk_thr))
-                    {
-                        const long slot = (long) t * p.pk_stride + bx;
-                        const int pos = atomicAdd(p.pk_cnt + slot, 1);
-                        if (pos < kPkCap)
-                        {
-                            p.pk_idx[slot * kPkCap + pos] = (int) (k0 + l);
-                            p.pk_val[slot * kPkCap + pos] = xi;
-                        }
-                    }
-                }
-            }
-        }
-    };
     auto template_body = [&](auto bar_tag, auto nt_tag, int j, const cx<T> *B, cx<T> *Wt, unsigned *mk, int ttid,
                              int bar_id, const T *invd_row) {
         constexpr int BAR = decltype(bar_tag)::value;
@@ -1042,7 +1049,7 @@ __device__ __forceinline__ int xcorr_tile(const XcorrParams<T> &p, const int bx,
                 team_sync<-1, kThreads>(bar_id);
                 if (pk)
                 {
-                    pk_scan(std::integral_constant<int, kThreads>(), mkt + ((it - 1) & 1) * MW, t_prev, ttid);
+                    pk_scan<T, kThreads, MW>(p, mkt + ((it - 1) & 1) * MW, t_prev, ttid, bx, k0);
                     if (ttid < MW) mkt[(it & 1) * MW + ttid] = 0u;
                 }
             }
@@ -1061,7 +1068,7 @@ __device__ __forceinline__ int xcorr_tile(const XcorrParams<T> &p, const int bx,
         if (pk && it > 0)
         {
             team_sync<-1, kThreads>(bar_id);
-            pk_scan(std::integral_constant<int, kThreads>(), mkt + ((it - 1) & 1) * MW, t_prev, ttid);
+            pk_scan<T, kThreads, MW>(p, mkt + ((it - 1) & 1) * MW, t_prev, ttid, bx, k0);
         }
     }
     else if constexpr (TEAMS)
@@ -1082,7 +1089,7 @@ __device__ __forceinline__ int xcorr_tile(const XcorrParams<T> &p, const int bx,
                 team_sync<-1, 128>(bar_id);
                 if (pk)
                 {
-                    pk_scan(std::integral_constant<int, 128>(), mkt + ((it - 1) & 1) * MW, t_prev, ttid);
+                    pk_scan<T, 128, MW>(p, mkt + ((it - 1) & 1) * MW, t_prev, ttid, bx, k0);
                     if (ttid < MW) mkt[(it & 1) * MW + ttid] = 0u;
                 }
             }
@@ -1093,7 +1100,7 @@ __device__ __forceinline__ int xcorr_tile(const XcorrParams<T> &p, const int bx,
         if (pk && it > 0)
         {
             team_sync<-1, 128>(bar_id);
-            pk_scan(std::integral_constant<int, 128>(), mkt + ((it - 1) & 1) * MW, t_prev, ttid);
+            pk_scan<T, 128, MW>(p, mkt + ((it - 1) & 1) * MW, t_prev, ttid, bx, k0);
         }
     }
     else
@@ -1107,8 +1114,7 @@ __device__ __forceinline__ int xcorr_tile(const XcorrParams<T> &p, const int bx,
                 __syncthreads();  // previous template finished reading W and its spectrum buffer
                 if (pk)
                 {
-                    pk_scan(std::integral_constant<int, kThreads>(), Mk + ((j - 1) & 1) * MW,
-                            p.tids[t_begin + j - 1], tid);
+                    pk_scan<T, kThreads, MW>(p, Mk + ((j - 1) & 1) * MW, p.tids[t_begin + j - 1], tid, bx, k0);
                     if (tid < MW) Mk[(j & 1) * MW + tid] = 0u;
                 }
             }
@@ -1152,7 +1158,7 @@ __device__ __forceinline__ int xcorr_tile(const XcorrParams<T> &p, const int bx,
         if (pk)
         {
             __syncthreads();
-            pk_scan(std::integral_constant<int, kThreads>(), Mk + ((ntl - 1) & 1) * MW, p.tids[t_end - 1], tid);
+            pk_scan<T, kThreads, MW>(p, Mk + ((ntl - 1) & 1) * MW, p.tids[t_end - 1], tid, bx, k0);
         }
     }
     return 1;

@@ -11,6 +11,7 @@
 #include "kernels_util.cuh"
 #include "tc_params.h"
 #include "fix_params.h"
+#include "int_params.h"
 #include "mfgpu.h"
 
 namespace mfgpu {
@@ -41,6 +42,15 @@ template <class T> void twiddle_split(int log2p, std::vector<cx<T>> &out);
 // (optional) receives max - min per channel
 template <class T> cudaError_t launch_dead(const T *x, long ldx, int nch, long n, unsigned char *dead, T *pmin,
                                            T *pmax, int nchunks, cudaStream_t s, float *range = nullptr);
+// FP64 correlator in integer arithmetic (kernels_int.cuh): twiddles to upload,
+// template table (4 x kIntN words per template), normalisation (rows per
+// channel, or per template in rho), correlator over blocks of x.S lags
+const std::vector<int> &int_twiddles();
+cudaError_t launch_int_bank(const double *tmpl, const long *toff, const int *tlen, int nt, const int *tw, int *B,
+                            cudaStream_t s);
+cudaError_t launch_int_den(const IntDenParams &p, bool multi, int ntiles, int ngroups, cudaStream_t s);
+cudaError_t launch_int_xcorr(const XcorrParams<double> &x, bool shared_den, const int *B, const int *tw, int Lmax, long n,
+                             int nblocks, int ngroups, cudaStream_t s);
 // tensor-core correlator (FP32, one template length): shared memory per CTA,
 // the template bank in MMA layout (ngroups * Gp slots), the persistent launch
 size_t tc_smem_bytes(int Kp, int Gp);

@@ -483,8 +483,9 @@ class MatchedFilter:
     # -- extensions ---------------------------------------------------------
     def get_plan(self):
         """The plan chosen at initialize: FFT length, lags per block, blocks,
-        and the correlator (1-3, 5 FFT organisations, 4 tensor cores; for the
-        latter also the templates per group and the padded K)."""
+        and the correlator (1-3, 5, 6 FFT organisations, 4 tensor cores, 7
+        integer transforms for FP64 data; for the tensor cores also the
+        templates per group and the padded K)."""
         a, b, c = C.c_int(), C.c_int(), C.c_int()
         _lib.call("mfgpu_mf_get_plan", self._h, C.byref(a), C.byref(b), C.byref(c))
         v, g, k = C.c_int(), C.c_int(), C.c_int()
@@ -578,8 +579,9 @@ class MatchedFilter:
                 if ms is None:
                     continue
                 plans = [(bp["fft_length"], bp["correlator"]) for bp in self.get_plan()["bucket_plans"]]
-                if any(v == 4 for _, v in plans):
-                    plans = [(0, 0)] * len(plans)  # the automatic choice took the tensor cores: tune the FFT plans
+                if any(v in (4, 7) for _, v in plans):
+                    # the automatic choice took the tensor cores or (FP64) the integer correlator: tune the FFT plans
+                    plans = [(0, 0)] * len(plans)
                 cur_ms, cur = ms, plans
                 for b in range(len(plans)):
                     f0 = plans[b][0] if plans[b][0] > 0 else self.get_plan()["fft_length"]

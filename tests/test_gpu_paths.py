@@ -70,3 +70,85 @@ def test_prune_per_trace(gpu, oracle, rng, dtype, thr, dist, fused):
         for t in range(len(lens)):
             ref = oracle.peaks(f.get_matched_filtered_signal(t).astype(np.float64), thr, dist)
             np.testing.assert_array_equal(f.get_peaks(t), ref)
+
+
+def _pearson(tp, z):
+    """Two-pass Pearson coefficients and window 2-norms about the mean, each
+    window taken relative to its first sample (so that a small deviation on a
+    large level keeps its digits)."""
+    b = tp - tp.mean()
+    b /= np.linalg.norm(b)
+    w = np.lib.stride_tricks.sliding_window_view(z, tp.size)
+    rho, norm = np.empty(w.shape[0]), np.empty(w.shape[0])
+    for i in range(0, w.shape[0], 2048):
+        d = w[i:i + 2048] - w[i:i + 2048, :1]
+        d -= d.mean(axis=1, keepdims=True)
+        norm[i:i + 2048] = np.sqrt((d * d).sum(axis=1))
+        rho[i:i + 2048] = (d @ b) / norm[i:i + 2048]
+    return rho, norm
+
+
+# FP64 in integer arithmetic: the longest and shortest templates, block and
+# tile edges (a last block of one lag), several lengths and one, offsets and
+# scales near the ends of the FP64 range.  Bound: that of the reference's own
+# tests (1e-13; the two-pass sums it is compared with err by about L 2^-53)
+# plus, against the window's own deviation, the samples' rounding (at most
+# 2^-50 of the signal's largest deviation each) and the rounding of the
+# template's mean (its demeaned samples sum to up to L 2^-52 of it, times the
+# window's level).
+@pytest.mark.parametrize("lens,n", [((2,), 4097), ((500,), 3585 + 499), ((500,) * 3, 3584 + 499), ((31, 32, 33, 200), 9000),
+                                    ((4065,), 4065), ((4065, 4064, 64), 8193 + 32), ((1000,) * 21, 16_385),
+                                    ((2801, 700, 1500, 700), 20_000)])
+@pytest.mark.parametrize("scale,offset", [(1.0, 0.0), (3e-2, 4e4), (1e-150, 0.0), (1e150, -1e150)])
+def test_integer_correlator(gpu, oracle, rng, lens, n, scale, offset):
+    x = rng.standard_normal((2, n))
+    x[1] *= np.where(np.arange(n) < n // 2, 1.0, 40.0)
+    tps = [rng.standard_normal(L) for L in lens]
+    chan = [t % 2 for t in range(len(lens))]
+    f = _filter(gpu, tps, chan, 2, n, np.float64)
+    assert f.get_plan()["correlator"] == 7
+    f.set_channel_signals(x * scale + offset)
+    f.apply()
+    if scale < 1e-100:
+        # deviations below the normalisation's floor of 1e-12: coefficients
+        # are the numerators over it
+        assert all(np.max(np.abs(f.get_valid_matched_filtered_signal(t))) < 1e-130 for t in range(len(tps)))
+        return
+    # the coefficients do not depend on scale and offset; the reference is
+    # taken on the samples as rounded, moved back to the middle of the range
+    y = (x * scale + offset - offset) / scale if abs(scale) < 1e100 else x * scale / 1e150 + offset / 1e150
+    tol = 1e-13 if abs(offset) <= scale * 1e3 else 1e-9  # digits the samples lost to the offset
+    for t, tp in enumerate(tps):
+        z = y[chan[t]]
+        ref, norm = _pearson(tp, z)
+        off = tp.size * 2.0 ** -52 * abs(tp.mean()) / np.linalg.norm(tp - tp.mean())
+        bound = tol + (np.sqrt(tp.size) * 2.0 ** -50 + off) * np.max(np.abs(z - z.mean())) / norm
+        err = np.abs(f.get_valid_matched_filtered_signal(t) - ref)
+        assert np.all(err < bound), float(np.max(err / bound))
+
+
+def test_integer_correlator_special_values(gpu, oracle, rng):
+    n, L = 30_000, 300
+    x = rng.standard_normal((3, n))
+    x[0, 10_000] = np.nan
+    x[1, 20_000] = -np.inf
+    x[2, 9_000:15_000] = 7.25  # constant windows: 0
+    tp = rng.standard_normal(L)
+    f = _filter(gpu, [tp] * 3, [0, 1, 2], 3, n, np.float64)
+    f.set_channel_signals(x)
+    f.apply()
+    S = f.get_plan()["lags_per_block"]
+    for c, at in ((0, 10_000), (1, 20_000)):
+        r = f.get_valid_matched_filtered_signal(c)
+        assert np.all(np.isnan(r[at - L + 1:at + 1]))  # every window that holds it
+        clean = np.where(np.isfinite(x[c]), x[c], 0.0)
+        ref = oracle.pearson_naive(tp, clean)
+        b = np.arange(r.size) // S * S
+        far = (at < b) | (at >= b + 4096)  # blocks that do not read it
+        assert np.max(np.abs(r[far] - ref[far])) < 1e-13
+    r = f.get_valid_matched_filtered_signal(2)
+    assert np.all(r[9_000:15_000 - L + 1] == 0.0)
+    ref = oracle.pearson_naive(tp, x[2])
+    keep = np.ones(r.size, bool)
+    keep[9_000:15_000 - L + 1] = False
+    assert np.max(np.abs(r[keep] - ref[keep])) < 1e-13
