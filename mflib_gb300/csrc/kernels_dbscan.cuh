@@ -406,4 +406,222 @@ static __global__ void db_count_kernel(int nseg, const int *seg_off, const long 
     n_clusters[s] = (int) (root_pos[seg_off[s + 1]] - root_pos[seg_off[s]]);
 }
 
+// ----------------------------------------------------------------------------
+// One feature, segments of at most kDb1Cap points: one CTA does a segment in
+// shared memory, from its unsorted points to its labels.  Sorted by (value,
+// index) with NaN last, a point's neighbourhood is a range of positions; the
+// clusters are the runs of consecutive core points with gaps of at most eps,
+// numbered by their lowest point index.  One launch between one upload and
+// one read-back, where the sort on the host, nine uploads, nine launches and
+// the scans took 465 of the 535 us of an association (9,500 points in 8
+// segments; now 106 us in all).  Larger segments keep the launches above.
+constexpr int kDb1Cap = 8192, kDb1Threads = 1024;
+__host__ __device__ constexpr size_t db1_bytes(int n2) { return (sizeof(double) + 3 * sizeof(int)) * (size_t) n2; }
+
+// exclusive scan over the CTA of one value per thread (sum or maximum);
+// sh: 33 ints; the total goes to *total
+template <bool MAX> __device__ __forceinline__ int db1_scan(int v, int *sh, int *total)
+{
+    constexpr int none = MAX ? -1 : 0;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    int x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1)
+    {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x = MAX ? max(x, y) : x + y;
+    }
+    __syncthreads();
+    if (lane == 31) sh[w] = x;
+    __syncthreads();
+    int before = none, all = none;
+    for (int i = 0; i < kDb1Threads / 32; ++i)
+    {
+        const int t = sh[i];
+        if (i < w) before = MAX ? max(before, t) : before + t;
+        all = MAX ? max(all, t) : all + t;
+    }
+    *total = all;
+    int e = __shfl_up_sync(0xffffffffu, x, 1);
+    if (lane == 0) e = none;
+    return MAX ? max(before, e) : before + e;
+}
+
+static __global__ void __launch_bounds__(kDb1Threads) db1_segment_kernel(const double *X, const double *wt,
+                                                                        const int *seg_off, int n2max, double eps,
+                                                                        double min_obs, int *labels, int *n_clusters)
+{
+    extern __shared__ __align__(16) unsigned char smem_db[];
+    __shared__ int sh[33];
+    unsigned long long *key = reinterpret_cast<unsigned long long *>(smem_db);
+    double *xs = reinterpret_cast<double *>(smem_db);  // the sorted values, over the keys
+    int *idx = reinterpret_cast<int *>(key + n2max);   // point of each position
+    int *run = idx + n2max;                            // run of each position (-1: not core)
+    int *aux = run + n2max;                            // per run, then per point
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, s = blockIdx.x;
+    const int b = seg_off[s], n = seg_off[s + 1] - b;
+    if (n <= 0)
+    {
+        if (tid == 0) n_clusters[s] = 0;
+        return;
+    }
+    int n2 = 1;
+    while (n2 < n) n2 <<= 1;
+    // ---- sort: order-preserving integer keys (-0 as +0), NaN and padding last
+    for (int i = tid; i < n2; i += kDb1Threads)
+    {
+        unsigned long long k = ~0ull;
+        if (i < n)
+        {
+            const double v = X[b + i] + 0.0;
+            const long long u = __double_as_longlong(v);
+            if (!isnan(v)) k = u < 0 ? ~(unsigned long long) u : (unsigned long long) u | (1ull << 63);
+        }
+        key[i] = k;
+        idx[i] = i;
+    }
+    __syncthreads();
+    for (int k = 2; k <= n2; k <<= 1)
+        for (int j = k >> 1; j > 0; j >>= 1)
+        {
+            for (int i = tid; i < n2 / 2; i += kDb1Threads)
+            {
+                const int p = 2 * i - (i & (j - 1)), q = p + j;
+                const unsigned long long ka = key[p], kb = key[q];
+                const int ia = idx[p], ib = idx[q];
+                const bool gt = ka > kb || (ka == kb && ia > ib);
+                if (gt == ((p & k) == 0))
+                {
+                    key[p] = kb;
+                    key[q] = ka;
+                    idx[p] = ib;
+                    idx[q] = ia;
+                }
+            }
+            __syncthreads();
+        }
+    // ---- values in place; nv: points that are no NaN
+    int mine = 0;
+    for (int i = tid; i < n; i += kDb1Threads)
+    {
+        const unsigned long long k = key[i];
+        if (k != ~0ull)
+        {
+            ++mine;
+            xs[i] = __longlong_as_double((long long) (k >> 63 ? k & ~(1ull << 63) : ~k));
+        }
+    }
+    int nv;
+    db1_scan<false>(mine, sh, &nv);
+    __syncthreads();
+    // ---- core points (weights summed as db1_core_kernel does)
+    if (!wt)
+    {
+        for (int r = tid; r < nv; r += kDb1Threads)
+        {
+            int lo, hi;
+            db1_range(xs, 0, nv, xs[r], eps, lo, hi);
+            run[r] = (double) (hi > lo ? hi - lo : 0) >= min_obs ? 0 : -1;
+        }
+    }
+    else
+    {
+        for (int r = w; r < nv; r += kDb1Threads / 32)
+        {
+            int lo, hi;
+            db1_range(xs, 0, nv, xs[r], eps, lo, hi);
+            double acc = 0;
+            for (int i = lo + lane; i < hi; i += 32) acc += wt[b + idx[i]];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+            if (lane == 0) run[r] = acc >= min_obs ? 0 : -1;
+        }
+    }
+    __syncthreads();
+    // ---- runs: each thread a piece of consecutive positions
+    const int per = (nv + kDb1Threads - 1) / kDb1Threads, r0 = min(nv, tid * per), r1 = min(nv, r0 + per);
+    int last = -1, tot;
+    for (int r = r0; r < r1; ++r)
+        if (run[r] == 0) last = r;
+    int prev = db1_scan<true>(last, sh, &tot);  // nearest core position before the piece
+    const int prev0 = prev;
+    int starts = 0;
+    for (int r = r0; r < r1; ++r)
+        if (run[r] == 0)
+        {
+            if (prev < 0 || !(xs[r] - xs[prev] <= eps)) ++starts;
+            prev = r;
+        }
+    int nrun;
+    int id = db1_scan<false>(starts, sh, &nrun) - 1;  // the run the piece begins in
+    prev = prev0;
+    for (int r = r0; r < r1; ++r)
+        if (run[r] == 0)
+        {
+            if (prev < 0 || !(xs[r] - xs[prev] <= eps)) ++id;
+            prev = r;
+            run[r] = id;
+        }
+    for (int i = tid; i < nrun; i += kDb1Threads) aux[i] = n;
+    __syncthreads();
+    for (int r = tid; r < nv; r += kDb1Threads)
+        if (run[r] >= 0) atomicMin(aux + run[r], idx[r]);
+    __syncthreads();
+    // ---- cluster number of a run: how many runs have a lower first point.
+    // The first points in index order, by a scan over marks
+    int root[kDb1Cap / kDb1Threads];
+#pragma unroll
+    for (int u = 0; u < kDb1Cap / kDb1Threads; ++u)
+    {
+        const int i = tid + u * kDb1Threads;
+        root[u] = i < nrun ? aux[i] : -1;
+    }
+    __syncthreads();
+    for (int i = tid; i < n; i += kDb1Threads) aux[i] = 0;
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < kDb1Cap / kDb1Threads; ++u)
+        if (root[u] >= 0) aux[root[u]] = 1;
+    __syncthreads();
+    const int pern = (n + kDb1Threads - 1) / kDb1Threads, i0 = min(n, tid * pern), i1 = min(n, i0 + pern);
+    int marks = 0;
+    for (int i = i0; i < i1; ++i) marks += aux[i];
+    int base = db1_scan<false>(marks, sh, &tot);
+    for (int i = i0; i < i1; ++i)
+    {
+        const int m = aux[i];
+        aux[i] = base;
+        base += m;
+    }
+    __syncthreads();
+    int num[kDb1Cap / kDb1Threads];
+#pragma unroll
+    for (int u = 0; u < kDb1Cap / kDb1Threads; ++u) num[u] = root[u] >= 0 ? aux[root[u]] : 0;
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < kDb1Cap / kDb1Threads; ++u)
+        if (root[u] >= 0) aux[tid + u * kDb1Threads] = num[u];
+    __syncthreads();
+    // ---- labels: a core point's run; else the lowest cluster among the core neighbours
+    for (int r = tid; r < n; r += kDb1Threads)
+    {
+        int lab = -1;
+        if (r < nv)
+        {
+            if (run[r] >= 0) lab = aux[run[r]];
+            else
+            {
+                int lo, hi;
+                db1_range(xs, 0, nv, xs[r], eps, lo, hi);
+                int best = n;
+                for (int i = nrun > 0 ? lo : hi; i < hi; ++i)
+                    if (run[i] >= 0) best = min(best, aux[run[i]]);
+                if (best < n) lab = best;
+            }
+        }
+        labels[b + idx[r]] = lab;
+    }
+    if (tid == 0) n_clusters[s] = nrun;
+}
+
 }  // namespace mfgpu

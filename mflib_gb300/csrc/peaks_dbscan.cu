@@ -266,6 +266,34 @@ int run_dbscan(int n, int nf, const double *X, const double *w, double eps, int 
         for (int i = 0; i < nseg; ++i) nclusters_host[i] = 0;
         return 0;
     }
+    int most = 0;
+    for (int sg = 0; sg < nseg; ++sg) most = std::max(most, seg_off_host[sg + 1] - seg_off_host[sg]);
+    if (nf == 1 && most <= kDb1Cap)
+    {
+        // one CTA per segment: points (and weights) up, labels and counts down
+        int n2 = 1;
+        while (n2 < most) n2 <<= 1;
+        MF_TRY(ws.X.ensure(sizeof(double) * (size_t) n * (w ? 2 : 1)));
+        MF_TRY(ws.seg_off.ensure(sizeof(int) * (size_t) (nseg + 1)));
+        MF_TRY(ws.labels.ensure(sizeof(int) * (size_t) (n + nseg)));
+        double *wd = w ? ws.X.as<double>() + n : nullptr;
+        int *lab = ws.labels.as<int>();
+        MF_TRY(cudaMemcpyAsync(ws.X.p, X, sizeof(double) * (size_t) n, cudaMemcpyHostToDevice, s));
+        if (w) MF_TRY(cudaMemcpyAsync(wd, w, sizeof(double) * (size_t) n, cudaMemcpyHostToDevice, s));
+        MF_TRY(cudaMemcpyAsync(ws.seg_off.p, seg_off_host, sizeof(int) * (size_t) (nseg + 1), cudaMemcpyHostToDevice, s));
+        static SmemCap cap;
+        MF_TRY(raise_smem_cap(db1_segment_kernel, db1_bytes(n2), cap));
+        db1_segment_kernel<<<nseg, kDb1Threads, db1_bytes(n2), s>>>(ws.X.as<double>(), wd, ws.seg_off.as<int>(), n2, eps,
+                                                                  (double) min_obs, lab, lab + n);
+        ++*launches;
+        MF_TRY(cudaGetLastError());
+        std::vector<int> got((size_t) n + nseg);
+        MF_TRY(cudaMemcpyAsync(got.data(), lab, sizeof(int) * got.size(), cudaMemcpyDeviceToHost, s));
+        MF_TRY(cudaStreamSynchronize(s));
+        std::copy(got.begin(), got.begin() + n, labels_host);
+        std::copy(got.begin() + n, got.end(), nclusters_host);
+        return 0;
+    }
     MF_TRY(ws.X.ensure(sizeof(double) * (size_t) n * nf));
     MF_TRY(ws.w.ensure(sizeof(double) * (size_t) n));
     MF_TRY(ws.seg_of.ensure(sizeof(int) * (size_t) n));

@@ -152,3 +152,31 @@ def test_integer_correlator_special_values(gpu, oracle, rng):
     keep = np.ones(r.size, bool)
     keep[9_000:15_000 - L + 1] = False
     assert np.max(np.abs(r[keep] - ref[keep])) < 1e-13
+
+
+# association segments in one CTA each: sizes around the powers of two of the
+# sorting network, up to the largest one CTA takes and one above it (the
+# general launches), empty segments, ties, NaN, infinities, both zeros
+@pytest.mark.parametrize("sizes", [(1, 2, 3, 0, 4, 5), (31, 32, 33, 1023, 1024, 1025), (8192, 8191, 7), (8193, 20)])
+@pytest.mark.parametrize("weighted", [False, True])
+def test_segment_clustering(gpu, oracle, rng, sizes, weighted):
+    off = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int32)
+    x = np.round(rng.uniform(-off[-1] / 8, off[-1] / 8, off[-1]) * 4) / 4
+    x[::37] = -0.0
+    x[1::53] = np.inf
+    x[2::59] = -np.inf
+    if max(sizes) <= 8192:
+        x[3::61] = np.nan
+    w = rng.integers(1, 7, x.size) / 2.0 if weighted else None
+    db = gpu.DBSCAN()
+    for eps, mo in ((0.0, 1), (0.25, 3), (0.75, 6)):
+        db.initialize(eps, mo)
+        labels, ncl = db.cluster_segments(x, off, w)
+        for s in range(len(sizes)):
+            a, b = off[s], off[s + 1]
+            if a == b:
+                assert ncl[s] == 0
+                continue
+            n_ref, ref = oracle.dbscan(x[a:b], eps, mo, None if w is None else w[a:b])
+            assert ncl[s] == n_ref
+            np.testing.assert_array_equal(labels[a:b], ref)
