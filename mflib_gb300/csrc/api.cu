@@ -1112,14 +1112,14 @@ try
     mfgpu_status s2 = MFGPU_OK;
     if (mf->intx)
     {
-        const std::vector<int> &tw = int_twiddles();
+        const std::vector<unsigned> &tw = int_twiddles();
         CU(mf->int_tw.ensure(sizeof(int) * tw.size()));
         CU(cudaMemcpyAsync(mf->int_tw.p, tw.data(), sizeof(int) * tw.size(), cudaMemcpyHostToDevice, mf->stream));
         CU(mf->int_B.ensure(sizeof(int) * (size_t) nt * kIntPrimes * kIntN));
-        mf->int_lags = ((kIntTile - maxLen) / 32) * 32;
+        mf->int_lags = ((int_tile(maxLen) - maxLen) / 32) * 32;
         mf->int_tiles = (std::max(1, maxvalid_f) + mf->int_lags - 1) / mf->int_lags;
         CU(launch_int_bank(mf->tmpl_d.as<double>(), mf->toff_d.as<long>(), mf->tlen_d.as<int>(), nt,
-                           mf->int_tw.as<int>(), mf->int_B.as<int>(), mf->stream));
+                           mf->int_tw.as<unsigned>(), mf->int_B.as<unsigned>(), mf->stream));
         ++mf->launches;
     }
     else
@@ -1937,10 +1937,11 @@ template <class T> static mfgpu_status mf_launch_xcorr(mfgpu_mf *mf)
         {
             IntDenParams d{};
             d.x = p.x; d.ldx = p.ldx; d.n = mf->n; d.dead = p.dead; d.tol = p.tol; d.lags = mf->int_lags;
+            d.scale = int_numerator_scale() * (mf->shared_den ? std::sqrt((double) mf->fLen) : 1.0);
             d.L = mf->fLen; d.nv = mf->n - mf->fLen + 1; d.den = mf->den.as<double>(); d.ldd = p.ldd;
             d.grp_chan = p.grp_chan; d.grp_tb = p.grp_tb; d.grp_te = p.grp_te; d.tids = p.tids;
             d.tlen = p.tlen; d.nvalid = p.nvalid; d.rho = p.rho; d.ldr = p.ldr;
-            CU(launch_int_den(d, !mf->shared_den, mf->int_tiles, mf->shared_den ? mf->nch : mf->ngroups, mf->stream));
+            CU(launch_int_den(d, !mf->shared_den, int_tile(mf->fLen), mf->int_tiles, mf->shared_den ? mf->nch : mf->ngroups, mf->stream));
             ++mf->launches;
         }
     if (mf->shared_den && !mf->intx && !(sizeof(T) == 4 && mf->fx_on))
@@ -2022,7 +2023,7 @@ template <class T> static mfgpu_status mf_launch_xcorr(mfgpu_mf *mf)
     if constexpr (sizeof(T) == 8)
     {
         if (mf->intx)
-            CU(launch_int_xcorr(p, mf->shared_den, mf->int_B.as<int>(), mf->int_tw.as<int>(), mf->fLen, mf->n, mf->nblocks,
+            CU(launch_int_xcorr(p, mf->shared_den, mf->int_B.as<unsigned>(), mf->int_tw.as<unsigned>(), mf->fLen, mf->n, mf->nblocks,
                                 mf->ngroups, mf->stream));
     }
     if (!mf->intx)

@@ -8,26 +8,28 @@ constexpr int kIntN = 4096;       // transform length: the samples of a block
 constexpr int kIntPrimes = 4;
 constexpr int kIntThreads = 1024;
 constexpr int kIntTw = 240 + 3840;  // twiddles per prime: rows r = 1 .. 15 of the second and third pass
-constexpr int kIntTile = 8192;    // samples of a normalisation tile
+// samples of a normalisation tile for templates of up to L samples
+constexpr int int_tile(int L) { return L <= 1024 ? 4096 : 8192; }
 constexpr int kIntXBits = 50;     // bits of a quantised sample of a normalisation tile
 constexpr int kIntBBits = 53;     // fraction bits of a template coefficient
-constexpr float kIntNormBits = 54.6f;  // a block's windows: 2-norm below 2^54.6, so that a numerator stays below
-                                       // 2^107.6 and half the primes' product (2^107.7)
+constexpr float kIntNormBits = 55.1f;  // a block's windows: 2-norm below 2^55.1, so that a numerator stays below
+                                       // 2^108.1 and half the primes' product (2^108.19)
 
-// One prime: everything but p and nq is times R = 2^32 modulo p, centred.
+// One prime: c25, rrn and crt are times R = 2^32 modulo p; all in [0, p).
 struct IntPrime
 {
-    int p, nq;                      // nq = -p^-1 mod 2^32
-    int one;                        // 1
-    int w1, w2, w3, w4, w6, w9;     // powers of the 16th root
-    int c25;                        // 2^25
-    int rrn;                        // R / N (so that a product with it gives a value times R / N)
+    unsigned p, nq;                 // nq = -p^-1 mod 2^32
+    unsigned p2, p4, p8, p16;       // multiples of p
+    unsigned inv;                   // floor(2^32 / p)
+    unsigned w[10], ws[10];         // powers of the 16th root, floor(w 2^32 / p)
+    unsigned c25;                   // 2^25
+    unsigned rrn;                   // R / N (a product with it gives a value times R / N)
+    unsigned crt;                   // (M / p)^-1, M the product of the primes
+    unsigned f0, f1, f2;            // floor(2^96 / p), low word first
 };
 struct IntConsts
 {
     IntPrime prime[kIntPrimes];
-    int i01, i02, i12, i03, i13, i23;  // inverse of prime a modulo prime b, times R
-    unsigned long long p01;            // product of the first two primes
 };
 
 struct IntBankParams
@@ -35,8 +37,8 @@ struct IntBankParams
     const double *tmpl;
     const long *toff;
     const int *tlen;
-    int *B;                         // [template][prime][kIntN]
-    const int *tw;                  // [prime][kIntTw]
+    unsigned *B;                    // [template][prime][kIntN]
+    const unsigned *tw;             // [prime][kIntTw]
     IntConsts c;
 };
 
@@ -47,6 +49,8 @@ struct IntDenParams
     long n;                         // samples per row
     const unsigned char *dead;
     double tol;
+    double scale;                   // factor of the correlator's numerators (int_numerator_scale);
+                                    // one length: times sqrt(L)
     int lags;                       // lags per tile
     // one length: L, valid lags, rows den
     int L;

@@ -4,37 +4,40 @@
 // 32x32 -> 64-bit integer multiply-adds and 110 integer additions, so FP64
 // data are correlated without the FP64 pipe:
 //
-//   * A block of N = 4096 samples becomes integers X of up to 54 bits: each
+//   * A block of N = 4096 samples becomes integers X of up to 55 bits: each
 //     sample's significand shifted to a common exponent (62 bits, exact for
 //     samples within 2^9 of the largest), the block's mean level taken off
 //     (the numerator does not depend on it, templates are zero-mean), the
 //     result rounded once.  The unit is the finest at which every window's
-//     2-norm stays below 2^54.6 (about 2^-52 of the largest deviation for a
+//     2-norm stays below 2^55.1 (about 2^-53 of the largest deviation for a
 //     seismogram).  Template coefficients (demeaned, unit norm) become
 //     integers B = round(b 2^53).
 //   * The numerators sum X[k + j] B[j] are then computed exactly: cyclic
 //     correlation by number-theoretic transforms of N points modulo four
-//     primes p = 1 mod 8192 just below 2^31 / 14, and the Chinese remainder
-//     theorem.  |numerator| <= 2^54.6 2^53 stays below half the primes' product
-//     (2^107.7) by Cauchy-Schwarz.
+//     primes p = 1 mod 8192 just below 2^32 / 26, and the Chinese remainder
+//     theorem.  |numerator| <= 2^55.1 2^53 stays below half the primes' product
+//     (2^108.19) by Cauchy-Schwarz.
 //   * Window variances come from prefix sums of X (50 bits, sums 64) and X^2
 //     (sums 128 bits) of a tile: V = L S2 - S1^2 is exact.  1 / sqrt(V) starts from the
 //     FP32 reciprocal square root and takes one third-order step in 60-bit
 //     fixed point.
+//   * The Chinese remainder theorem as a sum of fractions, numerator / M = sum
+//     y_i / p_i modulo 1 (M the product of the primes), in 96-bit fixed point:
+//     the numerator to 2^-64 of M.
 //
 // The remaining errors are the two roundings of the inputs and three roundings
 // to FP64 at the end: below those of an FP64 transform, whose rounding grows
 // with the block's energy and log N (relative errors of the coefficients of
 // band-passed templates of 200 .. 2,000 samples against two-pass sums in
-// quadruple precision: 5.9e-16 .. 7.6e-16, FP64 transforms 7.8e-16 ..
+// quadruple precision: 3.7e-16 .. 5.7e-16, FP64 transforms 7.8e-16 ..
 // 1.75e-15).
 //
-// Arithmetic modulo p: signed Montgomery products with R = 2^32 (three
-// instructions: wide multiply, low multiply, wide multiply-add), whose result
-// is at most |a b| / 2^32 + p / 2 in magnitude.  With constants |b| <= p / 2
-// and |a| < 2^31 that is at most 0.75 p, so a 16-point transform of such
-// values, additions only between the products, stays within 12 p < 2^31:
-// no reduction is needed inside a pass.
+// Arithmetic modulo p: Montgomery products with R = 2^32 on unsigned words
+// (wide multiply, low multiply, wide multiply-add; the signed forms cost two
+// more instructions each), whose result is below p (1 + a / 2^32) < 2 p for any
+// 32-bit a and a constant b < p.  A 16-point transform of values below 2 p,
+// with multiples of p added to keep differences positive, stays below 26 p <
+// 2^32 with one reduction of one value inside.
 #pragma once
 #include "kernels_mf.cuh"
 #include "int_params.h"
@@ -44,62 +47,78 @@ namespace mfgpu {
 struct IntParams
 {
     XcorrParams<double> x;  // as the FFT correlator's (spectra and twiddles unused)
-    const int *B;           // [template][prime][kIntN]
-    const int *tw;          // [prime][kIntTw]
+    const unsigned *B;      // [template][prime][kIntN]
+    const unsigned *tw;     // [prime][kIntTw]
     int Lmax;               // longest template
     long n;                 // samples per row
     IntConsts c;
 };
 
-// a b R^-1 mod p (nq = -p^-1 mod 2^32)
-__device__ __forceinline__ int mont(int a, int b, int p, int nq)
+// a b R^-1 mod p, below p (1 + a / 2^32) for b < p (nq = -p^-1 mod 2^32)
+__device__ __forceinline__ unsigned mont(unsigned a, unsigned b, unsigned p, unsigned nq)
 {
-    long long t, r;
-    int m;
-    asm("mul.wide.s32 %0, %1, %2;" : "=l"(t) : "r"(a), "r"(b));
-    m = (int) t * nq;
-    asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(r) : "r"(m), "r"(p), "l"(t));
-    return (int) (r >> 32);
+    const unsigned long long t = (unsigned long long) a * b;
+    const unsigned m = (unsigned) t * nq;
+    return (unsigned) ((t + (unsigned long long) m * p) >> 32);
 }
 
-// the constants of one prime, in registers
+// a w mod p for a constant w with ws = floor(w 2^32 / p): below 2 p for any
+// 32-bit a.  One wide and two low multiplies where mont takes two wide and one
+// low (a wide one occupies the integer multiplier twice as long).
+__device__ __forceinline__ unsigned shoup(unsigned a, unsigned w, unsigned ws, unsigned p)
+{
+    return a * w - __umulhi(a, ws) * p;
+}
+
+// The constants of one prime.  `c` is the same for all threads of a warp: the
+// fields are read from the kernel parameters where they are used.
 struct IntField
 {
-    int p, nq, one, w1, w2, w3, w4, w6, w9;
-    __device__ __forceinline__ explicit IntField(const IntPrime &c)
-        : p(c.p), nq(c.nq), one(c.one), w1(c.w1), w2(c.w2), w3(c.w3), w4(c.w4), w6(c.w6), w9(c.w9)
-    {
-    }
-    __device__ __forceinline__ int mul(int a, int b) const { return mont(a, b, p, nq); }
+    const IntPrime &c;
+    __device__ __forceinline__ explicit IntField(const IntPrime &cc) : c(cc) {}
+    __device__ __forceinline__ unsigned mul(unsigned a, unsigned b) const { return mont(a, b, c.p, c.nq); }
+    template <int K> __device__ __forceinline__ unsigned root(unsigned a) const { return shoup(a, c.w[K], c.ws[K], c.p); }
+    // a mod p, below 2 p
+    __device__ __forceinline__ unsigned reduce(unsigned a) const { return a - __umulhi(a, c.inv) * c.p; }
 };
 
-__device__ __forceinline__ void int_dft4(const IntField &f, int &a0, int &a1, int &a2, int &a3)
+// 4-point transform.  MB = 2: a0 below 8 p, the others below 2 p, outputs below
+// 14 p (8 p if a0 is below 2 p); MB = 8: a0 below 2 p, the others below 8 p,
+// outputs below 26 p.  The multiples of p are parameters of their own, so that
+// the offsets are additions.
+template <int MB>
+__device__ __forceinline__ void int_dft4(const IntField &f, unsigned &a0, unsigned &a1, unsigned &a2, unsigned &a3)
 {
-    const int s0 = a0 + a2, d0 = a0 - a2, s1 = a1 + a3, d1 = f.mul(a1 - a3, f.w4);
+    const unsigned m1 = MB == 8 ? f.c.p8 : f.c.p2, m2 = MB == 8 ? f.c.p16 : f.c.p4;
+    const unsigned s0 = a0 + a2, d0 = a0 - a2 + m1, s1 = a1 + a3, d1 = f.root<4>(a1 - a3 + m1);
     a0 = s0 + s1;
-    a2 = s0 - s1;
+    a2 = s0 - s1 + m2;
     a1 = d0 + d1;
-    a3 = d0 - d1;
+    a3 = d0 - d1 + f.c.p2;
 }
 
-// 16-point transform with the 16th root w1; input at most 0.75 p, output at
-// most 12 p in magnitude (the same index scheme as dft16)
-__device__ __forceinline__ void int_dft16(const IntField &f, int (&a)[16])
+// 16-point transform with the 16th root w1; input below 2 p, output below 26 p
+// (the same index scheme as dft16).  After the first four transforms every
+// value is below 8 p; the products bring theirs below 2 p again, so only row
+// m = 0 meets values of up to 8 p: one of its four is reduced.
+__device__ __forceinline__ void int_dft16(const IntField &f, unsigned (&a)[16])
 {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) int_dft4(f, a[j], a[j + 4], a[j + 8], a[j + 12]);
-    a[5] = f.mul(a[5], f.w1);
-    a[9] = f.mul(a[9], f.w2);
-    a[13] = f.mul(a[13], f.w3);
-    a[6] = f.mul(a[6], f.w2);
-    a[10] = f.mul(a[10], f.w4);
-    a[14] = f.mul(a[14], f.w6);
-    a[7] = f.mul(a[7], f.w3);
-    a[11] = f.mul(a[11], f.w6);
-    a[15] = f.mul(a[15], f.w9);
+    for (int j = 0; j < 4; ++j) int_dft4<2>(f, a[j], a[j + 4], a[j + 8], a[j + 12]);
+    a[5] = f.root<1>(a[5]);
+    a[9] = f.root<2>(a[9]);
+    a[13] = f.root<3>(a[13]);
+    a[6] = f.root<2>(a[6]);
+    a[10] = f.root<4>(a[10]);
+    a[14] = f.root<6>(a[14]);
+    a[7] = f.root<3>(a[7]);
+    a[11] = f.root<6>(a[11]);
+    a[15] = f.root<9>(a[15]);
+    a[0] = f.reduce(a[0]);
+    int_dft4<8>(f, a[0], a[1], a[2], a[3]);
 #pragma unroll
-    for (int m = 0; m < 4; ++m) int_dft4(f, a[4 * m], a[4 * m + 1], a[4 * m + 2], a[4 * m + 3]);
-    int t[16];
+    for (int m = 1; m < 4; ++m) int_dft4<2>(f, a[4 * m], a[4 * m + 1], a[4 * m + 2], a[4 * m + 3]);
+    unsigned t[16];
 #pragma unroll
     for (int i = 0; i < 16; ++i) t[i] = a[i];
 #pragma unroll
@@ -120,7 +139,8 @@ __device__ __forceinline__ int int_swz(int i) { return i ^ ((i >> 5) & 15) ^ ((i
 // of it are done on return.  tw: rows r = 1 .. 15 of the twiddles of the
 // second (16 columns) and third pass (256 columns).
 template <bool LD_ALIAS>
-__device__ __forceinline__ void int_ntt(const IntField &f, int (&a)[16], int *s, const int *tw, int q, int bar_id)
+__device__ __forceinline__ void int_ntt(const IntField &f, unsigned (&a)[16], unsigned *s, const unsigned *tw, int q,
+                                        int bar_id)
 {
     int_dft16(f, a);
     if constexpr (LD_ALIAS) __syncthreads();  // the first pass's inputs lie in the exchange buffers
@@ -137,7 +157,7 @@ __device__ __forceinline__ void int_ntt(const IntField &f, int (&a)[16], int *s,
     team_sync<-1, 256>(bar_id);
     {
         const int k = q & 15;
-        a[0] = f.mul(a[0], f.one);
+        a[0] = f.reduce(a[0]);
 #pragma unroll
         for (int r = 1; r < 16; ++r) a[r] = f.mul(a[r], tw[(r - 1) * 16 + k]);
         int_dft16(f, a);
@@ -150,16 +170,16 @@ __device__ __forceinline__ void int_ntt(const IntField &f, int (&a)[16], int *s,
 #pragma unroll
     for (int r = 0; r < 16; ++r) a[r] = s[256 * r + ((r & 1) ? qo : qe)];
     team_sync<-1, 256>(bar_id);
-    a[0] = f.mul(a[0], f.one);
+    a[0] = f.reduce(a[0]);
 #pragma unroll
     for (int r = 1; r < 16; ++r) a[r] = f.mul(a[r], tw[240 + (r - 1) * 256 + q]);
     int_dft16(f, a);
 }
 
-// v mod p for |v| <= 2^54: v = vh 2^25 + vl (at most 0.79 p)
-__device__ __forceinline__ int int_mod(const IntField &f, int c25, long long v)
+// v mod p for |v| <= 2^55: v = vh 2^25 + vl, vh made positive by 8 p (below 1.8 p)
+__device__ __forceinline__ unsigned int_mod(const IntField &f, unsigned c25, long long v)
 {
-    return f.mul((int) (v >> 25), c25) + (int) (v & ((1 << 25) - 1));
+    return f.mul((unsigned) (int) (v >> 25) + f.c.p8, c25) + ((unsigned) v & ((1u << 25) - 1));
 }
 
 // ---- fixed point ------------------------------------------------------------
@@ -176,8 +196,8 @@ __device__ __forceinline__ long long int_fixed(long long bits, int emax)
     const int e = (int) (bits >> 52) & 2047;
     unsigned long long m = (unsigned long long) bits & ((1ull << 52) - 1);
     if (e > 0) m |= 1ull << 52;
-    const int d = emax - (e > 0 ? e : 1) - 9;
-    m = d <= 0 ? m << -d : (d < 60 ? (m + (1ull << (d - 1))) >> d : 0ull);
+    const int d = min(emax - max(e, 1), 63);
+    m = ((m << 9) + ((1ull << d) >> 1)) >> d;  // (up to d = 9 the half is shifted out again)
     return bits < 0 ? -(long long) m : (long long) m;
 }
 
@@ -205,18 +225,48 @@ template <int NTH> __device__ __forceinline__ long long int_block_sum(long long 
     return v;
 }
 
-template <int NTH> __device__ __forceinline__ float int_block_fsum(float v, float *red)
+// log2 of a bound on sum v^2 over any L consecutive samples, |v| <= 2^nb, sample
+// tid + 1024 i in v[i]: the largest sum of the runs of 32 samples that a window
+// can touch, each sample's square taken above its value (12 bits).  red: 128 words.
+template <int NTH, int PER>
+__device__ __forceinline__ float int_window_norm(const long long (&v)[PER], int nb, int L, unsigned *red)
 {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    static_assert(NTH * PER == 4096 && NTH == 1024, "128 runs, four per lane");
+    const int lane = threadIdx.x & 31, d = max(0, nb - 12);
     __syncthreads();
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-    __syncthreads();
-    const int l = threadIdx.x & 31;
-    v = l < NTH / 32 ? red[l] : 0.f;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
+    for (int i = 0; i < PER; ++i)
+    {
+        const unsigned y = (unsigned) ((v[i] < 0 ? -v[i] : v[i]) >> d) + 1u;
+        const unsigned q = __reduce_add_sync(0xffffffffu, y * y);  // below 2^30
+        if (lane == 0) red[32 * i + (threadIdx.x >> 5)] = (q >> 5) + 1u;
+    }
+    __syncthreads();
+    uint4 r = reinterpret_cast<const uint4 *>(red)[lane];
+    r.y += r.x;
+    r.z += r.y;
+    r.w += r.z;
+    unsigned inc = r.w;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1)
+    {
+        const unsigned u = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += u;
+    }
+    const unsigned ex = inc - r.w, total = __shfl_sync(0xffffffffu, inc, 31);
+    const unsigned P[5] = {ex, ex + r.x, ex + r.y, ex + r.z, inc};  // sums of the runs before 4 lane .. 4 lane + 4
+    const int nc = (L + 62) / 32;                                   // runs touched
+    unsigned best = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+    {
+        const int to = k + nc, j = to & 3;
+        const unsigned src = j == 0 ? P[0] : j == 1 ? P[1] : j == 2 ? P[2] : P[3];
+        const unsigned e = __shfl_sync(0xffffffffu, src, (lane + (to >> 2)) & 31);
+        best = max(best, (4 * lane + to < 128 ? e : total) - P[k]);
+    }
+    best = __reduce_max_sync(0xffffffffu, best);
+    return fminf(log2f((float) best) + 5.f, log2f((float) L) + (float) (2 * (nb - d))) + (float) (2 * d);
 }
 
 // Quantises the PER samples (bit patterns) each of NTH threads holds, N = NTH
@@ -224,10 +274,9 @@ template <int NTH> __device__ __forceinline__ float int_block_fsum(float v, floa
 // their unit (x - level = v 2^ex up to half a unit).  An infinity or NaN
 // counts as 0 and sets *bad.  NORM false: at most kIntXBits bits.  NORM true:
 // the finest unit at which the 2-norm of every window of at most L samples
-// stays below 2^kIntNormBits (bounded by sqrt(L) times the largest deviation
-// and by the norm of all samples), at most 54 bits.
+// stays below 2^kIntNormBits, at most 55 bits; lred: 64 words.
 template <int NTH, int PER, bool NORM>
-__device__ __forceinline__ int int_quantise(long long (&v)[PER], int *ired, long long *lred, float L, bool *bad)
+__device__ __forceinline__ int int_quantise(long long (&v)[PER], int *ired, long long *lred, int L, bool *bad)
 {
     constexpr int LOG2N = NTH * PER == 4096 ? 12 : 13;
     static_assert(NTH * PER == 1 << LOG2N, "the level is a sum shifted by log2 N");
@@ -258,28 +307,19 @@ __device__ __forceinline__ int int_quantise(long long (&v)[PER], int *ired, long
         s += v[i] >> LOG2N;
     }
     const long long lev = int_block_sum<NTH>(s, lred);  // about the mean
-    int nb = 0;
+    unsigned long long any = 0;
 #pragma unroll
     for (int i = 0; i < PER; ++i)
     {
         v[i] -= lev;
-        nb = max(nb, 64 - __clzll(v[i] < 0 ? -v[i] : v[i]));
+        any |= (unsigned long long) (v[i] ^ (v[i] >> 63));
     }
-    nb = int_block_max<NTH>(nb, ired);
+    const int nb = int_block_max<NTH>(64 - __clzll((long long) any), ired);  // |v| <= 2^nb
     int sh;
     if constexpr (NORM)
     {
-        const int d = max(0, nb - 31);
-        float q = 0.f;
-#pragma unroll
-        for (int i = 0; i < PER; ++i)
-        {
-            const float y = (float) (int) (v[i] >> d);
-            q = fmaf(y, y, q);
-        }
-        q = int_block_fsum<NTH>(q, reinterpret_cast<float *>(ired));
-        const float n2 = fminf(1.02f * q, L * exp2f((float) (2 * (nb - d))));
-        sh = max(max(0, nb - 54), (int) ceilf(0.5f * log2f(n2) + ((float) d + 0.02f - kIntNormBits)));
+        const float n2 = int_window_norm<NTH, PER>(v, nb, L, reinterpret_cast<unsigned *>(lred));
+        sh = max(max(0, nb - 55), (int) ceilf(0.5f * n2 - kIntNormBits));
     }
     else
         sh = max(0, nb - kIntXBits);
@@ -292,15 +332,15 @@ __device__ __forceinline__ int int_quantise(long long (&v)[PER], int *ired, long
 // ---- template table -----------------------------------------------------------
 // One CTA per (template, prime): B[t][prime][k] = transform of round(b 2^53),
 // b the demeaned unit-norm template (FP64, as template_spectra_kernel), times
-// R / N modulo p, centred.
+// R / N modulo p, in [0, p).
 __global__ void __launch_bounds__(256) int_bank_kernel(IntBankParams p)
 {
     __shared__ double red[8];
-    __shared__ int buf[kIntN];
+    __shared__ unsigned buf[kIntN];
     const int t = blockIdx.x / kIntPrimes, pi = blockIdx.x % kIntPrimes, tid = threadIdx.x;
     const IntField f(p.c.prime[pi]);
     const int L = p.tlen[t];
-    int *out = p.B + ((long) t * kIntPrimes + pi) * kIntN;
+    unsigned *out = p.B + ((long) t * kIntPrimes + pi) * kIntN;
     if (L > kIntN) return;  // correlated directly: in no plan
     const double *b = p.tmpl + p.toff[t];
     double s = 0;
@@ -314,76 +354,132 @@ __global__ void __launch_bounds__(256) int_bank_kernel(IntBankParams p)
     }
     const double nrm2 = block_sum<double>(q, red);
     const double inv = nrm2 > 0 ? 1.0 / sqrt(nrm2) : 0.0, scale = ldexp(1.0, kIntBBits);
-    int a[16];
+    unsigned a[16];
 #pragma unroll
     for (int r = 0; r < 16; ++r)
     {
         const int j = tid + 256 * r;
-        a[r] = j < L ? int_mod(f, p.c.prime[pi].c25, llrint((b[j] - mean) * inv * scale)) : 0;
+        a[r] = j < L ? int_mod(f, p.c.prime[pi].c25, llrint((b[j] - mean) * inv * scale)) : 0u;
     }
     int_ntt<false>(f, a, buf, p.tw + pi * kIntTw, tid, 1);
 #pragma unroll
     for (int r = 0; r < 16; ++r)
     {
-        int v = f.mul(a[r], p.c.prime[pi].rrn);
-        v = v > f.p / 2 ? v - f.p : (v < -(f.p / 2) ? v + f.p : v);
-        out[tid + 256 * r] = v;
+        const unsigned v = f.mul(a[r], p.c.prime[pi].rrn);
+        out[tid + 256 * r] = min(v, v - f.c.p);
     }
 }
 
 // ---- normalisation -----------------------------------------------------------
-// sqrt(L) / sqrt(V 2^(2 ex)) for V > 0 (0 for V = 0, a constant window; sqrt(L)
-// / tol where the deviation is at most tol), as DenOps<double>::out
-__device__ __forceinline__ double int_inv_den(unsigned __int128 V, int ex, double sqrtL, double tol, long long tol2_bits)
+// The smallest integer V whose V 2^(2 ex), rounded down to FP64, is above
+// tol2 >= 0 (all ones: none)
+__device__ __forceinline__ unsigned __int128 int_tol(double tol2, int ex)
 {
-    if (V == 0) return 0.0;
-    const unsigned long long vh = (unsigned long long) (V >> 64);
-    const int lz = vh ? __clzll((long long) vh) : 64 + __clzll((long long) (unsigned long long) V);
-    const unsigned long long m = (unsigned long long) ((V << lz) >> 64);  // V = m 2^(64 - lz), m >= 2^63
-    int E = 128 - lz + 2 * ex;  // V 2^(2 ex) = (m / 2^64) 2^E
-    // its FP64 bit pattern, for the comparison with tol^2 (exponents below
-    // FP64's range are below tol^2, above it above)
-    const long long vb = E < -1000 ? 0 : (E > 1000 ? 0x7fe0000000000000ll : ((long long) (E + 1021) << 52) + (long long) (m >> 11));
-    if (vb <= tol2_bits) return sqrtL / tol;
-    // fm in [1/4, 1) with an even exponent
-    unsigned long long fm = m;
-    if (E & 1)
-    {
-        fm >>= 1;
-        E += 1;
-    }
-    const float f0 = (float) (unsigned) (fm >> 32) * 0x1p-32f;
-    // y in (1, 2]: 30 fractional bits of the FP32 value
-    const unsigned y = (unsigned) (rsqrtf(f0) * 0x1p30f);
-    const unsigned long long y2 = (unsigned long long) y * y;                   // 60 fractional bits
-    const long long e = (1ll << 60) - (long long) __umul64hi(fm, y2);            // 1 - fm y^2, about 2^-21
-    const long long es = e >> 16;                                                // 44 bits
-    const long long corr = (e >> 1) + ((3 * (es * es)) >> 31);                   // e / 2 + 3 e^2 / 8, 60 bits
-    const long long lo = (long long) (unsigned) corr * y, hi = (corr >> 32) * (long long) y;  // corr y, 90 bits
-    const unsigned long long y60 = ((unsigned long long) y << 30) + (unsigned long long) ((hi << 2) + (long long) ((unsigned long long) lo >> 30));
-    // y60 in [2^60, 2^61]: 1 / sqrt(V) = y60 2^-60 2^(-E / 2)
-    const long long yb = ((long long) (1022 - (E >> 1)) << 52) + (long long) ((y60 + 128) >> 8);
-    return sqrtL * __longlong_as_double(yb);
+    const long long b = __double_as_longlong(tol2) + 1;
+    const int e = (int) (b >> 52) & 2047;
+    unsigned long long m = (unsigned long long) b & ((1ull << 52) - 1);
+    if (e > 0) m |= 1ull << 52;
+    const int sh = max(e, 1) - 1075 - 2 * ex;  // V >= m 2^sh
+    if (sh >= 75) return ~(unsigned __int128) 0;
+    if (sh >= 0) return (unsigned __int128) m << sh;
+    return sh <= -64 ? 1 : (unsigned __int128) ((m - 1) >> -sh) + 1;
 }
 
-// One CTA per (tile of kIntTile samples, group).  MULTI false (one template
-// length): the channel's row den[c][k].  MULTI true: for every template of
-// the group, its own rows, written where the coefficients go (the correlator
-// reads each value before it stores the coefficient in its place).
-//
-// The tile's prefix sums (24 bytes per sample, 196 KB of shared memory) give
-// any window of any length in two loads each of S1 and S2: about 60 integer
-// instructions and one FP64 product per lag, against some 27 FP64 operations
-// (16 clocks per SM) of the running FP64 form.
-__device__ __forceinline__ int int_pswz(int i) { return i ^ ((i >> 3) & 15); }
+// scale / sqrt(V 2^(2 ex)) for V > 0
+__device__ __forceinline__ double int_inv_den(unsigned __int128 V, int ex, double scale)
+{
+    // V = fm 2^E, fm in [1/4, 1), E even
+    unsigned w3 = (unsigned) (V >> 96), w2 = (unsigned) (V >> 64), w1 = (unsigned) (V >> 32), w0 = (unsigned) V;
+    int E2 = 64 + ex;  // E / 2 + ex
+    while (w3 == 0)
+    {
+        w3 = w2;
+        w2 = w1;
+        w1 = w0;
+        w0 = 0;
+        E2 -= 16;
+    }
+    const int sh = __clz((int) w3) & ~1;
+    E2 -= sh >> 1;
+    const unsigned fh = __funnelshift_l(w2, w3, sh), fl = __funnelshift_l(w1, w2, sh);
+    const unsigned long long fm = ((unsigned long long) fh << 32) | fl;
+    // y in [1, 2): FP32 reciprocal square root, 23 fractional bits (formed in
+    // and taken from the bit patterns: conversions go through the slow pipe)
+    const float f0 = __uint_as_float(0x3f800000u | (fh >> 9)) - 1.0f;
+    const unsigned y = (__float_as_uint(fminf(rsqrtf(f0), 0x1.fffffep0f)) & 0x7fffffu) | 0x800000u;
+    const unsigned long long y2 = (unsigned long long) (y << 7) * (y << 7);    // 60 fractional bits
+    const long long e = (1ll << 60) - (long long) __umul64hi(fm, y2);          // 1 - fm y^2, below 2^-19
+    const int es = (int) (e >> 16);                                            // 44 bits
+    const long long corr = (e >> 1) + ((3 * ((long long) es * es)) >> 31);     // e / 2 + 3 e^2 / 8, 60 bits
+    const unsigned long long y60 = ((unsigned long long) y << 37) + (unsigned long long) ((corr * (long long) y) >> 23);
+    // y60 in [2^60, 2^61]: 1 / sqrt(V 2^(2 ex)) = y60 2^-60 2^-E2
+    // (0 where that is below FP64's normal range)
+    const long long yb = E2 > 1021 ? 0 : ((long long) (1022 - E2) << 52) + (long long) ((y60 + 128) >> 8);
+    return scale * __longlong_as_double(yb);
+}
 
-template <bool MULTI> __global__ void __launch_bounds__(kIntThreads, 1) int_den_kernel(IntDenParams p)
+// One CTA per (tile of T samples, group).  MULTI false (one template length):
+// the channel's row den[c][k].  MULTI true: for every template of the group,
+// its own rows, written where the coefficients go (the correlator reads each
+// value before it stores the coefficient in its place).
+//
+// The tile's prefix sums (24 bytes per sample) give any window of any length
+// in two loads each of S1 and S2: about 90 integer instructions and one FP64
+// product per lag, against some 27 FP64 operations (16 clocks per SM) of the
+// running FP64 form.  T = 4096 (98 KB, two CTAs of 512 threads per SM, whose
+// loads, scans and lags overlap) for templates of up to 1,024 samples, where
+// the windows' overlap costs at most a third; T = 8192 above (64 x 360,000, L
+// = 500: 308 us, in tiles of 8192 346; 8 x 360,000, 160 templates of 200 ..
+// 2,000: 424 us, in tiles of 4096 444).
+// Bound by the integer pipes (ALU 61 %, issue 59 %).  Before the sums in three
+// words, the integer normalisation of V and the square roots of L taken out of
+// the threads: 396 and 562 us in tiles of 8192.
+__device__ __forceinline__ int int_pswz(int i) { return i ^ ((i >> 3) & 15); }
+__host__ __device__ constexpr size_t int_den_bytes(int T) { return 3 * sizeof(long long) * (size_t) (T + 16); }
+
+// sums of x and of x^2 as al^2 + 2^26 ah al + 2^50 ah^2, |x| = 2^25 ah + al <=
+// 2^50: three multiplies and no carries (the sums of 8,192 stay below 2^63)
+struct IntSums
+{
+    long long s;
+    unsigned long long a, b, c;
+    __device__ __forceinline__ void add(long long v)
+    {
+        s += v;
+        const unsigned long long m = v < 0 ? -v : v;
+        const unsigned l = (unsigned) m & ((1u << 25) - 1), h = (unsigned) (m >> 25);
+        a += (unsigned long long) l * l;
+        b += (unsigned long long) h * l;
+        c += (unsigned long long) h * h;
+    }
+    __device__ __forceinline__ void add(const IntSums &o)
+    {
+        s += o.s;
+        a += o.a;
+        b += o.b;
+        c += o.c;
+    }
+    __device__ __forceinline__ IntSums shfl_up(int d) const
+    {
+        return IntSums{__shfl_up_sync(0xffffffffu, s, d), __shfl_up_sync(0xffffffffu, a, d),
+                       __shfl_up_sync(0xffffffffu, b, d), __shfl_up_sync(0xffffffffu, c, d)};
+    }
+    __device__ __forceinline__ void squares(unsigned long long &lo, unsigned long long &hi) const
+    {
+        const unsigned __int128 q = ((unsigned __int128) c << 50) + ((unsigned __int128) b << 26) + a;
+        lo = (unsigned long long) q;
+        hi = (unsigned long long) (q >> 64);
+    }
+};
+
+template <bool MULTI, int T> __global__ void __launch_bounds__(T / 8, T == 4096 ? 2 : 1) int_den_kernel(IntDenParams p)
 {
     extern __shared__ __align__(16) unsigned char smem_id[];
-    __shared__ long long lred[32], wlo[33], whi[33], w1[33];
+    __shared__ long long lred[32];
+    __shared__ IntSums wsum[32];
     __shared__ int ired[32];
-    constexpr int PER = kIntTile / kIntThreads;  // consecutive samples per thread
-    constexpr int NP = kIntTile + 16;            // prefixes 0 .. kIntTile, swizzled in groups of 16
+    constexpr int PER = 8, NTH = T / PER;  // consecutive samples per thread
+    constexpr int NP = T + 16;             // prefixes 0 .. T, swizzled in groups of 16
     long long *P1 = reinterpret_cast<long long *>(smem_id);
     unsigned long long *PL = reinterpret_cast<unsigned long long *>(P1 + NP), *PH = PL + NP;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, g = blockIdx.y;
@@ -405,85 +501,88 @@ template <bool MULTI> __global__ void __launch_bounds__(kIntThreads, 1) int_den_
         v[i + 1] = k + 1 < p.n ? d.y : first;
     }
     bool bad;
-    const int ex = int_quantise<kIntThreads, PER, false>(v, ired, lred, 0.f, &bad);
+    const int ex = int_quantise<NTH, PER, false>(v, ired, lred, 0, &bad);
     // ---- prefix sums: thread, warp, block
-    long long s1 = 0;
-    unsigned __int128 s2 = 0;
+    IntSums inc{0, 0, 0, 0};
 #pragma unroll
-    for (int i = 0; i < PER; ++i)
-    {
-        s1 += v[i];
-        s2 += (unsigned __int128) ((__int128) v[i] * v[i]);
-    }
-    long long i1 = s1;
-    unsigned __int128 i2 = s2;
+    for (int i = 0; i < PER; ++i) inc.add(v[i]);
+    // (the products are formed again below: 24 of them would not stay in registers)
+#pragma unroll
+    for (int i = 0; i < PER; ++i) asm volatile("" : "+l"(v[i]));
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1)
     {
-        const long long u1 = __shfl_up_sync(0xffffffffu, i1, o);
-        const unsigned long long ul = __shfl_up_sync(0xffffffffu, (unsigned long long) i2, o);
-        const unsigned long long uh = __shfl_up_sync(0xffffffffu, (unsigned long long) (i2 >> 64), o);
-        if (lane >= o)
-        {
-            i1 += u1;
-            i2 += ((unsigned __int128) uh << 64) | ul;
-        }
+        const IntSums u = inc.shfl_up(o);
+        if (lane >= o) inc.add(u);
     }
-    if (lane == 31)
+    if (lane == 31) wsum[w] = inc;
+    __syncthreads();
+    if (w == 0)
     {
-        w1[w] = i1;
-        wlo[w] = (long long) (unsigned long long) i2;
-        whi[w] = (long long) (unsigned long long) (i2 >> 64);
+        IntSums t = lane < NTH / 32 ? wsum[lane] : IntSums{0, 0, 0, 0};
+#pragma unroll
+        for (int o = 1; o < NTH / 32; o <<= 1)
+        {
+            const IntSums u = t.shfl_up(o);
+            if (lane >= o) t.add(u);
+        }
+        if (lane < NTH / 32) wsum[lane] = t;
     }
     __syncthreads();
-    long long e1 = i1 - s1;
-    unsigned __int128 e2 = i2 - s2;
-    for (int u = 0; u < w; ++u)
-    {
-        e1 += w1[u];
-        e2 += ((unsigned __int128) (unsigned long long) whi[u] << 64) | (unsigned long long) wlo[u];
-    }
+    IntSums ex_ = inc.shfl_up(1);
+    if (lane == 0) ex_ = IntSums{0, 0, 0, 0};
+    if (w > 0) ex_.add(wsum[w - 1]);
 #pragma unroll
     for (int i = 0; i < PER; ++i)
     {
         const int k = int_pswz(PER * tid + i);
-        P1[k] = e1;
-        PL[k] = (unsigned long long) e2;
-        PH[k] = (unsigned long long) (e2 >> 64);
-        e1 += v[i];
-        e2 += (unsigned __int128) ((__int128) v[i] * v[i]);
+        P1[k] = ex_.s;
+        ex_.squares(PL[k], PH[k]);
+        ex_.add(v[i]);
     }
-    if (tid == kIntThreads - 1)
+    if (tid == NTH - 1)
     {
-        const int k = int_pswz(kIntTile);
-        P1[k] = e1;
-        PL[k] = (unsigned long long) e2;
-        PH[k] = (unsigned long long) (e2 >> 64);
+        const int k = int_pswz(T);
+        P1[k] = ex_.s;
+        ex_.squares(PL[k], PH[k]);
     }
     __syncthreads();
-    const long long tol2 = __double_as_longlong(p.tol * p.tol);
-    auto lags_of = [&](int L, long nv, double *out) {
-        const double sqrtL = sqrt((double) L);
+    const unsigned __int128 vtol = int_tol(p.tol * p.tol, ex);
+    // sqrtL: sqrt(L) times the factor of the correlator's numerators
+    auto lags_of = [&](int L, long nv, double *out, double sqrtL) {
         const int n = (int) (nv - k0 < (long) p.lags ? nv - k0 : (long) p.lags);
-        for (int k = tid; k < n; k += kIntThreads)
+        for (int k = tid; k < n; k += NTH)
         {
             const int a = int_pswz(k), b = int_pswz(k + L);
             const long long S1 = P1[b] - P1[a];
+            const unsigned long long u = S1 < 0 ? 0ull - (unsigned long long) S1 : (unsigned long long) S1;
             const unsigned __int128 S2 = (((unsigned __int128) PH[b] << 64) | PL[b]) - (((unsigned __int128) PH[a] << 64) | PL[a]);
-            const unsigned __int128 V = S2 * (unsigned) L - (unsigned __int128) ((__int128) S1 * S1);
-            out[k0 + k] = int_inv_den(V, ex, sqrtL, p.tol, tol2);
+            const unsigned __int128 V = S2 * (unsigned) L - (unsigned __int128) u * u;
+            // 0 for a constant window, sqrt(L) / tol where the deviation is
+            // at most tol, as DenOps<double>::out
+            out[k0 + k] = V < vtol ? (V == 0 ? 0.0 : sqrtL / p.tol) : int_inv_den(V, ex, sqrtL);
         }
     };
     if constexpr (MULTI)
     {
-        for (int j = p.grp_tb[g]; j < p.grp_te[g]; ++j)
+        // square roots of up to 64 templates at a time: by every thread they
+        // would cost more (FP64 pipe) than a template's lags
+        __shared__ double rootL[64];
+        for (int j0 = p.grp_tb[g], je = p.grp_te[g]; j0 < je; j0 += 64)
         {
-            const int t = p.tids[j];
-            lags_of(p.tlen[t], p.nvalid[t], p.rho + (long) t * p.ldr);
+            const int m = min(64, je - j0);
+            __syncthreads();
+            if (tid < m) rootL[tid] = sqrt((double) p.tlen[p.tids[j0 + tid]]) * p.scale;
+            __syncthreads();
+            for (int j = 0; j < m; ++j)
+            {
+                const int t = p.tids[j0 + j];
+                lags_of(p.tlen[t], p.nvalid[t], p.rho + (long) t * p.ldr, rootL[j]);
+            }
         }
     }
     else
-        lags_of(p.L, p.nv, p.den + (long) c * p.ldd);
+        lags_of(p.L, p.nv, p.den + (long) c * p.ldd, p.scale);
 }
 
 // ---- correlator --------------------------------------------------------------
@@ -494,37 +593,53 @@ template <bool MULTI> __global__ void __launch_bounds__(kIntThreads, 1) int_den_
 // threads combine them, four lags each.  Shared memory: the block's four
 // spectra (64 KB), four exchange buffers (64 KB), the twiddles (65 KB).
 //
-// Bound by the integer pipes.  160 templates of 200 .. 2,000 samples against 8
-// channels x 360,000: 8.35 ms (FP64 transforms with in-block normalisation)
-// -> 2.14 ms + 0.54 ms normalisation; 64 channels x 360,000 with one template
-// of 500 each: 2.69 + 1.15 (den_kernel) -> 0.98 + 0.38 ms.
+// Bound by the integer pipes (multiplier and ALU; issue 2 of 4 per clock).  160
+// templates of 200 .. 2,000 samples against 8 channels x 360,000: 8.35 ms (FP64
+// transforms with in-block normalisation) -> 1.73 ms + 0.42 ms normalisation;
+// 64 channels x 360,000 with one template of 500 each: 2.69 + 1.15 (den_kernel)
+// -> 0.87 + 0.31 ms.  Signed words with centred residues took 2.14 and 0.98 ms.
 struct IntLayout
 {
     static constexpr size_t off_red = 64;                    // after the barrier: reductions
-    static constexpr size_t off_mask = off_red + 512;        // two masks of 64 chunk bits
+    static constexpr size_t off_mask = off_red + 640;        // two masks of 64 chunk bits
     static constexpr size_t off_xh = 1024;
     static constexpr size_t off_buf = off_xh + sizeof(int) * kIntPrimes * kIntN;
     static constexpr size_t off_tw = off_buf + sizeof(int) * kIntPrimes * kIntN;
     static constexpr size_t bytes = off_tw + sizeof(int) * kIntPrimes * kIntTw;
 };
 
-// FP64 value of the numerator in (v0, v1, v2, v3) mixed radix times 2^e2
-__device__ __forceinline__ double int_value(const IntConsts &c, int v0, int v1, int v2, int v3, int e2)
+// numerator / M as a signed 64-bit fraction, from the residues r (any 32 bits):
+// sum of y_i / p_i modulo 1, y_i = r_i (M / p_i)^-1 mod p_i, with 1 / p_i to 96
+// bits
+__device__ __forceinline__ long long int_fraction(const IntConsts &c, const unsigned (&r)[kIntPrimes])
 {
-    const long long A = (long long) c.prime[2].p * v3 + v2;
-    const unsigned long long B = (unsigned long long) ((long long) c.prime[0].p * v1 + v0);
-    const __int128 V = (__int128) A * (long long) c.p01 + (__int128) B;
-    const bool neg = V < 0;
-    const unsigned __int128 u = neg ? (unsigned __int128) -V : (unsigned __int128) V;
-    const unsigned long long uh = (unsigned long long) (u >> 64), ul = (unsigned long long) u;
-    if ((uh | ul) == 0) return 0.0;
-    const int lz = uh ? __clzll((long long) uh) : 64 + __clzll((long long) ul);
-    const unsigned long long m = (unsigned long long) ((u << lz) >> 64);  // u = m 2^(64 - lz)
-    const int E = 1150 - lz + e2;  // value = (m / 2^11) 2^(75 - lz + e2)
+    unsigned long long t0 = 1ull << 31, t1 = 0;  // rounds to nearest: a numerator of 0 stays 0
+    unsigned t2 = 0;
+#pragma unroll
+    for (int i = 0; i < kIntPrimes; ++i)
+    {
+        const unsigned y = mont(r[i], c.prime[i].crt, c.prime[i].p, c.prime[i].nq);
+        t0 += (unsigned long long) y * c.prime[i].f0;
+        t1 += (unsigned long long) y * c.prime[i].f1;
+        t2 += y * c.prime[i].f2;
+    }
+    t1 += t0 >> 32;
+    t2 += (unsigned) (t1 >> 32);
+    return (long long) (((unsigned long long) t2 << 32) | (unsigned) t1);
+}
+
+// v 2^e as FP64, rounded to nearest (0 below, infinity above its range)
+__device__ __forceinline__ double int_to_double(long long v, int e)
+{
+    if (v == 0) return 0.0;
+    const unsigned long long u = v < 0 ? 0ull - (unsigned long long) v : (unsigned long long) v;
+    const int lz = __clzll((long long) u);
+    const unsigned long long m = u << lz;
+    const int E = 1086 - lz + e;  // value = (m / 2^11) 2^(11 - lz + e)
     unsigned long long bits = ((unsigned long long) (unsigned) (E - 1) << 52) + ((m >> 11) + ((m >> 10) & 1));
     if (E < 2) bits = 0;
     else if (E > 2045) bits = 0x7ff0000000000000ull;
-    return __longlong_as_double((long long) (bits | (neg ? 1ull << 63 : 0ull)));
+    return __longlong_as_double((long long) (bits | ((unsigned long long) v & (1ull << 63))));
 }
 
 template <bool SHARED_DEN> __global__ void __launch_bounds__(kIntThreads, 1) int_xcorr_kernel(IntParams p)
@@ -532,11 +647,11 @@ template <bool SHARED_DEN> __global__ void __launch_bounds__(kIntThreads, 1) int
     extern __shared__ __align__(128) unsigned char smem_ix[];
     uint64_t *bar = reinterpret_cast<uint64_t *>(smem_ix);
     long long *lred = reinterpret_cast<long long *>(smem_ix + IntLayout::off_red);
-    int *ired = reinterpret_cast<int *>(lred + 32);
+    int *ired = reinterpret_cast<int *>(lred + 64);
     unsigned *Mk = reinterpret_cast<unsigned *>(smem_ix + IntLayout::off_mask);
-    int *xh = reinterpret_cast<int *>(smem_ix + IntLayout::off_xh);
-    int *buf = reinterpret_cast<int *>(smem_ix + IntLayout::off_buf);
-    int *tws = reinterpret_cast<int *>(smem_ix + IntLayout::off_tw);
+    unsigned *xh = reinterpret_cast<unsigned *>(smem_ix + IntLayout::off_xh);
+    unsigned *buf = reinterpret_cast<unsigned *>(smem_ix + IntLayout::off_buf);
+    unsigned *tws = reinterpret_cast<unsigned *>(smem_ix + IntLayout::off_tw);
     const int tid = threadIdx.x, bx = blockIdx.x, g = blockIdx.y;
     const XcorrParams<double> &x = p.x;
     const int c = x.grp_chan[g], S = x.S;
@@ -590,7 +705,7 @@ template <bool SHARED_DEN> __global__ void __launch_bounds__(kIntThreads, 1) int
             const int j = tid + kIntThreads * i;
             v[i] = seg[k0 + j < p.n ? j : 0];
         }
-        ex = int_quantise<kIntThreads, PER, true>(v, ired, lred, (float) p.Lmax, &bad);
+        ex = int_quantise<kIntThreads, PER, true>(v, ired, lred, p.Lmax, &bad);
 #pragma unroll
         for (int i = 0; i < PER; ++i) xq[(kIntN - (tid + kIntThreads * i)) & (kIntN - 1)] = v[i];
         __syncthreads();
@@ -608,14 +723,15 @@ template <bool SHARED_DEN> __global__ void __launch_bounds__(kIntThreads, 1) int
         }
         return;
     }
-    const int team = tid >> 8, q = tid & 255, bar_id = 1 + team;
+    // (the same for the warp, and known to be: the constants stay uniform)
+    const int team = __shfl_sync(0xffffffffu, tid >> 8, 0), q = tid & 255, bar_id = 1 + team;
     const IntField f(p.c.prime[team]);
-    const int *tw = tws + team * kIntTw;
-    int *s = buf + team * kIntN, *xt = xh + team * kIntN;
-    int a[16];
+    const unsigned *tw = tws + team * kIntTw;
+    unsigned *s = buf + team * kIntN, *xt = xh + team * kIntN;
+    unsigned a[16];
     {
         const long long *xq = reinterpret_cast<const long long *>(buf) + kIntN;
-        const int c25 = p.c.prime[team].c25;
+        const unsigned c25 = p.c.prime[team].c25;
 #pragma unroll
         for (int r = 0; r < 16; ++r) a[r] = int_mod(f, c25, xq[q + 256 * r]);
         int_ntt<true>(f, a, s, tw, q, bar_id);
@@ -623,12 +739,11 @@ template <bool SHARED_DEN> __global__ void __launch_bounds__(kIntThreads, 1) int
         for (int r = 0; r < 16; ++r) xt[q + 256 * r] = a[r];  // read by this thread only
     }
     const bool pk = x.pk_on != 0;
-    const int e2 = ex - kIntBBits;
     int t_prev = -1;
     for (int ti = t_begin; ti < t_end; ++ti)
     {
         const int t = x.tids[ti], it = ti - t_begin;
-        const int *Bt = p.B + ((long) t * kIntPrimes + team) * kIntN;
+        const unsigned *Bt = p.B + ((long) t * kIntPrimes + team) * kIntN;
 #pragma unroll
         for (int r = 0; r < 16; ++r) a[r] = f.mul(xt[q + 256 * r], __ldg(Bt + q + 256 * r));
         if (it > 0)
@@ -653,19 +768,9 @@ template <bool SHARED_DEN> __global__ void __launch_bounds__(kIntThreads, 1) int
         for (int k = tid; k < kmax; k += kIntThreads)
         {
             const double inv = den[k];
-            // mixed-radix digits of the numerator, the last one centred
-            const IntConsts &cc = p.c;
-            const int p0 = cc.prime[0].p, p1 = cc.prime[1].p, p2 = cc.prime[2].p, p3 = cc.prime[3].p;
-            const int n1 = cc.prime[1].nq, n2 = cc.prime[2].nq, n3 = cc.prime[3].nq;
-            int v0 = mont(buf[k], cc.prime[0].one, p0, cc.prime[0].nq);
-            v0 += (v0 >> 31) & p0;
-            int v1 = mont(buf[kIntN + k] - v0, cc.i01, p1, n1);
-            v1 += (v1 >> 31) & p1;
-            int v2 = mont(mont(buf[2 * kIntN + k] - v0, cc.i02, p2, n2) - v1, cc.i12, p2, n2);
-            v2 += (v2 >> 31) & p2;
-            int v3 = mont(mont(mont(buf[3 * kIntN + k] - v0, cc.i03, p3, n3) - v1, cc.i13, p3, n3) - v2, cc.i23, p3, n3);
-            v3 = v3 > p3 / 2 ? v3 - p3 : (v3 < -(p3 / 2) ? v3 + p3 : v3);
-            const double r = clamp_rho(int_value(cc, v0, v1, v2, v3, e2) * inv);
+            const unsigned rs[kIntPrimes] = {buf[k], buf[kIntN + k], buf[2 * kIntN + k], buf[3 * kIntN + k]};
+            // (the factor M / 2^64 2^-53 is in the normalisation)
+            const double r = clamp_rho(int_to_double(int_fraction(p.c, rs), ex) * inv);
             dst[k] = r;
             if (pk && r > x.pk_thr) atomicOr(mk + (k >> 11), 1u << ((k >> 6) & 31));
         }

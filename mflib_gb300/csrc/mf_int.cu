@@ -23,27 +23,27 @@ bool is_prime(uint32_t n)
     return true;
 }
 
-// v times 2^32 modulo p, in (-p/2, p/2)
-int mont_of(uint64_t v, uint32_t p)
-{
-    const uint64_t r = (v % p) * ((1ull << 32) % p) % p;
-    return r > p / 2 ? (int) ((long long) r - (long long) p) : (int) r;
-}
+// v times 2^32 modulo p
+unsigned mont_of(uint64_t v, uint32_t p) { return (unsigned) ((v % p) * ((1ull << 32) % p) % p); }
 
 struct Tables
 {
     IntConsts c;
-    std::vector<int> tw;
+    std::vector<unsigned> tw;
+    double scale;
     Tables() : tw((size_t) kIntPrimes * kIntTw)
     {
-        // the largest primes = 1 mod 8192 below 2^31 / 14
-        uint32_t cand = ((uint32_t) ((1ull << 31) / 14) - 1) / 8192 * 8192 + 1;
+        // the largest primes = 1 mod 8192 below 2^32 / 26 (int_dft16)
+        uint32_t cand = (uint32_t) ((1ull << 32) / 26) / 8192 * 8192 + 1;
+        if (cand > (1ull << 32) / 26) cand -= 8192;
         uint64_t pr[kIntPrimes];
+        double M = 1.0;
         for (int i = 0; i < kIntPrimes; ++i, cand -= 8192)
         {
             while (!is_prime(cand)) cand -= 8192;
             const uint32_t p = cand;
             pr[i] = p;
+            M *= p;
             // a root of order N: g^((p-1)/N) with its N/2-th power = -1
             uint64_t w = 0;
             for (uint64_t g = 2; !w; ++g)
@@ -52,22 +52,30 @@ struct Tables
                 if (pow_mod(r, kIntN / 2, p) == p - 1) w = r;
             }
             IntPrime &q = c.prime[i];
-            q.p = (int) p;
+            q.p = p;
             uint32_t inv = 1;  // p^-1 modulo 2^32 by Newton's iteration
             for (int k = 0; k < 6; ++k) inv *= 2u - p * inv;
-            q.nq = (int) (0u - inv);
-            q.one = mont_of(1, p);
+            q.nq = 0u - inv;
+            q.p2 = 2 * p;
+            q.p4 = 4 * p;
+            q.p8 = 8 * p;
+            q.p16 = 16 * p;
+            q.inv = (unsigned) ((1ull << 32) / p);
             const uint64_t w16 = pow_mod(w, kIntN / 16, p);
-            q.w1 = mont_of(w16, p);
-            q.w2 = mont_of(pow_mod(w16, 2, p), p);
-            q.w3 = mont_of(pow_mod(w16, 3, p), p);
-            q.w4 = mont_of(pow_mod(w16, 4, p), p);
-            q.w6 = mont_of(pow_mod(w16, 6, p), p);
-            q.w9 = mont_of(pow_mod(w16, 9, p), p);
+            for (int k = 0; k < 10; ++k)
+            {
+                const uint64_t v = pow_mod(w16, k, p);
+                q.w[k] = (unsigned) v;
+                q.ws[k] = (unsigned) ((v << 32) / p);
+            }
             q.c25 = mont_of(1ull << 25, p);
             const uint64_t R = (1ull << 32) % p;
             q.rrn = mont_of(R * pow_mod(kIntN, p - 2, p) % p, p);
-            int *t = &tw[(size_t) i * kIntTw];
+            unsigned __int128 f = ((unsigned __int128) 1 << 96) / p;
+            q.f0 = (unsigned) f;
+            q.f1 = (unsigned) (f >> 32);
+            q.f2 = (unsigned) (f >> 64);
+            unsigned *t = &tw[(size_t) i * kIntTw];
             const uint64_t w256 = pow_mod(w, kIntN / 256, p);
             for (int r = 1; r < 16; ++r)
             {
@@ -77,14 +85,14 @@ struct Tables
                 for (int k = 0; k < 256; ++k, v = v * wr % p) t[240 + (r - 1) * 256 + k] = mont_of(v, p);
             }
         }
-        auto inv_of = [&](int a, int b) { return mont_of(pow_mod(pr[a], pr[b] - 2, pr[b]), (uint32_t) pr[b]); };
-        c.i01 = inv_of(0, 1);
-        c.i02 = inv_of(0, 2);
-        c.i12 = inv_of(1, 2);
-        c.i03 = inv_of(0, 3);
-        c.i13 = inv_of(1, 3);
-        c.i23 = inv_of(2, 3);
-        c.p01 = pr[0] * pr[1];
+        for (int i = 0; i < kIntPrimes; ++i)
+        {
+            uint64_t m = 1;
+            for (int k = 0; k < kIntPrimes; ++k)
+                if (k != i) m = m * (pr[k] % pr[i]) % pr[i];
+            c.prime[i].crt = mont_of(pow_mod(m, pr[i] - 2, pr[i]), (uint32_t) pr[i]);
+        }
+        scale = std::ldexp(M, -64 - kIntBBits);
     }
 };
 
@@ -96,9 +104,10 @@ const Tables &tables()
 
 }  // namespace
 
-const std::vector<int> &int_twiddles() { return tables().tw; }
+const std::vector<unsigned> &int_twiddles() { return tables().tw; }
+double int_numerator_scale() { return tables().scale; }
 
-cudaError_t launch_int_bank(const double *tmpl, const long *toff, const int *tlen, int nt, const int *tw, int *B,
+cudaError_t launch_int_bank(const double *tmpl, const long *toff, const int *tlen, int nt, const unsigned *tw, unsigned *B,
                             cudaStream_t s)
 {
     IntBankParams p{tmpl, toff, tlen, B, tw, tables().c};
@@ -106,18 +115,22 @@ cudaError_t launch_int_bank(const double *tmpl, const long *toff, const int *tle
     return cudaGetLastError();
 }
 
-cudaError_t launch_int_den(const IntDenParams &p, bool multi, int ntiles, int ngroups, cudaStream_t s)
+template <bool MULTI, int T> static cudaError_t go_den(const IntDenParams &p, int ntiles, int ngroups, cudaStream_t s)
 {
-    const size_t bytes = 3 * sizeof(long long) * (kIntTile + 16);
-    static SmemCap cap1, capm;
-    cudaError_t e = multi ? raise_smem_cap(int_den_kernel<true>, bytes, capm) : raise_smem_cap(int_den_kernel<false>, bytes, cap1);
+    static SmemCap cap;
+    cudaError_t e = raise_smem_cap(int_den_kernel<MULTI, T>, int_den_bytes(T), cap);
     if (e != cudaSuccess) return e;
-    if (multi) int_den_kernel<true><<<dim3(ntiles, ngroups), kIntThreads, bytes, s>>>(p);
-    else int_den_kernel<false><<<dim3(ntiles, ngroups), kIntThreads, bytes, s>>>(p);
+    int_den_kernel<MULTI, T><<<dim3(ntiles, ngroups), T / 8, int_den_bytes(T), s>>>(p);
     return cudaGetLastError();
 }
 
-cudaError_t launch_int_xcorr(const XcorrParams<double> &x, bool shared_den, const int *B, const int *tw, int Lmax, long n,
+cudaError_t launch_int_den(const IntDenParams &p, bool multi, int tile, int ntiles, int ngroups, cudaStream_t s)
+{
+    if (tile == 4096) return multi ? go_den<true, 4096>(p, ntiles, ngroups, s) : go_den<false, 4096>(p, ntiles, ngroups, s);
+    return multi ? go_den<true, 8192>(p, ntiles, ngroups, s) : go_den<false, 8192>(p, ntiles, ngroups, s);
+}
+
+cudaError_t launch_int_xcorr(const XcorrParams<double> &x, bool shared_den, const unsigned *B, const unsigned *tw, int Lmax, long n,
                              int nblocks, int ngroups, cudaStream_t s)
 {
     IntParams p{x, B, tw, Lmax, n, tables().c};
