@@ -11,11 +11,11 @@
 //     reference (normalizeSignal, src/matchedFilter.cpp:94-166) subtract the
 //     sums of samples that leave the window, so a quiet window next to a
 //     loud one inherits the loud samples' rounding error.  Here each
-//     32-sample chunk keeps its statistics about its own mean (cm, cs, cq);
-//     the window's core (the samples shared by a run of 32 lags) combines
-//     whole chunks about a reference R taken from the core (every term is
-//     the sum of squares of one chunk about R, so nothing cancels); only the
-//     31 samples at each edge of the run slide in and out, in FP32.  A run
+//     32-sample chunk keeps its statistics about its own mean; the first
+//     window of a run of 32 lags combines whole chunks about a reference R
+//     taken from its middle (every term is the sum of squares of one chunk
+//     about R, so nothing cancels); only the 31 samples at each edge of the
+//     run slide in and out, in FP32.  A run
 //     whose sliding samples carry more than 100x the variance of its
 //     quietest window is marked for the fix-up below.  Per run it also
 //     records the quietest window's M2, R and the spread of the window means
@@ -58,14 +58,70 @@ __device__ __forceinline__ void fix_mark(unsigned *fbits, int *flist, int *fcoun
     if (!(old & bit)) flist[atomicAdd(fcount, 1)] = (int) ((long) c * ldrs + r);
 }
 
-// Shared memory of den_robust_kernel: staged samples (padded as den_kernel),
-// chunk statistics, reduction scratch.
+// Shared memory of den_robust_kernel: staged samples (rows of 32 with 4 words
+// of padding, so that the threads' 16-byte loads of their own rows meet
+// different banks), chunk statistics (mean, sums of d and d^2 about it, twice
+// the former), reduction scratch.
 struct DenRobustLayout
 {
+    static constexpr int kRow = kDenRun + 4;
     static constexpr int nruns(int L) { return kThreads * den_runs_per_thread(L); }
-    static constexpr size_t y_bytes(int L) { return DenLayout<float>::y_bytes(L); }
-    static constexpr size_t bytes(int L) { return y_bytes(L) + sizeof(float) * (3 * (size_t) nruns(L) + 64); }
+    static constexpr size_t y_bytes(int L) { return sizeof(float) * kRow * (size_t) nruns(L); }
+    static constexpr size_t bytes(int L) { return y_bytes(L) + sizeof(float4) * (size_t) nruns(L) + 64 * sizeof(float); }
 };
+
+// rsqrtf of a normal number (rsqrtf itself spends three more instructions on subnormals)
+__device__ __forceinline__ float rsqrt_normal(float v)
+{
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+    return r;
+}
+
+// The 32 lags of a run from its first window's sums S and Q about Rr: M2 per
+// lag, their minimum, the largest |S|, the sum QB of the entering squares.
+// own: the run's row of samples; in: the row of its first entering sample,
+// which has index 4 col + A there (A at compile time: 16-byte loads, the
+// samples picked from two neighbouring vectors).
+template <int A>
+__device__ __forceinline__ void den_slide(const float *own, const float *in, int col, float Rr, float invL, float S,
+                                          float Q, float (&M2)[kDenRun], float &mn, float &Smax, float &QB)
+{
+    constexpr int kRow = DenRobustLayout::kRow;
+    auto vec = [&](int j) {
+        const int k = col + j;  // below 16: this row or the next
+        return *reinterpret_cast<const float4 *>(in + 4 * k + (k >> 3) * (kRow - kDenRun));
+    };
+    const f2 nR = f2_dup(-Rr);
+    float4 cur = vec(0);
+#pragma unroll
+    for (int g = 0; g < kDenRun / 4; ++g)
+    {
+        const float4 nxt = A || g < kDenRun / 4 - 1 ? vec(g + 1) : cur;
+        const float4 out = *reinterpret_cast<const float4 *>(own + 4 * g);
+        const float e[8] = {cur.x, cur.y, cur.z, cur.w, nxt.x, nxt.y, nxt.z, nxt.w};
+        float zi[4], zo[4];
+        f2_split(f2_make(e[A], e[A + 1]) + nR, zi[0], zi[1]);
+        f2_split(f2_make(e[A + 2], e[A + 3]) + nR, zi[2], zi[3]);
+        f2_split(f2_make(out.x, out.y) + nR, zo[0], zo[1]);
+        f2_split(f2_make(out.z, out.w) + nR, zo[2], zo[3]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+        {
+            const int q = 4 * g + i;
+            M2[q] = fmaf(-S, S * invL, Q);
+            mn = fminf(mn, M2[q]);
+            Smax = fmaxf(Smax, fabsf(S));
+            if (q < kDenRun - 1)
+            {
+                S += zi[i] - zo[i];
+                Q = fmaf(zi[i], zi[i], fmaf(-zo[i], zo[i], Q));
+                QB = fmaf(zi[i], zi[i], QB);
+            }
+        }
+        cur = nxt;
+    }
+}
 
 // Window variances of length L over channel c's lags [k0, k0 + lpc), one CTA
 // per (lag block, channel) as den_kernel.  den (optional) receives
@@ -74,63 +130,65 @@ struct DenRobustLayout
 // kRunConst, or -1 when the run is unreliable; R; max |window mean - R|; 0),
 // cst one float2 per 32-sample chunk: (mean, sum of squares about it), for
 // the chunks of the CTA's lags (the last CTA: every staged chunk).
-__global__ void __launch_bounds__(kThreads) den_robust_kernel(const float *x, long ldx, int L, float *den, long ldd,
-                                                             float tol, float4 *rstat, long ldrs, float2 *cst,
-                                                             long ldc)
+//
+// Bound by shared-memory loads and issue (data pipe 76 %, issue 69 %; 4 CTAs per
+// SM by registers).  Per lag: 16-byte loads of the samples, demeaned once, and
+// no test of the windows inside the slide (constant or non-finite ones are
+// sorted out per run, below).  72 channels x 1.08 M lags, L = 500: 159 us, its
+// 622 MB take 93; single-word loads with computed addresses, the mean taken off
+// at each use and the tests per lag took 107 instructions per lag and 243 us
+// (now 57; 171 us with 80 registers and 3 CTAs per SM).
+__global__ void __launch_bounds__(kThreads, 4) den_robust_kernel(const float *x, long ldx, int L, float *den, long ldd,
+                                                                float tol, float4 *rstat, long ldrs, float2 *cst,
+                                                                long ldc)
 {
     extern __shared__ __align__(16) unsigned char smem_dr[];
+    constexpr int kRow = DenRobustLayout::kRow;
     const int tid = threadIdx.x, c = blockIdx.y;
     const int R = den_runs_per_thread(L);
     const int nruns = kThreads * R;
     const int lpc = den_lags_per_cta(L);
     const long k0 = (long) blockIdx.x * lpc;
     float *y = reinterpret_cast<float *>(smem_dr);
-    float *cm = reinterpret_cast<float *>(smem_dr + DenRobustLayout::y_bytes(L));
-    float *cs = cm + nruns, *cq = cs + nruns;
-    float *red = cq + nruns;
+    float4 *ck = reinterpret_cast<float4 *>(smem_dr + DenRobustLayout::y_bytes(L));
+    float *red = reinterpret_cast<float *>(ck + nruns);
 
-    // ---- stage 32 * nruns samples (16-byte loads), CTA mean
-    const float *xr = x + (long) c * ldx + k0;
+    // ---- stage 32 * nruns samples, CTA mean
+    const float4 *xr = reinterpret_cast<const float4 *>(x + (long) c * ldx + k0);
     constexpr int NB = 8;
-    const int nvec = nruns * kDenRun / 4;
     MeanAcc<float> macc;
-    for (int i0 = tid; i0 < nvec; i0 += kThreads * NB)
+    for (int i0 = tid; i0 < nruns * (kDenRun / 4); i0 += kThreads * NB)  // a multiple of kThreads * NB
     {
         float4 v[NB];
 #pragma unroll
-        for (int b = 0; b < NB; ++b)
-        {
-            const int i = i0 + b * kThreads;
-            if (i < nvec) v[b] = reinterpret_cast<const float4 *>(xr)[i];
-        }
+        for (int b = 0; b < NB; ++b) v[b] = xr[i0 + b * kThreads];
 #pragma unroll
         for (int b = 0; b < NB; ++b)
         {
             const int i = i0 + b * kThreads;
-            if (i >= nvec) break;
-            const float e[4] = {v[b].x, v[b].y, v[b].z, v[b].w};
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-            {
-                y[den_pad(4 * i + q)] = e[q];
-                macc.add(e[q]);
-            }
+            *reinterpret_cast<float4 *>(y + 4 * i + (i >> 3) * (kRow - kDenRun)) = v[b];
+            macc.add((v[b].x + v[b].y) + (v[b].z + v[b].w));
         }
     }
     const float m = block_mean<float>(macc, red, nruns * kDenRun);
 
-    // ---- chunk statistics about each chunk's own mean
+    // ---- samples less the CTA mean, chunk statistics about each chunk's own mean
     for (int r = 0; r < R; ++r)
     {
         const int j = tid + kThreads * r;
-        const float *yc = y + 33 * j;
+        float4 *yc = reinterpret_cast<float4 *>(y + kRow * j);
+        const f2 nm = f2_dup(-m);
         float v[32];
         float s = 0.f;
 #pragma unroll
-        for (int q = 0; q < 32; ++q)
+        for (int q = 0; q < 32; q += 4)
         {
-            v[q] = yc[q] - m;
-            s += v[q];
+            const float4 e = yc[q >> 2];
+            f2_split(f2_make(e.x, e.y) + nm, v[q], v[q + 1]);
+            f2_split(f2_make(e.z, e.w) + nm, v[q + 2], v[q + 3]);
+            yc[q >> 2] = make_float4(v[q], v[q + 1], v[q + 2], v[q + 3]);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) s += v[q + i];
         }
         const float mu = s * (1.f / 32.f);
         float a = 0.f, b = 0.f;
@@ -141,9 +199,7 @@ __global__ void __launch_bounds__(kThreads) den_robust_kernel(const float *x, lo
             a += d;
             b = fmaf(d, d, b);
         }
-        cm[j] = mu;
-        cs[j] = a;
-        cq[j] = b;
+        ck[j] = make_float4(mu, a, b, 2.f * a);
         if (j < den_lags_per_cta(L) / kDenRun || blockIdx.x == gridDim.x - 1)
             cst[(long) c * ldc + k0 / kDenRun + j] = make_float2(mu + m, fmaf(-a, a * (1.f / 32.f), b));
     }
@@ -154,7 +210,6 @@ __global__ void __launch_bounds__(kThreads) den_robust_kernel(const float *x, lo
     const int Lq = L >> 5, re = L & 31;
     float *drow = den ? den + (long) c * ldd + k0 : nullptr;
     float4 *rs = rstat + (long) c * ldrs + k0 / kDenRun;
-    auto yv = [&](int i) { return y[den_pad(i)] - m; };
     constexpr int CPR = kDenRun / 4;
     float *ob = y;
     const int rounds = (nlr + kThreads - 1) / kThreads;
@@ -167,57 +222,73 @@ __global__ void __launch_bounds__(kThreads) den_robust_kernel(const float *x, lo
         {
             float M2min = kRunConst, Smax = 0.f, Rabs;
             bool bad = false;
-            const int b0 = 32 * v;
+            const float *own = y + kRow * v;
             if (L >= 64)
             {
-                // core [32v + 31, 32v + L): sample 32v + 31, chunks v+1 .. v+Lq-1,
-                // the first re samples of chunk v + Lq
-                const float Rr = cm[v + 1 + (Lq - 1) / 2];
-                float SC = 0.f, QC = 0.f;
-                for (int j = v + 1; j < v + Lq; ++j)
+                // first window [32v, 32v + L): chunks v .. v+Lq-1 and the first
+                // re samples of chunk v + Lq, about a mean of its middle
+                const float Rr = ck[v + 1 + (Lq - 1) / 2].x;
+                const float *in = own + kRow * Lq;
+                float S = 0.f, Q = 0.f, QA = 0.f;
+#pragma unroll 4
+                for (int j = 0; j < Lq; ++j)
                 {
-                    const float d = cm[j] - Rr, sj = cs[j];
-                    SC += fmaf(32.f, d, sj);
-                    QC += fmaf(d, fmaf(32.f, d, 2.f * sj), cq[j]);
+                    const float4 k = ck[v + j];
+                    const float d = k.x - Rr, q = fmaf(d, fmaf(32.f, d, k.w), k.z);
+                    S += fmaf(32.f, d, k.y);
+                    Q += q;
+                    if (j == 0) QA = q;
                 }
+                for (int i = 0; i < re; i += 4)
                 {
-                    const float z = yv(b0 + 31) - Rr;
-                    SC += z;
-                    QC = fmaf(z, z, QC);
-                }
-                for (int i = 0; i < re; ++i)
-                {
-                    const float z = yv(32 * (v + Lq) + i) - Rr;
-                    SC += z;
-                    QC = fmaf(z, z, QC);
-                }
-                // the run's first window adds samples 32v .. 32v + 30
-                float SA = 0.f, QA = 0.f;
-#pragma unroll 8
-                for (int i = 0; i < 31; ++i)
-                {
-                    const float z = yv(b0 + i) - Rr;
-                    SA += z;
-                    QA = fmaf(z, z, QA);
-                }
-                float S = SC + SA, Q = QC + QA, QB = 0.f;
+                    const float4 e = *reinterpret_cast<const float4 *>(in + i);
+                    const float w[4] = {e.x, e.y, e.z, e.w};
 #pragma unroll
-                for (int q = 0; q < kDenRun; ++q)
-                {
-                    const float M2 = fmaf(-S, S * invL, Q);
-                    if (drow) o[q] = M2 > 0.f ? DenOps<float>::out(Lf * M2, sqrtL, tol) : 0.f;
-                    if (M2 > 0.f) M2min = fminf(M2min, M2);
-                    bad |= M2 < 0.f;
-                    Smax = fmaxf(Smax, fabsf(S));
-                    if (q < kDenRun - 1)
+                    for (int k = 0; k < 4; ++k)
                     {
-                        const float zo = yv(b0 + q) - Rr, zi = yv(b0 + q + L) - Rr;
-                        S += zi - zo;
-                        Q = fmaf(zi, zi, fmaf(-zo, zo, Q));
-                        QB = fmaf(zi, zi, QB);
+                        const float z = i + k < re ? w[k] - Rr : 0.f;
+                        S += z;
+                        Q = fmaf(z, z, Q);
                     }
                 }
-                const float slide = QA + QB;
+                float mn = kRunConst, QB = 0.f;
+                switch (re & 3)
+                {
+                case 0: den_slide<0>(own, in, re >> 2, Rr, invL, S, Q, o, mn, Smax, QB); break;
+                case 1: den_slide<1>(own, in, re >> 2, Rr, invL, S, Q, o, mn, Smax, QB); break;
+                case 2: den_slide<2>(own, in, re >> 2, Rr, invL, S, Q, o, mn, Smax, QB); break;
+                default: den_slide<3>(own, in, re >> 2, Rr, invL, S, Q, o, mn, Smax, QB); break;
+                }
+                // a NaN among the M2 stays to the last: S or Q is infinite or
+                // NaN from there on, so the last is NaN too or the least -inf
+                if (Lf * mn > tol * tol && o[kDenRun - 1] == o[kDenRun - 1])
+                {
+                    M2min = mn;
+                    if (drow)
+                    {
+                        const f2 L2 = f2_dup(Lf), s2 = f2_dup(sqrtL);
+#pragma unroll
+                        for (int q = 0; q < kDenRun; q += 2)
+                        {
+                            // DenOps<float>::out for normal numbers above tol^2
+                            float a, b;
+                            f2_split(f2_make(o[q], o[q + 1]) * L2, a, b);
+                            f2_split(f2_make(rsqrt_normal(a), rsqrt_normal(b)) * s2, o[q], o[q + 1]);
+                        }
+                    }
+                }
+                else
+                {
+#pragma unroll
+                    for (int q = 0; q < kDenRun; ++q)
+                    {
+                        const float M2 = o[q];
+                        o[q] = M2 > 0.f ? DenOps<float>::out(Lf * M2, sqrtL, tol) : 0.f;
+                        if (M2 > 0.f) M2min = fminf(M2min, M2);
+                        bad |= M2 < 0.f;
+                    }
+                }
+                const float slide = QA + QB;  // (one leaving sample, the run's last, more than slides)
                 if (M2min < kRunConst) bad |= slide > 100.f * M2min;
                 else bad |= slide > 0.f;
                 Rabs = Rr + m;
@@ -226,17 +297,18 @@ __global__ void __launch_bounds__(kThreads) den_robust_kernel(const float *x, lo
             else
             {
                 // short templates: each window about its own mean
+                auto yv = [&](int i) { return own[i + (i >> 5) * (kRow - kDenRun)]; };
                 float R0 = 0.f;
 #pragma unroll
                 for (int q = 0; q < kDenRun; ++q)
                 {
                     float s = 0.f;
-                    for (int i = 0; i < L; ++i) s += yv(b0 + q + i);
+                    for (int i = 0; i < L; ++i) s += yv(q + i);
                     const float mu = s * invL;
                     float a = 0.f, b = 0.f;
                     for (int i = 0; i < L; ++i)
                     {
-                        const float d = yv(b0 + q + i) - mu;
+                        const float d = yv(q + i) - mu;
                         a += d;
                         b = fmaf(d, d, b);
                     }

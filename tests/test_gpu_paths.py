@@ -48,6 +48,27 @@ def test_listed_runs(gpu, oracle, rng, lens):
     assert _worst(f, oracle, tps, [x] * len(lens)) < FP32_TOL
 
 
+# window variances in runs of 32 lags: every remainder of the length modulo 4,
+# the shortest and longest of one and two runs per thread, a constant stretch
+# inside the data (its windows give exactly 0) next to windows that leave it.
+# Bound: the flagging bound's, as above.
+@pytest.mark.parametrize("L", [64, 65, 66, 67, 93, 95, 96, 128, 500, 501, 4062, 4063, 4064, 4065, 4099])
+def test_window_variances(gpu, oracle, rng, L):
+    n = 30_011
+    x = (rng.standard_normal(n) + 20.0).astype(np.float32)
+    x[9_000:9_000 + L + 777] = 3.0
+    tp = rng.standard_normal(L)
+    f = _filter(gpu, [tp], [0], 1, n, np.float32, correlator_variant=1)
+    f.set_channel_signals(x[None, :])
+    f.apply()
+    r = f.get_valid_matched_filtered_signal(0)
+    assert np.all(r[9_000:9_778] == 0.0)
+    live = np.ones(n - L + 1, bool)
+    live[9_000:9_778] = False
+    ref = oracle.pearson_naive(tp, x)
+    assert float(np.max(np.abs(r.astype(np.float64) - ref)[live])) < FP32_TOL
+
+
 # pruning per trace: traces without a candidate, with more than one CTA
 # prunes (the general rounds take over) and with more candidates in a chunk
 # than its slot holds; separations from none to the trace's length.  Indices
