@@ -25,6 +25,9 @@ from .matched_filter import MatchedFilter
 from .waveform import MatchedFilterDetectionMode, NetworkStationPhase, Polarity
 
 
+_RAW = np.dtype(_lib.MfgpuDetection)  # the records of mfgpu_mf_get_detections
+
+
 class MaximumMatchedFilterPolicy(enum.IntEnum):
     """include/mflib/enums.hpp:53-60."""
     maximum = 0
@@ -268,17 +271,20 @@ class Detection:
         positive."""
         if not value > 0:
             raise ValueError("Scaling factor = %g must be positive" % value)
-        self._amp[RelativeMagnitudeType(int(mag_type))] = float(value)
+        self._amp[int(RelativeMagnitudeType(int(mag_type)))] = float(value)
 
     def get_amplitude_scaling_factor(self, mag_type):
-        return self._get(self._amp.get(RelativeMagnitudeType(int(mag_type))), "Amplitude scaling factor")
+        v = self._amp.get(int(mag_type))  # keys are ints: an enum's hash is a Python call
+        if v is None:
+            RelativeMagnitudeType(int(mag_type))  # refuses anything else
+        return self._get(v, "Amplitude scaling factor")
 
     def have_amplitude_scaling_factor(self, mag_type=None):
         """With a type: that factor is set.  Without one, as pymflib
         (python/singleChannel/detection.cpp:353-362): both factors are set."""
         if mag_type is None:
             return len(self._amp) == len(RelativeMagnitudeType)
-        return RelativeMagnitudeType(int(mag_type)) in self._amp
+        return int(RelativeMagnitudeType(int(mag_type))) in self._amp
 
     def get_magnitude_perturbation(self, mag_type):
         """log10 of the amplitude scaling factor (relativeMagnitude.cpp)."""
@@ -301,7 +307,7 @@ class Detection:
         ident = None if self._id is None else (self._id[0].__getstate__(), self._id[1])
         return {"id": ident, "xc": self._xc, "sig": None if self._sig is None else self._sig.tolist(),
                 "t": self._t, "ti": self._ti, "tt": self._tt, "po": self._po, "poi": self._poi,
-                "amp": {int(k): v for k, v in self._amp.items()}, "pol": int(self._pol)}
+                "amp": dict(self._amp), "pol": int(self._pol)}
 
     def __setstate__(self, st):
         self.clear()
@@ -312,7 +318,7 @@ class Detection:
         self._xc = st["xc"]
         self._sig = None if st["sig"] is None else np.array(st["sig"], dtype=np.float64)
         self._t, self._ti, self._tt, self._po, self._poi = st["t"], st["ti"], st["tt"], st["po"], st["poi"]
-        self._amp = {RelativeMagnitudeType(k): v for k, v in st["amp"].items()}
+        self._amp = {int(RelativeMagnitudeType(k)): v for k, v in st["amp"].items()}
         self._pol = Polarity(st["pol"])
 
 
@@ -372,37 +378,42 @@ class Detector:
         signals = {}
         meta = {}
         pols = {v: Polarity(v) for v in (-1, 0, 1)}
-        for r in raw[: n.value]:
-            it = r.template_index
+        gr, sr = int(RelativeMagnitudeType.gibbons_ringdal_2006), int(RelativeMagnitudeType.schaff_richards_2014)
+        new, out = Detection.__new__, self._dets
+        # one conversion of all records, every field of a Detection set once:
+        # 353 detections in 320 us (with the release of the last ones), 410 with a ctypes
+        # access per field
+        for it, sample, rho, t, ti, sign, have_amp, a_gr, a_sr in np.frombuffer(raw, _RAW, n.value).tolist():
             if it not in meta:
                 wt = templates[it]
-                meta[it] = (wt.get_identifier() if wt.have_identifier() else (NetworkStationPhase(), it),
+                ident = wt.get_identifier() if wt.have_identifier() else (NetworkStationPhase(), it)
+                meta[it] = ((ident[0], int(ident[1])),
                             wt.get_phase_onset_time_in_signal() if wt.have_phase_onset_time() else None,
                             int(wt.get_polarity()),
                             wt.get_phase_travel_time() if wt.have_travel_time() else None,
                             wt.get_signal_length())
             ident, onset, pol, travel, L = meta[it]
-            d = Detection()
-            d._id = (ident[0], int(ident[1]))
-            d._xc = r.correlation  # clamped to [-1, 1] on the device
-            d._t = r.detection_time
-            d._ti = r.interpolated_time
-            if onset is not None:
-                d._po = r.detection_time + onset
-                d._poi = r.interpolated_time + onset
-            d._pol = pols[r.sign * pol]
-            if travel is not None:
-                d._tt = travel
-            if r.have_amplitude:
-                d._amp = {RelativeMagnitudeType.gibbons_ringdal_2006: r.gibbons_ringdal,
-                          RelativeMagnitudeType.schaff_richards_2014: r.schaff_richards}
+            d = new(Detection)
+            d._id = ident
+            d._xc = rho  # clamped to [-1, 1] on the device
+            d._sig = None
+            d._t = t
+            d._ti = ti
+            d._tt = travel
+            if onset is None:
+                d._po = d._poi = None
+            else:
+                d._po = t + onset
+                d._poi = ti + onset
+            d._amp = {gr: a_gr, sr: a_sr} if have_amp else {}
+            d._pol = pols[sign * pol]
             if want_wave:
                 # single-channel objects hold one signal (slot 0)
                 slot = 0 if mf._params.get_detection_mode() == MatchedFilterDetectionMode.single_channel else it
                 if slot not in signals:
                     signals[slot] = MatchedFilter.get_signal(mf, slot)
-                d.set_detected_signal(signals[slot][r.sample:r.sample + L])
-            self._dets.append(d)
+                d.set_detected_signal(signals[slot][sample:sample + L])
+            out.append(d)
         return self
 
     def get_number_of_detections(self):

@@ -138,7 +138,7 @@ def unpack_detection(rec, signal=None, det=None):
     # public setters refuse
     for i, t in enumerate(_AMP):
         if r["have_amplitude%d" % (i + 1)]:
-            det._amp[t] = float(r["amplitude%d" % (i + 1)])
+            det._amp[int(t)] = float(r["amplitude%d" % (i + 1)])
     if r["have_correlation_coefficient"]:
         det._xc = float(r["correlation_coefficient"])
     for f, attr in _TIME_ATTRS:
