@@ -941,7 +941,11 @@ try
         // automatic choice: seconds per template-lag measured on GB300 (two
         // MMAs per K step), about 3.6e-15 per padded template sample plus
         // 5.7e-12 per tile row shared by the Gp templates of a group, against
-        // the FFT plan's estimate
+        // the FFT plan's estimate.  With the epilogue in four warpgroups the
+        // form beats the FFT beyond this line (12 channels x 540,000, 4
+        // templates of 200 each: 120 against 138 us; 8 of 400: 165 against
+        // 187), but its coefficients err twice as much (5.5e-7 of their norm
+        // against 2.3e-7), so calls past the line keep the FFT's accuracy.
         if (!mf->tc && gmax >= 2)
             mf->tc = 3.6e-15 * Kp + 5.7e-12 / Gp < 0.9 * fft_cost_per_lag;
     }

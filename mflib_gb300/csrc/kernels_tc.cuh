@@ -24,13 +24,21 @@
 // Persistent, warp-specialised CTA (one per SM):
 //   warp 0 lane 0   issues the MMAs (K/16 steps x 2) and the commits;
 //   warps 1-3       stage strips: FP32 load, offset, scale, hi/lo split;
-//   warps 4-11      epilogue, two warpgroups taking alternate templates:
+//   warps 4-19      epilogue, four warpgroups taking every fourth template:
 //                   tcgen05.ld of the accumulator rows (the buffer is
-//                   released before the stores), scales, normalisation row
-//                   (prefetched a tile ahead), |rho| > 1.1 clamp, 32-byte
-//                   stores.
+//                   released before the stores), scales (a lane per template,
+//                   renewed with the group), normalisation row (prefetched a
+//                   tile ahead), |rho| > 1.1 clamp, 32-byte stores.
 // Strips and accumulators are double-buffered (mbarriers, bounded waits);
 // the group's template operands stay resident in shared memory.
+//
+// Bound by the epilogue's latency and the coefficient writes at short
+// templates (24 channels x 1.08 M lags, 384 templates of 200: 362 us, 16 per
+// group; the writes alone take 248 at the measured copy rate, the MMAs 216 at
+// the nominal one).  With two epilogue warpgroups (two warps per scheduler), 64-bit
+// divisions for the tile's place, template numbers and scales loaded and divided
+// per template and each coefficient clamped on its own: 659 us.  Loads of the
+// next template's accumulators issued ahead of the current one's stores: 376.
 //
 // BF16 operands (template flag BF, an option): the same kernel with BF16 hi
 // and lo (about 16 of the 24 bits kept, against 22 for FP16; BF16's
@@ -161,6 +169,21 @@ __global__ void __launch_bounds__(256) tc_bank_kernel(const double *tmpl, const 
     }
 }
 
+// tile w: group g, tile j of its channel
+struct TcTile
+{
+    int g, j;
+    __device__ __forceinline__ TcTile(long w, int tiles) : g((int) (w / tiles)), j((int) (w % tiles)) {}
+    __device__ __forceinline__ void next(int tiles)
+    {
+        if (++j == tiles)
+        {
+            j = 0;
+            ++g;
+        }
+    }
+};
+
 template <bool BF>
 __global__ void __launch_bounds__(kTcThreads, 1) tc_xcorr_kernel(TcParams p)
 {
@@ -212,9 +235,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_xcorr_kernel(TcParams p)
             uint32_t bph = 0;
             bool ok = true;
             long issued = 0;
-            for (long w = w0, n = 0; w < w1 && ok; ++w, ++n)
+            TcTile at(w0, p.tiles);
+            for (long w = w0, n = 0; w < w1 && ok; ++w, ++n, at.next(p.tiles))
             {
-                const int g = (int) (w / p.tiles);
+                const int g = at.g;
                 const int buf = (int) (n & 1);
                 if (g != cur)
                 {
@@ -260,9 +284,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_xcorr_kernel(TcParams p)
         // ---- strips: x[k0, k0 + 1024 + Kp) -> (x - off) * s -> FP16 hi, lo
         const int ptid = tid - 32;
         bool ok = true;
-        for (long w = w0, n = 0; w < w1; ++w, ++n)
+        TcTile at(w0, p.tiles);
+        for (long w = w0, n = 0; w < w1; ++w, ++n, at.next(p.tiles))
         {
-            const int g = (int) (w / p.tiles), j = (int) (w % p.tiles);
+            const int g = at.g, j = at.j;
             const int buf = (int) (n & 1);
             if (n >= 2 && ok)
             {
@@ -314,22 +339,24 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_xcorr_kernel(TcParams p)
     else
     {
         // ---- epilogue: row i of the tile = TMEM lane i; warpgroup eg takes
-        //      templates eg, eg + 2, ...
+        //      templates eg, eg + 4, ...
+        constexpr int NG = kTcEpiWarps / 4;
         const int q = warp & 3, i = 32 * q + lane, eg = (warp - 4) >> 2;
         constexpr int TB = 2;  // templates per batch of TMEM loads (two halves each)
-        float dv[8];
-        auto load_den = [&](long w) {
-            const int c = p.grp_chan[(int) (w / p.tiles)];
-            const long lag0 = (long) (w % p.tiles) * kTcLags + 8 * i;
-            const float4 d0 = *reinterpret_cast<const float4 *>(p.den + (long) c * p.ldd + lag0);
-            const float4 d1 = *reinterpret_cast<const float4 *>(p.den + (long) c * p.ldd + lag0 + 4);
-            dv[0] = d0.x; dv[1] = d0.y; dv[2] = d0.z; dv[3] = d0.w;
-            dv[4] = d1.x; dv[5] = d1.y; dv[6] = d1.z; dv[7] = d1.w;
+        float4 dv[2];
+        auto load_den = [&](const TcTile &a) {
+            const float4 *d = reinterpret_cast<const float4 *>(p.den + (long) p.grp_chan[a.g] * p.ldd +
+                                                               (long) a.j * kTcLags + 8 * i);
+            dv[0] = d[0];
+            dv[1] = d[1];
         };
-        if (w0 < w1) load_den(w0);
+        TcTile at(w0, p.tiles);
+        if (w0 < w1) load_den(at);
+        const int nmine = (Gp - eg + NG - 1) / NG;  // templates eg, eg + NG, ... below Gp
+        int cur = -1, my_t = -1;                    // lane t: template of the group's slot t and its scale
+        float my_sc = 0.f;
         for (long w = w0, n = 0; w < w1; ++w, ++n)
         {
-            const int g = (int) (w / p.tiles), j = (int) (w % p.tiles);
             const int buf = (int) (n & 1);
             if (!mbar_wait_bounded(&acc_full[buf], (uint32_t) ((n >> 1) & 1)))
             {
@@ -337,14 +364,19 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_xcorr_kernel(TcParams p)
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const int c = p.grp_chan[g];
-            const long lag0 = (long) j * kTcLags + 8 * i;
-            const float s = tc_pow2_scale(p.xrange[c], 13);
-            const bool dead = p.dead[c] != 0;
-            float dcur[8];
-#pragma unroll
-            for (int f = 0; f < 8; ++f) dcur[f] = dv[f];
-            const int nmine = (Gp - eg + 1) / 2;  // templates eg, eg + 2, ... below Gp
+            if (at.g != cur)
+            {
+                cur = at.g;
+                const int c = p.grp_chan[cur];
+                const float s = tc_pow2_scale(p.xrange[c], 13);
+                my_t = lane < Gp ? p.grp_tid[cur * Gp + lane] : -1;
+                // a dead channel's tiles store zeros (scale 0, no flags)
+                my_sc = lane < Gp && !p.dead[c] ? p.bscale[cur * Gp + lane] / s : 0.f;
+            }
+            const long lag0 = (long) at.j * kTcLags + 8 * i;
+            const f2 dcur[4] = {f2_make(dv[0].x, dv[0].y), f2_make(dv[0].z, dv[0].w), f2_make(dv[1].x, dv[1].y),
+                                f2_make(dv[1].z, dv[1].w)};
+            at.next(p.tiles);
             bool released = false;
             for (int b0 = 0; b0 < nmine; b0 += TB)
             {
@@ -354,7 +386,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_xcorr_kernel(TcParams p)
                 {
                     if (b0 + u < nmine)  // uniform across the warp
                     {
-                        const int t = eg + 2 * (b0 + u);
+                        const int t = eg + NG * (b0 + u);
                         const uint32_t taddr = tmem + ((uint32_t) (32 * q) << 16) + (uint32_t) (buf * 2 * N + 8 * t);
                         asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                                      : "=r"(r[u][0]), "=r"(r[u][1]), "=r"(r[u][2]), "=r"(r[u][3]), "=r"(r[u][4]),
@@ -376,40 +408,46 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_xcorr_kernel(TcParams p)
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&acc_empty[buf]);
                     released = true;
-                    if (w + 1 < w1) load_den(w + 1);
+                    if (w + 1 < w1) load_den(at);
                 }
 #pragma unroll
                 for (int u = 0; u < TB; ++u)
                 {
                     if (b0 + u >= nmine) break;
-                    const int t = eg + 2 * (b0 + u);
-                    const int tt = p.grp_tid[g * Gp + t];
+                    const int t = eg + NG * (b0 + u);
+                    const int tt = __shfl_sync(0xffffffffu, my_t, t);
+                    const f2 sc = f2_dup(__shfl_sync(0xffffffffu, my_sc, t));
                     if (tt < 0) continue;
-                    // a dead channel's tiles store zeros (sc = 0, no flags)
-                    const float sc = dead ? 0.f : p.bscale[g * Gp + t] / s;
                     float o[8];
 #pragma unroll
-                    for (int f = 0; f < 8; ++f)
-                        o[f] = clamp_rho((__uint_as_float(r[u][f]) + __uint_as_float(h[u][f])) * sc * dcur[f]);
-                    if (p.pk_flags)
+                    for (int f = 0; f < 4; ++f)
                     {
-                        // one bit per 64 lags (8 rows); values above the
-                        // threshold are rare, so each such row sets its bit
-                        // itself, without a warp-wide vote; the lag bound
-                        // matters only in the last tile
-                        float mx = o[0];
+                        const f2 v = (f2_make(__uint_as_float(r[u][2 * f]), __uint_as_float(r[u][2 * f + 1])) +
+                                      f2_make(__uint_as_float(h[u][2 * f]), __uint_as_float(h[u][2 * f + 1])));
+                        f2_split(v * sc * dcur[f], o[2 * f], o[2 * f + 1]);
+                    }
+                    // clamp_rho of all eight where the largest needs it (rare)
+                    float mx = fabsf(o[0]);
 #pragma unroll
-                        for (int f = 1; f < 8; ++f) mx = fmaxf(mx, o[f]);
-                        if (mx > p.pk_thr)
+                    for (int f = 1; f < 8; ++f) mx = fmaxf(mx, fabsf(o[f]));
+                    if (mx > 1.1f)
+                    {
+#pragma unroll
+                        for (int f = 0; f < 8; ++f) o[f] = clamp_rho(o[f]);
+                    }
+                    // one bit per 64 lags (8 rows); values above the threshold
+                    // are rare, so each such row sets its bit itself, without
+                    // a warp-wide vote; the lag bound matters only in the last
+                    // tile
+                    if (p.pk_flags && (mx > p.pk_thr || p.pk_thr < 0.f))
+                    {
+                        bool above = false;
+#pragma unroll
+                        for (int f = 0; f < 8; ++f) above |= lag0 + f < p.nv && o[f] > p.pk_thr;
+                        if (above)
                         {
-                            bool above = false;
-#pragma unroll
-                            for (int f = 0; f < 8; ++f) above |= lag0 + f < p.nv && o[f] > p.pk_thr;
-                            if (above)
-                            {
-                                const long c = lag0 >> 6;
-                                atomicOr(p.pk_flags + (long) tt * p.pk_words + (c >> 5), 1u << (c & 31));
-                            }
+                            const long c = lag0 >> 6;
+                            atomicOr(p.pk_flags + (long) tt * p.pk_words + (c >> 5), 1u << (c & 31));
                         }
                     }
                     float *dst = p.rho + (long) tt * p.ldr + lag0;
@@ -435,7 +473,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_xcorr_kernel(TcParams p)
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&acc_empty[buf]);
-                if (w + 1 < w1) load_den(w + 1);
+                if (w + 1 < w1) load_den(at);
             }
         }
     }

@@ -8,9 +8,9 @@ namespace mfgpu {
 
 constexpr int kTcRows = 128;              // MMA M: rows of a tile
 constexpr int kTcLags = 8 * kTcRows;      // lags per tile (8 phases per row)
-constexpr int kTcThreads = 384;           // warp 0 MMA issue, warps 1-3 strips, warps 4-11 epilogue
+constexpr int kTcThreads = 640;           // warp 0 MMA issue, warps 1-3 strips, warps 4-19 epilogue
 constexpr int kTcProducers = 96;
-constexpr int kTcEpiWarps = 8;            // two warpgroups, each covering the 128 rows
+constexpr int kTcEpiWarps = 16;           // four warpgroups, each covering the 128 rows
 
 struct TcParams
 {

@@ -69,6 +69,30 @@ def test_window_variances(gpu, oracle, rng, L):
     assert float(np.max(np.abs(r.astype(np.float64) - ref)[live])) < FP32_TOL
 
 
+# tensor-core form: groups whose templates the four epilogue warpgroups share
+# unevenly or not at all, partly filled groups, a tile of one lag, a dead
+# channel.  Bound: the flagging bound's, as above.
+@pytest.mark.parametrize("group,per", [(2, 1), (2, 3), (4, 3), (6, 6), (10, 9), (16, 15), (16, 18)])
+def test_tensor_epilogue(gpu, oracle, rng, group, per):
+    L, nch = 96, 3
+    n = 5 * 1024 + L  # lags 0 .. 5 * 1024
+    x = (rng.standard_normal((nch, n)) + 5.0).astype(np.float32)
+    x[1] = 2.0
+    tps = [rng.standard_normal(L) for _ in range(nch * per)]
+    chan = [t % nch for t in range(nch * per)]
+    for t in (0, nch * per - 1):  # coefficients near 1 and -1
+        x[chan[t], 2000 + 7 * t:2000 + 7 * t + L] = (1 - 2 * (t & 1)) * 40.0 * tps[t] + 5.0
+    f = _filter(gpu, tps, chan, nch, n, np.float32, correlator_variant=4, tc_group=group)
+    f.set_channel_signals(x)
+    f.apply()
+    for t in range(nch * per):
+        r = f.get_valid_matched_filtered_signal(t)
+        if chan[t] == 1:
+            assert np.all(r == 0.0)
+        else:
+            assert float(np.max(np.abs(r.astype(np.float64) - oracle.pearson_naive(tps[t], x[chan[t]])))) < FP32_TOL
+
+
 # pruning per trace: traces without a candidate, with more than one CTA
 # prunes (the general rounds take over) and with more candidates in a chunk
 # than its slot holds; separations from none to the trace's length.  Indices
