@@ -69,6 +69,27 @@ def test_window_variances(gpu, oracle, rng, L):
     assert float(np.max(np.abs(r.astype(np.float64) - ref)[live])) < FP32_TOL
 
 
+# work groups: channels with one template, uneven counts, more CTAs than one
+# wave holds with the last channels split finer.  Every template's row is
+# compared (a template in no group, or in two of one channel, shows).
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("per,n", [((1,), 3000), ((1, 0, 5, 33), 3000), ((31,) * 12 + (32,) * 4, 42_000), ((7, 64, 3), 90_000)])
+@pytest.mark.parametrize("equal", [False, True])
+def test_work_groups(gpu, oracle, rng, dtype, per, n, equal):
+    x = rng.standard_normal((len(per), n)).astype(dtype)
+    chan = [c for c, m in enumerate(per) for _ in range(m)]
+    lens = [300 if equal else 200 + 13 * (t % 31) for t in range(len(chan))]
+    tps = [rng.standard_normal(L) for L in lens]
+    f = _filter(gpu, tps, chan, len(per), n, dtype)
+    f.set_channel_signals(x)
+    f.apply()
+    for t in range(0, len(tps), 1 if n < 10_000 else 7):
+        r = f.get_valid_matched_filtered_signal(t).astype(np.float64)
+        assert float(np.max(np.abs(r - oracle.pearson_naive(tps[t], x[chan[t]])))) < (FP32_TOL if dtype == np.float32 else 1e-12)
+    for t in range(len(tps)):  # rows written to the end
+        assert np.any(f.get_valid_matched_filtered_signal(t)[-32:] != 0)
+
+
 # tensor-core form: groups whose templates the four epilogue warpgroups share
 # unevenly or not at all, partly filled groups, a tile of one lag, a dead
 # channel.  Bound: the flagging bound's, as above.
