@@ -15,7 +15,7 @@ constexpr int kIntBBits = 53;     // fraction bits of a template coefficient
 constexpr float kIntNormBits = 55.1f;  // a block's windows: 2-norm below 2^55.1, so that a numerator stays below
                                        // 2^108.1 and half the primes' product (2^108.19)
 
-// One prime: c25, rrn and crt are times R = 2^32 modulo p; all in [0, p).
+// One prime: c25 and rrn are times R = 2^32 modulo p; all in [0, p).
 struct IntPrime
 {
     unsigned p, nq;                 // nq = -p^-1 mod 2^32
@@ -23,8 +23,8 @@ struct IntPrime
     unsigned inv;                   // floor(2^32 / p)
     unsigned w[10], ws[10];         // powers of the 16th root, floor(w 2^32 / p)
     unsigned c25;                   // 2^25
-    unsigned rrn;                   // R / N (a product with it gives a value times R / N)
-    unsigned crt;                   // (M / p)^-1, M the product of the primes
+    unsigned rrn;                   // R / N (M / p)^-1, M the product of the primes (a product with it gives a
+                                    // value times that)
     unsigned f0, f1, f2;            // floor(2^96 / p), low word first
 };
 struct IntConsts

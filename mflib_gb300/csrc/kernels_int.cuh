@@ -332,7 +332,7 @@ __device__ __forceinline__ int int_quantise(long long (&v)[PER], int *ired, long
 // ---- template table -----------------------------------------------------------
 // One CTA per (template, prime): B[t][prime][k] = transform of round(b 2^53),
 // b the demeaned unit-norm template (FP64, as template_spectra_kernel), times
-// R / N modulo p, in [0, p).
+// R / N (M / p)^-1 modulo p, in [0, p).
 __global__ void __launch_bounds__(256) int_bank_kernel(IntBankParams p)
 {
     __shared__ double red[8];
@@ -595,9 +595,9 @@ template <bool MULTI, int T> __global__ void __launch_bounds__(T / 8, T == 4096 
 //
 // Bound by the integer pipes (multiplier and ALU; issue 2 of 4 per clock).  160
 // templates of 200 .. 2,000 samples against 8 channels x 360,000: 8.35 ms (FP64
-// transforms with in-block normalisation) -> 1.73 ms + 0.42 ms normalisation;
+// transforms with in-block normalisation) -> 1.71 ms + 0.42 ms normalisation;
 // 64 channels x 360,000 with one template of 500 each: 2.69 + 1.15 (den_kernel)
-// -> 0.87 + 0.31 ms.  Signed words with centred residues took 2.14 and 0.98 ms.
+// -> 0.84 + 0.31 ms.  Signed words with centred residues took 2.14 and 0.98 ms.
 struct IntLayout
 {
     static constexpr size_t off_red = 64;                    // after the barrier: reductions
@@ -608,9 +608,9 @@ struct IntLayout
     static constexpr size_t bytes = off_tw + sizeof(int) * kIntPrimes * kIntTw;
 };
 
-// numerator / M as a signed 64-bit fraction, from the residues r (any 32 bits):
-// sum of y_i / p_i modulo 1, y_i = r_i (M / p_i)^-1 mod p_i, with 1 / p_i to 96
-// bits
+// numerator / M as a signed 64-bit fraction: sum of y_i / p_i modulo 1 with
+// 1 / p_i to 96 bits, from r_i = y_i mod p_i (any 32 bits), y_i the numerator
+// times (M / p_i)^-1, a factor that the template table carries
 __device__ __forceinline__ long long int_fraction(const IntConsts &c, const unsigned (&r)[kIntPrimes])
 {
     unsigned long long t0 = 1ull << 31, t1 = 0;  // rounds to nearest: a numerator of 0 stays 0
@@ -618,7 +618,7 @@ __device__ __forceinline__ long long int_fraction(const IntConsts &c, const unsi
 #pragma unroll
     for (int i = 0; i < kIntPrimes; ++i)
     {
-        const unsigned y = mont(r[i], c.prime[i].crt, c.prime[i].p, c.prime[i].nq);
+        const unsigned y = r[i] - __umulhi(r[i], c.prime[i].inv) * c.prime[i].p;  // below 2 p
         t0 += (unsigned long long) y * c.prime[i].f0;
         t1 += (unsigned long long) y * c.prime[i].f1;
         t2 += y * c.prime[i].f2;
@@ -641,6 +641,16 @@ __device__ __forceinline__ double int_to_double(long long v, int e)
     else if (E > 2045) bits = 0x7ff0000000000000ull;
     return __longlong_as_double((long long) (bits | ((unsigned long long) v & (1ull << 63))));
 }
+
+// clamp_rho and v > thr >= 0 on the bit patterns (a comparison in FP64 costs
+// 19 clocks per warp and SM, as much as the product before it)
+__device__ __forceinline__ long long int_clamp(long long v)
+{
+    constexpr long long inf = 0x7ff0000000000000ll, lim = 0x3ff199999999999all;  // 1.1
+    const long long m = v & 0x7fffffffffffffffll;
+    return m > lim && m <= inf ? 0 : v;  // a NaN stays
+}
+__device__ __forceinline__ bool int_above(long long v, long long thr) { return v > thr && v <= 0x7ff0000000000000ll; }
 
 template <bool SHARED_DEN> __global__ void __launch_bounds__(kIntThreads, 1) int_xcorr_kernel(IntParams p)
 {
@@ -739,6 +749,7 @@ template <bool SHARED_DEN> __global__ void __launch_bounds__(kIntThreads, 1) int
         for (int r = 0; r < 16; ++r) xt[q + 256 * r] = a[r];  // read by this thread only
     }
     const bool pk = x.pk_on != 0;
+    const long long thr = __double_as_longlong(x.pk_thr + 0.0);  // (not -0)
     int t_prev = -1;
     for (int ti = t_begin; ti < t_end; ++ti)
     {
@@ -758,21 +769,21 @@ template <bool SHARED_DEN> __global__ void __launch_bounds__(kIntThreads, 1) int
         int_ntt<false>(f, a, s, tw, q, bar_id);
 #pragma unroll
         for (int r = 0; r < 16; ++r) s[q + 256 * r] = a[r];
-        __syncthreads();
         const long nv = x.nvalid[t];
         const int kmax = (int) (nv - k0 < (long) S ? nv - k0 : (long) S);
         double *dst = x.rho + (long) t * x.ldr + k0;
         const double *den = SHARED_DEN ? x.den + (long) c * x.ldd + k0 : dst;
         unsigned *mk = Mk + (it & 1) * 2;
+        __syncthreads();
 #pragma unroll 2
         for (int k = tid; k < kmax; k += kIntThreads)
         {
             const double inv = den[k];
             const unsigned rs[kIntPrimes] = {buf[k], buf[kIntN + k], buf[2 * kIntN + k], buf[3 * kIntN + k]};
             // (the factor M / 2^64 2^-53 is in the normalisation)
-            const double r = clamp_rho(int_to_double(int_fraction(p.c, rs), ex) * inv);
-            dst[k] = r;
-            if (pk && r > x.pk_thr) atomicOr(mk + (k >> 11), 1u << ((k >> 6) & 31));
+            const long long r = int_clamp(__double_as_longlong(int_to_double(int_fraction(p.c, rs), ex) * inv));
+            dst[k] = __longlong_as_double(r);
+            if (pk && int_above(r, thr)) atomicOr(mk + (k >> 11), 1u << ((k >> 6) & 31));
         }
         t_prev = t;
     }

@@ -90,7 +90,7 @@ struct Tables
             uint64_t m = 1;
             for (int k = 0; k < kIntPrimes; ++k)
                 if (k != i) m = m * (pr[k] % pr[i]) % pr[i];
-            c.prime[i].crt = mont_of(pow_mod(m, pr[i] - 2, pr[i]), (uint32_t) pr[i]);
+            c.prime[i].rrn = (unsigned) (c.prime[i].rrn * pow_mod(m, pr[i] - 2, pr[i]) % pr[i]);
         }
         scale = std::ldexp(M, -64 - kIntBBits);
     }
