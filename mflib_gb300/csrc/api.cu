@@ -809,9 +809,14 @@ try
     const int maxb = p->length_buckets > 0 ? p->length_buckets : 3;
     if (p->length_buckets < 0) return fail(MFGPU_EINVAL, "length_buckets must be >= 0");
     // FP64 data take the integer correlator unless the caller asks for an FFT
-    // plan (a length, an organisation, several buckets)
+    // plan (a length, an organisation, several buckets), or a bank of several
+    // lengths in buckets of its own lags per block costs the transforms less.
+    // A (template, block) takes 78 ns against 302 for the FP64 transforms (160
+    // templates of 200 .. 2,000 samples, 8 channels x 360,000), so that takes
+    // a few templates much longer than the others.
     mf->intx = mf->prec == 8 && ntf > 0 && v == 0 && p->fft_length == 0 && !bucket_forced && p->length_buckets <= 1;
-    if (!mf->intx && !all_equal && p->fft_length == 0 && (forced_mode <= 1 || forced_mode == 4) && maxb > 1)
+    const int int_S = ((kIntN - maxLen + 1) / 32) * 32;
+    if (!all_equal && p->fft_length == 0 && (forced_mode <= 1 || forced_mode == 4) && maxb > 1)
     {
         std::vector<int> pos{0};
         for (int q = 1; q < 64; ++q)
@@ -849,7 +854,13 @@ try
         // 2,000-template bank the model predicted 10 % for two buckets at N =
         // 8192 and GB300 measured 1 %; for three, 10 % and -4 %)
         if (p->length_buckets == 0 && dp[bk][M - 1] > 0.85 * dp[1][M - 1]) bk = 1;
-        if (dp[bk][M - 1] < 1e299 && bk > 1)
+        if (mf->intx && bk > 1)
+        {
+            // in the units of plan_for: 18.8e-9 s per (template, block) at N = 4096
+            const double nb = std::ceil((double) maxvalid_f / int_S);
+            mf->intx = 0.26 * 18.8e-9 * nb * ntf <= dp[bk][M - 1];
+        }
+        if (!mf->intx && dp[bk][M - 1] < 1e299 && bk > 1)
         {
             cuts.assign(1, ntf);
             for (int k = bk, b = M - 1; k > 0; b = from[k][b], --k) cuts.push_back(pos[from[k][b]]);
@@ -864,7 +875,7 @@ try
         if (is_direct[t]) bucket_of[t] = -1;  // in no FFT plan
     const int mv0 = ntf > 0 ? n - mf->lens[order[cuts[nbk - 1]]] + 1 : 0;
     const PlanPick best =
-        mf->intx ? PlanPick{11, ((kIntN - maxLen + 1) / 32) * 32, 0, 0.0}
+        mf->intx ? PlanPick{11, int_S, 0, 0.0}
                  : plan_for(maxLen, nbk > 1 ? mv0 : maxvalid_f, all_equal, bucket_nfft(nbk - 1), bucket_mode(nbk - 1));
     if (best.l2p < 0 && (bucket_nfft(nbk - 1) > 0 || bucket_mode(nbk - 1) >= 0))
         return fail(MFGPU_EINVAL, "the plan override of bucket " + std::to_string(nbk - 1) + " does not fit");

@@ -90,6 +90,20 @@ def test_work_groups(gpu, oracle, rng, dtype, per, n, equal):
         assert np.any(f.get_valid_matched_filtered_signal(t)[-32:] != 0)
 
 
+# FP64 banks of several lengths: integers, or buckets of FP64 transforms where
+# one template would leave the others few lags per block.
+@pytest.mark.parametrize("lens,integer", [((200,) * 20 + (4000,), False), ((200, 400, 3000) * 5, True), ((4065, 60), True)])
+def test_integer_or_buckets(gpu, oracle, rng, lens, integer):
+    n = 30_000
+    x = rng.standard_normal((1, n))
+    tps = [rng.standard_normal(L) for L in lens]
+    f = _filter(gpu, tps, [0] * len(lens), 1, n, np.float64)
+    f.set_channel_signals(x)
+    f.apply()
+    assert (f.get_plan()["correlator"] == 7) == integer
+    assert _worst(f, oracle, tps, [x[0]] * len(lens)) < 1e-12
+
+
 # tensor-core form: groups whose templates the four epilogue warpgroups share
 # unevenly or not at all, partly filled groups, a tile of one lag, a dead
 # channel.  Bound: the flagging bound's, as above.
