@@ -203,12 +203,25 @@ __global__ void stack_kernel(const T *rho, long ldr, int nt, const int *shifts, 
 {
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= outlen) return;
+    // FP64: eight rows in flight per thread, as the few CTAs (1,399 at 64 rows
+    // x 360,000) wait for one row after the other: 99 -> 52 us, 43 of which the
+    // FP64 pipe takes.  FP32: 72 rows x 1.08 M take 53 us row by row, at 5.9 TB/s;
+    // in batches of 2, 4 and 8 rows 93, 69 and 59.
+    constexpr int NB = sizeof(T) == 8 ? 8 : 1;
     T acc = 0;
-    for (int t = 0; t < nt; ++t)
+    for (int t0 = 0; t0 < nt; t0 += NB)
     {
-        long lag = (long) k + shifts[t];
-        T v = lag >= 0 ? rho[(long) t * ldr + lag] : (T) 0;
-        acc = acc + weights[t] * (stack_abs ? (T) fabs(v) : v);
+        T v[NB];
+#pragma unroll
+        for (int i = 0; i < NB; ++i)
+        {
+            const int t = t0 + i;
+            const long lag = t < nt ? (long) k + shifts[t] : -1;
+            v[i] = lag >= 0 ? rho[(long) t * ldr + lag] : (T) 0;
+        }
+#pragma unroll
+        for (int i = 0; i < NB; ++i)
+            if (t0 + i < nt) acc = acc + weights[t0 + i] * (stack_abs ? (T) fabs(v[i]) : v[i]);
     }
     out[k] = acc;
 }

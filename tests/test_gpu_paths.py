@@ -128,6 +128,36 @@ def test_tensor_epilogue(gpu, oracle, rng, group, per):
             assert float(np.max(np.abs(r.astype(np.float64) - oracle.pearson_naive(tps[t], x[chan[t]])))) < FP32_TOL
 
 
+# shift and stack in batches of eight rows: remainders of a batch, shifts
+# before the first lag.  Sums of at most nt coefficients of magnitude 1 in the
+# data type, weights that sum to 1: nt roundings.
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("nt", [1, 7, 8, 9, 17])
+def test_stack_batches(gpu, oracle, rng, dtype, nt):
+    n, L = 5003, 64
+    x = rng.standard_normal((nt, n)).astype(dtype)
+    p = gpu.MultiChannel.MatchedFilterParameters()
+    shifts = [7 * t for t in range(nt)]
+    for t in range(nt):
+        w = gpu.WaveformTemplate()
+        w.set_signal(rng.standard_normal(L))
+        w.set_sampling_rate(100.0)
+        w.set_phase_travel_time(1.0 + shifts[t] / 100.0)
+        w.set_phase_onset_time_in_signal(1.0 if t else 0.0)
+        p.add_template(w)
+    shifts[0] += 100
+    p.set_signal_size(n)
+    f = gpu.MultiChannel.MatchedFilter(dtype=dtype)
+    f.initialize(p)
+    f.set_channel_signals(x)
+    f.apply()
+    rows = [f.get_matched_filtered_signal(t).astype(np.float64) for t in range(nt)]
+    ref = oracle.shift_and_stack(rows, rows[0].size, shifts, [1] * nt)
+    out = f.shift_and_stack()
+    assert out.size == ref.size
+    assert float(np.max(np.abs(out.astype(np.float64) - ref))) <= (nt + 2) * np.finfo(dtype).eps
+
+
 # pruning per trace: traces without a candidate, with more than one CTA
 # prunes (the general rounds take over) and with more candidates in a chunk
 # than its slot holds; separations from none to the trace's length.  Indices
