@@ -1123,7 +1123,7 @@ try
         s2 = mf->prec == 4 ? mf_upload_tables<float>(mf, xb.log2p, xb.tw, xb.Bc, xb.mode == 4 ? &xb.tws : nullptr)
                            : mf_upload_tables<double>(mf, xb.log2p, xb.tw, xb.Bc);
         if (s2 != MFGPU_OK) return s2;
-        const Groups &gr = gx[b];
+        const WorkGroups &gr = gx[b];
         CU(xb.grp_chan.ensure(sizeof(int) * gr.gch.size()));
         CU(xb.grp_tb.ensure(sizeof(int) * gr.gch.size()));
         CU(xb.grp_te.ensure(sizeof(int) * gr.gch.size()));
