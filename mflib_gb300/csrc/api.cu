@@ -2547,7 +2547,7 @@ try
                                      min_distance, mf->pk, mf->stream, &mf->launches, mf->pk_off.data(), err,
                                      fused ? &fd : nullptr, nullptr, 0, mf->err.as<int>(), &dev_err);
     if (rc != 0) return fail(MFGPU_ECUDA, err);
-    if (dev_err != 0 || mf->pk.dense)
+    if (dev_err != 0)
     {
         mfgpu_status st = mf_sync(mf);
         if (st != MFGPU_OK) return st;

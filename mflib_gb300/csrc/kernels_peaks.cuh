@@ -324,31 +324,9 @@ static __global__ void peak_trace_beg_kernel(int ntr, int nchunks, const long lo
 // Candidates gathered by the correlator.  Chunk b of a trace is correlator
 // block b, lags [b*S, b*S + S): the correlator decided the body lags
 // [b*S+1, b*S+S-2] from the values it stored (count body_cnt, up to kPkCap
-// unordered slot entries, indexed by row * nblk + b); the seam kernel
-// decides the first and last lag of each block from the stored trace and
-// forms the chunk's total count.
-template <class T>
-static __global__ void peak_seam_kernel(PeakTraces<T> tr, int ntr, FusedSlots<T> fs, int *counts, unsigned char *ht)
-{
-    const long g = (long) blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= (long) ntr * fs.nblk) return;
-    const int trace = (int) (g / fs.nblk), b = (int) (g % fs.nblk);
-    const int row = tr.row[trace];
-    if (fs.row_nblk && b >= fs.row_nblk[row])
-    {
-        counts[g] = 0;  // past the last block of this template's plan
-        ht[g] = 0;
-        return;
-    }
-    const long S = fs.row_S ? fs.row_S[row] : fs.S;
-    const T *x = tr.x + (long) row * tr.ldx;
-    const long n = tr.len;
-    const long i0 = (long) b * S, i1 = i0 + S - 1;
-    const int h = (i0 < n && is_candidate<T>(x, (int) i0, (int) n, tr.thr)) ? 1 : 0;
-    const int tl = (i1 < n && is_candidate<T>(x, (int) i1, (int) n, tr.thr)) ? 1 : 0;
-    counts[g] = h + fs.cnt[(long) row * fs.nblk + b] + tl;
-    ht[g] = (unsigned char) (h | (tl << 1));
-}
+// unordered slot entries, indexed by row * nblk + b); peak_totals_kernel
+// decides the first and last lag of each block from the stored trace (bits 0
+// and 1 of ht) and forms the chunk's total count.
 
 // Packs chunk b of a trace in index order: first lag, body (slot entries
 // ranked by index, or a re-scan of the stored trace when more than kPkCap
@@ -454,8 +432,9 @@ static __global__ void __launch_bounds__(kPkThreads)
 // the candidate capacity, three scans and a compaction (25 launches, about
 // 130 us of mostly empty grids for the banks measured; now 15 us).  A trace
 // with more than kPkTraceCap candidates, or a chunk with more than its slot
-// holds, raises flags[0] and the host takes the launches above, which have no
-// such limit.
+// holds, makes the search dense: the totals raise flags[0], and the host takes
+// the launches above, which have no such limit.  More candidates in all than
+// the packed arrays hold leave the counts only; the host enlarges the arrays.
 constexpr int kPkTraceCap = 4096;
 constexpr int kPkTotThreads = 128;
 template <class T> constexpr size_t pk_prune_bytes() { return (sizeof(int) + sizeof(T) + 1) * (size_t) kPkTraceCap; }
@@ -493,8 +472,8 @@ static __device__ __forceinline__ bool last_cta(int *ticket, int *sh)
     return last;
 }
 
-// Candidates per trace (FUSED: with the block-edge lags decided here, as
-// peak_seam_kernel), and by the last CTA the traces' offsets.
+// Candidates per trace (FUSED: with the block-edge lags decided here), and by the last CTA the traces' offsets and flags[0] (1: a
+// dense search; flags[1] collects it and is left at 0).
 template <class T, bool FUSED>
 static __global__ void __launch_bounds__(kPkTotThreads)
     peak_totals_kernel(PeakTraces<T> tr, FusedSlots<T> fs, int nchunks, int *counts, unsigned char *ht, int *totals,
@@ -508,6 +487,7 @@ static __global__ void __launch_bounds__(kPkTotThreads)
     const int nb = FUSED && fs.row_nblk ? fs.row_nblk[row] : nchunks;
     const long S = FUSED && fs.row_S ? fs.row_S[row] : fs.S;
     long long mine = 0;
+    bool over = false;
     for (int b = threadIdx.x; b < nchunks; b += kPkTotThreads)
     {
         const long g = (long) trace * nchunks + b;
@@ -521,22 +501,32 @@ static __global__ void __launch_bounds__(kPkTotThreads)
             {
                 h = (i0 < n && is_candidate<T>(x, (int) i0, (int) n, tr.thr)) ? 1 : 0;
                 tl = (i1 < n && is_candidate<T>(x, (int) i1, (int) n, tr.thr)) ? 1 : 0;
-                cnt = h + fs.cnt[(long) row * fs.nblk + b] + tl;
+                cnt = fs.cnt[(long) row * fs.nblk + b];
+                over |= cnt > kPkCap;
+                cnt += h + tl;
             }
             counts[g] = cnt;
             ht[g] = (unsigned char) (h | (tl << 1));
         }
         else
+        {
             cnt = counts[g];
+            over |= cnt > kPkCap;
+        }
         mine += cnt;
     }
     long long tot;
     block_excl_scan(mine, sh, &tot);
-    if (threadIdx.x == 0) totals[trace] = (int) tot;
+    over = __syncthreads_or(over);
+    if (threadIdx.x == 0)
+    {
+        totals[trace] = (int) tot;
+        if (over || tot > kPkTraceCap) atomicOr(flags + 1, 1);
+    }
     if (last_cta(ticket, &lsh))
     {
         cta_prefix(totals, gridDim.x, trace_beg, sh);
-        if (threadIdx.x == 0) flags[0] = 0;
+        if (threadIdx.x == 0) flags[0] = atomicExch(flags + 1, 0);
     }
 }
 
@@ -546,7 +536,7 @@ template <class T, bool FUSED>
 static __global__ void __launch_bounds__(kPkThreads)
     peak_prune_kernel(PeakTraces<T> tr, FusedSlots<T> fs, int nchunks, const int *counts, const unsigned char *ht,
                       const int *slot_idx, const T *slot_val, int dist, const long long *trace_beg, long long cap,
-                      int *raw, int *nacc, long long *peak_off, int *ticket, int *flags)
+                      int *raw, int *nacc, long long *peak_off, int *ticket, const int *flags)
 {
     extern __shared__ __align__(16) unsigned char smem_pk[];
     __shared__ long long sh[32];
@@ -558,14 +548,12 @@ static __global__ void __launch_bounds__(kPkThreads)
     const long long tb = trace_beg[trace];
     const long long total = trace_beg[trace + 1] - tb;
     const T *x = tr.x + (long) row * tr.ldx;
-    bool ok = total <= kPkTraceCap && trace_beg[gridDim.x] <= cap;
     int accepted = 0;
-    if (ok && total > 0)
+    if (flags[0] == 0 && trace_beg[gridDim.x] <= cap && total > 0)
     {
         const int nc = (int) total;
         // ---- candidates in index order; a thread packs one chunk
         long long base = 0;
-        bool over = false;
         for (int b0 = 0; b0 < nchunks; b0 += kPkThreads)
         {
             const int b = b0 + tid;
@@ -581,11 +569,6 @@ static __global__ void __launch_bounds__(kPkThreads)
                 const long S = fs.row_S ? fs.row_S[row] : fs.S;
                 const long i0 = (long) b * S, bs = (long) row * fs.nblk + b;
                 const int bc = cnt - (hv & 1) - (hv >> 1);
-                if (bc > kPkCap)
-                {
-                    over = true;
-                    continue;
-                }
                 if (hv & 1)
                 {
                     idx[o] = (int) i0;
@@ -614,11 +597,6 @@ static __global__ void __launch_bounds__(kPkThreads)
             }
             else
             {
-                if (cnt > kPkCap)
-                {
-                    over = true;
-                    continue;
-                }
                 for (int q = 0; q < cnt; ++q)
                 {
                     idx[o + q] = slot_idx[g * kPkCap + q];
@@ -626,86 +604,78 @@ static __global__ void __launch_bounds__(kPkThreads)
                 }
             }
         }
-        ok = !__syncthreads_or(over);
-        if (ok)
+        __syncthreads();
+        for (int i = tid; i < nc; i += kPkThreads) state[i] = dist > 0 ? PK_UNDECIDED : PK_ACCEPTED;
+        __syncthreads();
+        // ---- rounds: each accepts at least the best undecided candidate
+        bool left = dist > 0;
+        while (left)
         {
-            for (int i = tid; i < nc; i += kPkThreads) state[i] = dist > 0 ? PK_UNDECIDED : PK_ACCEPTED;
-            __syncthreads();
-            // ---- rounds: each accepts at least the best undecided candidate
-            bool left = dist > 0;
-            while (left)
+            bool mine = false;
+            for (int g = tid; g < nc; g += kPkThreads)
             {
-                bool mine = false;
-                for (int g = tid; g < nc; g += kPkThreads)
-                {
-                    if (state[g] != PK_UNDECIDED) continue;
-                    const int ig = idx[g];
-                    const T vg = val[g];
-                    bool best = true;
-                    for (int k = g - 1; k >= 0 && ig - idx[k] <= dist; --k)
+                if (state[g] != PK_UNDECIDED) continue;
+                const int ig = idx[g];
+                const T vg = val[g];
+                bool best = true;
+                for (int k = g - 1; k >= 0 && ig - idx[k] <= dist; --k)
+                    if (state[k] <= PK_NEW && state[k] != PK_ACCEPTED && higher<T>(val[k], idx[k], vg, ig))
+                    {
+                        best = false;
+                        break;
+                    }
+                if (best)
+                    for (int k = g + 1; k < nc && idx[k] - ig <= dist; ++k)
                         if (state[k] <= PK_NEW && state[k] != PK_ACCEPTED && higher<T>(val[k], idx[k], vg, ig))
                         {
                             best = false;
                             break;
                         }
-                    if (best)
-                        for (int k = g + 1; k < nc && idx[k] - ig <= dist; ++k)
-                            if (state[k] <= PK_NEW && state[k] != PK_ACCEPTED && higher<T>(val[k], idx[k], vg, ig))
-                            {
-                                best = false;
-                                break;
-                            }
-                    if (best) state[g] = PK_NEW;
-                    else mine = true;
-                }
-                left = __syncthreads_or(mine);
-                for (int g = tid; g < nc; g += kPkThreads)
-                {
-                    if (state[g] != PK_NEW) continue;
-                    const int ig = idx[g];
-                    for (int k = g - 1; k >= 0 && ig - idx[k] <= dist; --k)
-                        if (state[k] == PK_UNDECIDED) state[k] = PK_REJECTED;
-                    for (int k = g + 1; k < nc && idx[k] - ig <= dist; ++k)
-                        if (state[k] == PK_UNDECIDED) state[k] = PK_REJECTED;
-                    state[g] = PK_ACCEPTED;
-                }
-                __syncthreads();
+                if (best) state[g] = PK_NEW;
+                else mine = true;
             }
-            // ---- accepted lags, ascending
-            for (int g0 = 0; g0 < nc; g0 += kPkThreads)
+            left = __syncthreads_or(mine);
+            for (int g = tid; g < nc; g += kPkThreads)
             {
-                const int g = g0 + tid;
-                const bool a = g < nc && state[g] == PK_ACCEPTED;
-                long long tot;
-                const long long o = block_excl_scan((long long) (a ? 1 : 0), sh, &tot);
-                if (a) raw[tb + accepted + o] = idx[g];
-                accepted += (int) tot;
+                if (state[g] != PK_NEW) continue;
+                const int ig = idx[g];
+                for (int k = g - 1; k >= 0 && ig - idx[k] <= dist; --k)
+                    if (state[k] == PK_UNDECIDED) state[k] = PK_REJECTED;
+                for (int k = g + 1; k < nc && idx[k] - ig <= dist; ++k)
+                    if (state[k] == PK_UNDECIDED) state[k] = PK_REJECTED;
+                state[g] = PK_ACCEPTED;
             }
+            __syncthreads();
+        }
+        // ---- accepted lags, ascending
+        for (int g0 = 0; g0 < nc; g0 += kPkThreads)
+        {
+            const int g = g0 + tid;
+            const bool a = g < nc && state[g] == PK_ACCEPTED;
+            long long tot;
+            const long long o = block_excl_scan((long long) (a ? 1 : 0), sh, &tot);
+            if (a) raw[tb + accepted + o] = idx[g];
+            accepted += (int) tot;
         }
     }
-    if (tid == 0)
-    {
-        nacc[trace] = accepted;
-        if (!ok) flags[0] = 1;
-    }
+    if (tid == 0) nacc[trace] = accepted;
     if (last_cta(ticket, &lsh)) cta_prefix(nacc, gridDim.x, peak_off, sh);
 }
 
-// The traces' accepted lags side by side; res[ntr + 1 ..]: candidates, bail
-// flag, the object's device status word.
+// The traces' accepted lags side by side (none in a dense search, or one with
+// more candidates than cap); res[ntr + 1 ..]: candidates, whether the search is
+// dense, the object's device status word.
 static __global__ void __launch_bounds__(64) peak_emit_kernel(int ntr, const int *raw, const long long *trace_beg,
                                                               const int *flags, const int *err, long long *res,
                                                               int *peaks)
 {
     const int t = blockIdx.x;
-    const bool bail = flags[0] != 0;
     if (t == 0 && threadIdx.x == 0)
     {
         res[ntr + 1] = trace_beg[ntr];
-        res[ntr + 2] = bail ? 1 : 0;
+        res[ntr + 2] = flags[0];
         res[ntr + 3] = err ? *err : 0;
     }
-    if (bail) return;
     const long long o = res[t], b = trace_beg[t];
     const int n = (int) (res[t + 1] - o);
     for (int i = threadIdx.x; i < n; i += 64) peaks[o + i] = raw[b + i];

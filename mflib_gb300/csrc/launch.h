@@ -173,7 +173,7 @@ struct PeakWS
 {
     DevBuf counts, offs, slot_idx, slot_val, cidx, cval, ctr, state, flags, pos, tiles, trace_beg, peak_off, peaks,
         counter, row, ht, totals, nacc, ticket;
-    bool dense = false;        // dense_search had a trace with more candidates than one CTA prunes
+    bool dense = false;        // dense_search's last traces held more candidates than one CTA prunes
     PeakSearch dense_search;
     long long npeaks = 0;
     long long cand_cap = 1 << 16;  // capacity of the packed candidate arrays
@@ -201,7 +201,7 @@ struct PeakWS
 // per 64 lags of each row, fwords words per row; see PeakTraces), when given,
 // lets the scan skip the lags no value above the threshold lies in.
 // host_err (optional) receives the device status word dev_err as of the end
-// of the search (0 when not read).
+// of the search.
 template <class T>
 int run_peaks(const T *x, long ldx, const int *host_rows, int ntr, int len, double thr, int dist, PeakWS &ws,
               cudaStream_t s, long long *launches, long long *host_peak_off, std::string &err,

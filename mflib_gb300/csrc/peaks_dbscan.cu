@@ -79,66 +79,78 @@ int run_peaks(const T *x, long ldx, const int *host_rows, int ntr, int len, doub
     const dim3 grid(nchunks, ntr);
     const bool prune = dist > 0;
 
-    // One CTA per trace, unless this search's candidates did not fit it the
-    // last time (the same traces are then as dense again)
+    // Candidates per chunk and trace, and whether any holds more than one CTA
+    // prunes (a dense search)
+    MF_TRY(ws.totals.ensure(sizeof(int) * ntr));
+    if (!ws.ticket.p)
+    {
+        MF_TRY(ws.ticket.ensure(4 * sizeof(int)));  // [0], [1] tickets, [2] the dense flag, [3] where it is collected
+        MF_TRY(cudaMemsetAsync(ws.ticket.p, 0, 4 * sizeof(int), s));
+    }
+    int *tick = ws.ticket.as<int>();
+    FusedSlots<T> none{};
+    if (fused)
+        peak_totals_kernel<T, true><<<ntr, kPkTotThreads, 0, s>>>(tr, *fused, nchunks, ws.counts.as<int>(),
+                                                                 ws.ht.as<unsigned char>(), ws.totals.as<int>(),
+                                                                 ws.trace_beg.as<long long>(), tick, tick + 2);
+    else
+    {
+        peak_cand_kernel<T><<<grid, kPkThreads, 0, s>>>(tr, nchunks, ws.counts.as<int>(), ws.slot_idx.as<int>(),
+                                                        ws.slot_val.as<T>());
+        peak_totals_kernel<T, false><<<ntr, kPkTotThreads, 0, s>>>(tr, none, nchunks, ws.counts.as<int>(), nullptr,
+                                                                  ws.totals.as<int>(), ws.trace_beg.as<long long>(),
+                                                                  tick, tick + 2);
+        ++*launches;
+    }
+    ++*launches;
+    MF_TRY(cudaGetLastError());
+
+    // One CTA per trace, not tried when the same search was dense the last
+    // time: an object's next traces are most often like its last ones, and an
+    // attempt that fails costs two launches and a wait.  The form below renews
+    // the flag from the counts of its own traces.
     const PeakSearch search{thr, ntr, len, dist, fused != nullptr};
-    if (!(ws.dense && ws.dense_search == search))
+    while (!(ws.dense && ws.dense_search == search))
     {
         const long long cap = ws.cand_cap;
-        MF_TRY(ws.totals.ensure(sizeof(int) * ntr));
         MF_TRY(ws.nacc.ensure(sizeof(int) * ntr));
         MF_TRY(ws.cidx.ensure(sizeof(int) * cap));
         MF_TRY(ws.peaks.ensure(sizeof(int) * cap));
-        if (!ws.ticket.p)
-        {
-            MF_TRY(ws.ticket.ensure(4 * sizeof(int)));  // [0], [1] tickets, [2] the bail flag
-            MF_TRY(cudaMemsetAsync(ws.ticket.p, 0, 4 * sizeof(int), s));
-        }
-        int *tick = ws.ticket.as<int>();
         long long *res = ws.peak_off.as<long long>();
         const size_t bytes = pk_prune_bytes<T>();
         static SmemCap capf, caps;
-        FusedSlots<T> none{};
         if (fused)
         {
-            peak_totals_kernel<T, true><<<ntr, kPkTotThreads, 0, s>>>(tr, *fused, nchunks, ws.counts.as<int>(),
-                                                                     ws.ht.as<unsigned char>(), ws.totals.as<int>(),
-                                                                     ws.trace_beg.as<long long>(), tick, tick + 2);
             MF_TRY(raise_smem_cap(peak_prune_kernel<T, true>, bytes, capf));
             peak_prune_kernel<T, true><<<ntr, kPkThreads, bytes, s>>>(
                 tr, *fused, nchunks, ws.counts.as<int>(), ws.ht.as<unsigned char>(), nullptr, nullptr, dist,
                 ws.trace_beg.as<long long>(), cap, ws.cidx.as<int>(), ws.nacc.as<int>(), res, tick + 1, tick + 2);
-            *launches += 3;
         }
         else
         {
-            peak_cand_kernel<T><<<grid, kPkThreads, 0, s>>>(tr, nchunks, ws.counts.as<int>(), ws.slot_idx.as<int>(),
-                                                            ws.slot_val.as<T>());
-            peak_totals_kernel<T, false><<<ntr, kPkTotThreads, 0, s>>>(tr, none, nchunks, ws.counts.as<int>(), nullptr,
-                                                                      ws.totals.as<int>(),
-                                                                      ws.trace_beg.as<long long>(), tick, tick + 2);
             MF_TRY(raise_smem_cap(peak_prune_kernel<T, false>, bytes, caps));
             peak_prune_kernel<T, false><<<ntr, kPkThreads, bytes, s>>>(
                 tr, none, nchunks, ws.counts.as<int>(), nullptr, ws.slot_idx.as<int>(), ws.slot_val.as<T>(), dist,
                 ws.trace_beg.as<long long>(), cap, ws.cidx.as<int>(), ws.nacc.as<int>(), res, tick + 1, tick + 2);
-            *launches += 4;
         }
         peak_emit_kernel<<<ntr, 64, 0, s>>>(ntr, ws.cidx.as<int>(), ws.trace_beg.as<long long>(), tick + 2, dev_err, res,
                                             ws.peaks.as<int>());
+        *launches += 2;
         MF_TRY(cudaGetLastError());
         std::vector<long long> got(ntr + 4);
         MF_TRY(cudaMemcpyAsync(got.data(), res, sizeof(long long) * (ntr + 4), cudaMemcpyDeviceToHost, s));
         MF_TRY(cudaStreamSynchronize(s));
         if (host_err) *host_err = (int) got[ntr + 3];
-        if (got[ntr + 2] == 0)
+        const long long ncand = got[ntr + 1];
+        ws.dense = got[ntr + 2] != 0;
+        ws.dense_search = search;
+        if (!ws.dense && ncand <= cap)
         {
             std::copy(got.begin(), got.begin() + ntr + 1, host_peak_off);
             ws.npeaks = host_peak_off[ntr];
-            ws.dense = false;
             return 0;
         }
-        ws.dense = true;
-        ws.dense_search = search;
+        if (!ws.dense) ws.cand_cap = std::max<long long>(2 * cap, ncand + ncand / 4 + 1024);
     }
 
     // Any number of candidates: rounds over all traces' packed candidates
@@ -159,14 +171,6 @@ int run_peaks(const T *x, long ldx, const int *host_rows, int ntr, int len, doub
         MF_TRY(ws.tiles.ensure(sizeof(long long) * (scan_tiles_needed(std::max<long>((long) nslots, (long) cap) + 1) + 8)));
         MF_TRY(cudaMemsetAsync(ws.counter.p, 0, 4 * sizeof(int), s));
 
-        if (fused)
-            peak_seam_kernel<T><<<(unsigned) ((nslots + 255) / 256), 256, 0, s>>>(tr, ntr, *fused, ws.counts.as<int>(),
-                                                                                ws.ht.as<unsigned char>());
-        else
-            peak_cand_kernel<T><<<grid, kPkThreads, 0, s>>>(tr, nchunks, ws.counts.as<int>(), ws.slot_idx.as<int>(),
-                                                            ws.slot_val.as<T>());
-        ++*launches;
-        MF_TRY(cudaGetLastError());
         MF_TRY(device_excl_scan(ws.counts.as<int>(), (long) nslots, ws.offs.as<long long>(),
                                 ws.tiles.as<long long>(), s, launches));
         peak_trace_beg_kernel<<<(ntr + 1 + 127) / 128, 128, 0, s>>>(ntr, nchunks, ws.offs.as<long long>(), cap,
@@ -192,7 +196,7 @@ int run_peaks(const T *x, long ldx, const int *host_rows, int ntr, int len, doub
         long long rounds_done = 0;
         int left = 0;
         long long ncand = 0;
-        int ovf = 0;
+        int ovf = 0, dense = 0;
         for (;;)
         {
             if (prune)
@@ -230,6 +234,9 @@ int run_peaks(const T *x, long ldx, const int *host_rows, int ntr, int len, doub
             MF_TRY(cudaMemcpyAsync(&ncand, ncand_dev, sizeof(long long), cudaMemcpyDeviceToHost, s));
             MF_TRY(cudaMemcpyAsync(&left, undecided, sizeof(int), cudaMemcpyDeviceToHost, s));
             MF_TRY(cudaMemcpyAsync(&ovf, overflow, sizeof(int), cudaMemcpyDeviceToHost, s));
+            MF_TRY(cudaMemcpyAsync(&dense, tick + 2, sizeof(int), cudaMemcpyDeviceToHost, s));
+            if (dev_err && host_err)
+                MF_TRY(cudaMemcpyAsync(host_err, dev_err, sizeof(int), cudaMemcpyDeviceToHost, s));
             MF_TRY(cudaStreamSynchronize(s));
             if (ovf || ncand > cap) break;
             if (!prune || left == 0) break;
@@ -245,6 +252,7 @@ int run_peaks(const T *x, long ldx, const int *host_rows, int ntr, int len, doub
             continue;
         }
         ws.npeaks = host_peak_off[ntr];
+        ws.dense = dense != 0;
         return 0;
     }
     err = "peak candidate capacity could not be sized";
