@@ -44,6 +44,9 @@ int run_peaks(const T *x, long ldx, const int *host_rows, int ntr, int len, doub
     if (len <= 0)
     {
         for (int t = 0; t <= ntr; ++t) host_peak_off[t] = 0;
+        if (dev_err && host_err)
+            MF_TRY(cudaMemcpyAsync(host_err, dev_err, sizeof(int), cudaMemcpyDeviceToHost, s));
+        MF_TRY(cudaStreamSynchronize(s));
         return 0;
     }
     // chunks: kPkChunk lags for the stand-alone scan, one correlator block
