@@ -604,10 +604,13 @@ __global__ void __launch_bounds__(32 * kFixListWarps) fix_list_kernel(FixParams<
             __syncwarp();
             if (q + kFixListWarps < np) fetch(q + kFixListWarps, nx);
             float v[32], s = 0.f;
+            // past the longest window (its coefficients are zero) samples count
+            // as zero, also an infinity; such a piece is in no window's statistics
+            const int nin = Lb - 32 * q;
 #pragma unroll
             for (int i = 0; i < 32; ++i)
             {
-                v[i] = ys[lane + 32 * q + i] - Rl;
+                v[i] = i < nin ? ys[lane + 32 * q + i] - Rl : 0.f;
                 s += v[i];
             }
             const float mu = s * (1.f / 32.f);
