@@ -297,10 +297,9 @@ struct mfgpu_mf
     bool test_wait_timeout = false;  // mfgpu_mf_test_wait_timeout: the next apply only
     int dev_smem = 0;                // opt-in shared memory per block of the device
     // FP64 data correlated in integer arithmetic (kernels_int.cuh): template
-    // table, twiddles, lags and number of the normalisation tiles
+    // table, twiddles, units of the blocks
     bool intx = false;
-    DevBuf int_B, int_tw;
-    int int_lags = 0, int_tiles = 0;
+    DevBuf int_B, int_tw, int_unit;
     bool persistent = false;         // FFT correlator as a persistent work-queue launch (option)
     bool tc_bf16 = false;            // tensor-core operands split into BF16 instead of FP16 (option)
     float tc_maxb = 0.f;             // largest coefficient of the unit-norm templates (tensor-core path)
@@ -315,7 +314,7 @@ struct mfgpu_mf
                          &xrange,   &tc_B,   &tc_bscale, &tc_grp_chan, &tc_grp_tid, &pk_flags,
                          &rstat,    &cst,    &fxbits, &fxlist, &fxcount, &tc_off, &fx_btid, &fx_boff,
                          &fx_bL,    &fx_cb0, &fx_cnb, &fx_bch, &dlags,
-                         &fx_bco,   &fx_bsum, &pk_dirty, &tws, &tickets, &int_B, &int_tw};
+                         &fx_bco,   &fx_bsum, &pk_dirty, &tws, &tickets, &int_B, &int_tw, &int_unit};
         for (DevBuf *d : all) f(*d);
         pk.each_buf(f);
         f(row_S);
@@ -1105,9 +1104,8 @@ try
         const std::vector<unsigned> &tw = int_twiddles();
         CU(mf->int_tw.ensure(sizeof(int) * tw.size()));
         CU(cudaMemcpyAsync(mf->int_tw.p, tw.data(), sizeof(int) * tw.size(), cudaMemcpyHostToDevice, mf->stream));
+        CU(mf->int_unit.ensure(sizeof(IntUnit) * (size_t) nch * std::max(0, mf->nblocks)));
         CU(mf->int_B.ensure(sizeof(int) * (size_t) nt * kIntPrimes * kIntN));
-        mf->int_lags = ((int_tile(maxLen) - maxLen) / 32) * 32;
-        mf->int_tiles = (std::max(1, maxvalid_f) + mf->int_lags - 1) / mf->int_lags;
         CU(launch_int_bank(mf->tmpl_d.as<double>(), mf->toff_d.as<long>(), mf->tlen_d.as<int>(), nt,
                            mf->int_tw.as<unsigned>(), mf->int_B.as<unsigned>(), mf->stream));
         ++mf->launches;
@@ -1926,12 +1924,12 @@ template <class T> static mfgpu_status mf_launch_xcorr(mfgpu_mf *mf)
         if (mf->intx)
         {
             IntDenParams d{};
-            d.x = p.x; d.ldx = p.ldx; d.n = mf->n; d.dead = p.dead; d.tol = p.tol; d.lags = mf->int_lags;
+            d.x = p.x; d.ldx = p.ldx; d.n = mf->n; d.dead = p.dead; d.tol = p.tol; d.S = mf->S; d.Lmax = int_norm_length(mf->fLen); d.unit = mf->int_unit.as<IntUnit>();
             d.scale = int_numerator_scale() * (mf->shared_den ? std::sqrt((double) mf->fLen) : 1.0);
             d.L = mf->fLen; d.nv = mf->n - mf->fLen + 1; d.den = mf->den.as<double>(); d.ldd = p.ldd;
             d.grp_chan = p.grp_chan; d.grp_tb = p.grp_tb; d.grp_te = p.grp_te; d.tids = p.tids;
             d.tlen = p.tlen; d.nvalid = p.nvalid; d.rho = p.rho; d.ldr = p.ldr;
-            CU(launch_int_den(d, !mf->shared_den, int_tile(mf->fLen), mf->int_tiles, mf->shared_den ? mf->nch : mf->ngroups, mf->stream));
+            CU(launch_int_den(d, !mf->shared_den, mf->nblocks, mf->shared_den ? mf->nch : mf->ngroups, mf->stream));
             ++mf->launches;
         }
     if (mf->shared_den && !mf->intx && !(sizeof(T) == 4 && mf->fx_on))
@@ -2013,8 +2011,8 @@ template <class T> static mfgpu_status mf_launch_xcorr(mfgpu_mf *mf)
     if constexpr (sizeof(T) == 8)
     {
         if (mf->intx)
-            CU(launch_int_xcorr(p, mf->shared_den, mf->int_B.as<unsigned>(), mf->int_tw.as<unsigned>(), mf->fLen, mf->n, mf->nblocks,
-                                mf->ngroups, mf->stream));
+            CU(launch_int_xcorr(p, mf->shared_den, mf->int_B.as<unsigned>(), mf->int_tw.as<unsigned>(),
+                                mf->int_unit.as<IntUnit>(), mf->n, mf->nblocks, mf->ngroups, mf->stream));
     }
     if (!mf->intx)
         CU(launch_xcorr<T>(mf->log2p, mf->shared_den, mf->mode_x, p, mf->nblocks, mf->ngroups, mf->stream));

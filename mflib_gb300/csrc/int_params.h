@@ -8,12 +8,13 @@ constexpr int kIntN = 4096;       // transform length: the samples of a block
 constexpr int kIntPrimes = 4;
 constexpr int kIntThreads = 1024;
 constexpr int kIntTw = 240 + 3840;  // twiddles per prime: rows r = 1 .. 15 of the second and third pass
-// samples of a normalisation tile for templates of up to L samples
-constexpr int int_tile(int L) { return L <= 1024 ? 4096 : 8192; }
-constexpr int kIntXBits = 50;     // bits of a quantised sample of a normalisation tile
+constexpr int kIntDenThreads = 512;
 constexpr int kIntBBits = 53;     // fraction bits of a template coefficient
 constexpr float kIntNormBits = 55.1f;  // a block's windows: 2-norm below 2^55.1, so that a numerator stays below
                                        // 2^108.1 and half the primes' product (2^108.19)
+// the window length that bounds a block's unit: of the longest template, at
+// least 2 (the sums of squares of 256 samples, IntSums)
+constexpr int int_norm_length(int Lmax) { return Lmax < 2 ? 2 : Lmax; }
 
 // One prime: c25 and rrn are times R = 2^32 modulo p; all in [0, p).
 struct IntPrime
@@ -42,6 +43,14 @@ struct IntBankParams
     IntConsts c;
 };
 
+// A block's integers: v = (f - level) 2^-sh, f the sample in units of 2^(emax -
+// 1084); emax -1: the block holds an infinity or NaN
+struct IntUnit
+{
+    long long level;
+    int emax, sh;
+};
+
 struct IntDenParams
 {
     const double *x;
@@ -51,7 +60,9 @@ struct IntDenParams
     double tol;
     double scale;                   // factor of the correlator's numerators (int_numerator_scale);
                                     // one length: times sqrt(L)
-    int lags;                       // lags per tile
+    int S;                          // lags per block, as the correlator's
+    int Lmax;                       // int_norm_length of the longest template
+    IntUnit *unit;                  // [channel][block]
     // one length: L, valid lags, rows den
     int L;
     long nv;

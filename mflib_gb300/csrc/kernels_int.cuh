@@ -17,8 +17,8 @@
 //     primes p = 1 mod 8192 just below 2^32 / 26, and the Chinese remainder
 //     theorem.  |numerator| <= 2^55.1 2^53 stays below half the primes' product
 //     (2^108.19) by Cauchy-Schwarz.
-//   * Window variances come from prefix sums of X (50 bits, sums 64) and X^2
-//     (sums 128 bits) of a tile: V = L S2 - S1^2 is exact.  1 / sqrt(V) starts from the
+//   * Window variances come from prefix sums of the same X (64 bits) and X^2 (128
+//     bits) of the block: V = L S2 - S1^2 is exact.  1 / sqrt(V) starts from the
 //     FP32 reciprocal square root and takes one third-order step in 60-bit
 //     fixed point.
 //   * The Chinese remainder theorem as a sum of fractions, numerator / M = sum
@@ -26,11 +26,15 @@
 //     the numerator to 2^-64 of M.
 //
 // The remaining errors are the two roundings of the inputs and three roundings
-// to FP64 at the end: below those of an FP64 transform, whose rounding grows
-// with the block's energy and log N (relative errors of the coefficients of
-// band-passed templates of 200 .. 2,000 samples against two-pass sums in
-// quadruple precision: 3.7e-16 .. 5.7e-16, FP64 transforms 7.8e-16 ..
-// 1.75e-15).
+// to FP64 at the end.  A sample's is at most half a unit of its block, so a
+// coefficient whose window has the 2-norm W about its mean, in a block whose
+// loudest window has the norm A, errs by less than 2^-53 sqrt(L) A / W, about
+// 2^-56 A / W as a rule, besides some 1e-16; no sample outside the block counts.  An FP64 transform's rounding is 2^-53 of the block's norm spread over its
+// lags, and running FP64 sums of squares lose (A / W)^2 2^-53 after the loud
+// part.  Against exact sums, windows of 200 .. 2,000 samples of noise: 0.8e-16 ..
+// 1.1e-16 here, 0.6e-16 .. 3.9e-16 by the transform and its in-block sums;
+// quiet windows of a block with a part 1e3 (1e6) times louder: 0.5e-15 .. 6e-14
+// (0.5e-12 .. 8e-11) here, 0.4e-15 .. 2e-10 (1e-12 .. 3e-4) by the others.
 //
 // Arithmetic modulo p: Montgomery products with R = 2^32 on unsigned words
 // (wide multiply, low multiply, wide multiply-add; the signed forms cost two
@@ -49,7 +53,7 @@ struct IntParams
     XcorrParams<double> x;  // as the FFT correlator's (spectra and twiddles unused)
     const unsigned *B;      // [template][prime][kIntN]
     const unsigned *tw;     // [prime][kIntTw]
-    int Lmax;               // longest template
+    const IntUnit *unit;    // [channel][block], by the normalisation
     long n;                 // samples per row
     IntConsts c;
 };
@@ -226,21 +230,23 @@ template <int NTH> __device__ __forceinline__ long long int_block_sum(long long 
 }
 
 // log2 of a bound on sum v^2 over any L consecutive samples, |v| <= 2^nb, sample
-// tid + 1024 i in v[i]: the largest sum of the runs of 32 samples that a window
-// can touch, each sample's square taken above its value (12 bits).  red: 128 words.
-template <int NTH, int PER>
-__device__ __forceinline__ float int_window_norm(const long long (&v)[PER], int nb, int L, unsigned *red)
+// 8 tid + i in v[i]: the largest sum of the runs of 32 samples that a window can
+// touch, each sample's square taken above its value (12 bits).  red: 128 words.
+__device__ __forceinline__ float int_window_norm(const long long (&v)[8], int nb, int L, unsigned *red)
 {
-    static_assert(NTH * PER == 4096 && NTH == 1024, "128 runs, four per lane");
+    static_assert(8 * kIntDenThreads == 4096, "128 runs, four per lane");
     const int lane = threadIdx.x & 31, d = max(0, nb - 12);
-    __syncthreads();
+    unsigned own = 0;
 #pragma unroll
-    for (int i = 0; i < PER; ++i)
+    for (int i = 0; i < 8; ++i)
     {
         const unsigned y = (unsigned) ((v[i] < 0 ? -v[i] : v[i]) >> d) + 1u;
-        const unsigned q = __reduce_add_sync(0xffffffffu, y * y);  // below 2^30
-        if (lane == 0) red[32 * i + (threadIdx.x >> 5)] = (q >> 5) + 1u;
+        own += y * y;
     }
+    own += __shfl_xor_sync(0xffffffffu, own, 1);
+    own += __shfl_xor_sync(0xffffffffu, own, 2);  // a run of 32: below 2^30
+    __syncthreads();
+    if ((lane & 3) == 0) red[threadIdx.x >> 2] = (own >> 5) + 1u;
     __syncthreads();
     uint4 r = reinterpret_cast<const uint4 *>(red)[lane];
     r.y += r.x;
@@ -269,21 +275,28 @@ __device__ __forceinline__ float int_window_norm(const long long (&v)[PER], int 
     return fminf(log2f((float) best) + 5.f, log2f((float) L) + (float) (2 * (nb - d))) + (float) (2 * d);
 }
 
-// Quantises the PER samples (bit patterns) each of NTH threads holds, N = NTH
-// PER in all: v[] receives the integers, the return value is the exponent of
-// their unit (x - level = v 2^ex up to half a unit).  An infinity or NaN
-// counts as 0 and sets *bad.  NORM false: at most kIntXBits bits.  NORM true:
-// the finest unit at which the 2-norm of every window of at most L samples
-// stays below 2^kIntNormBits, at most 55 bits; lred: 64 words.
-template <int NTH, int PER, bool NORM>
-__device__ __forceinline__ int int_quantise(long long (&v)[PER], int *ired, long long *lred, int L, bool *bad)
+// A block's integers, from the samples as bit patterns: what the normalisation
+// finds (int_quantise) and the correlator applies again.
+__device__ __forceinline__ long long int_sample(const IntUnit &u, long long fixed)
 {
-    constexpr int LOG2N = NTH * PER == 4096 ? 12 : 13;
-    static_assert(NTH * PER == 1 << LOG2N, "the level is a sum shifted by log2 N");
+    const long long half = u.sh > 0 ? 1ll << (u.sh - 1) : 0;
+    return (fixed - u.level + half) >> u.sh;
+}
+// exponent of their unit: x - level = v 2^ex up to half a unit
+__device__ __forceinline__ int int_unit_exponent(const IntUnit &u) { return u.emax - 1084 + u.sh; }
+
+// Quantises a block's samples, sample 8 tid + i in v[i]: the finest unit at which
+// the 2-norm of every window of at most L samples stays below 2^kIntNormBits, at
+// most 55 bits.  An infinity or NaN counts as 0 and sets emax to -1 (the others
+// keep their integers).  lred: 64 words.
+__device__ __forceinline__ IntUnit int_quantise(long long (&v)[8], int *ired, long long *lred, int L, int *ex)
+{
+    constexpr int LOG2N = 12, NTH = kIntDenThreads;
+    static_assert(kIntN == 1 << LOG2N, "the level is a sum shifted by log2 N");
     int em = 1;
     bool nf = false;
 #pragma unroll
-    for (int i = 0; i < PER; ++i)
+    for (int i = 0; i < 8; ++i)
     {
         const int e = int_expo(v[i]);
         if (e == 2047)
@@ -297,36 +310,33 @@ __device__ __forceinline__ int int_quantise(long long (&v)[PER], int *ired, long
     const int emx = int_block_max<NTH>(em | (nf ? 1 << 12 : 0), ired);
     // (with a non-finite sample the largest exponent of the others is found
     // again: rare)
-    *bad = (emx >> 12) != 0;
-    const int emax = *bad ? int_block_max<NTH>(em, ired) : emx;
+    const bool bad = (emx >> 12) != 0;
+    IntUnit u;
+    u.emax = bad ? int_block_max<NTH>(em, ired) : emx;
     long long s = 0;
 #pragma unroll
-    for (int i = 0; i < PER; ++i)
+    for (int i = 0; i < 8; ++i)
     {
-        v[i] = int_fixed(v[i], emax);
+        v[i] = int_fixed(v[i], u.emax);
         s += v[i] >> LOG2N;
     }
-    const long long lev = int_block_sum<NTH>(s, lred);  // about the mean
+    u.level = int_block_sum<NTH>(s, lred);  // about the mean
     unsigned long long any = 0;
+    long long d[8];
 #pragma unroll
-    for (int i = 0; i < PER; ++i)
+    for (int i = 0; i < 8; ++i)
     {
-        v[i] -= lev;
-        any |= (unsigned long long) (v[i] ^ (v[i] >> 63));
+        d[i] = v[i] - u.level;
+        any |= (unsigned long long) (d[i] ^ (d[i] >> 63));
     }
-    const int nb = int_block_max<NTH>(64 - __clzll((long long) any), ired);  // |v| <= 2^nb
-    int sh;
-    if constexpr (NORM)
-    {
-        const float n2 = int_window_norm<NTH, PER>(v, nb, L, reinterpret_cast<unsigned *>(lred));
-        sh = max(max(0, nb - 55), (int) ceilf(0.5f * n2 - kIntNormBits));
-    }
-    else
-        sh = max(0, nb - kIntXBits);
-    const long long half = sh > 0 ? 1ll << (sh - 1) : 0;
+    const int nb = int_block_max<NTH>(64 - __clzll((long long) any), ired);  // |d| <= 2^nb
+    const float n2 = int_window_norm(d, nb, L, reinterpret_cast<unsigned *>(lred));
+    u.sh = max(max(0, nb - 55), (int) ceilf(0.5f * n2 - kIntNormBits));
 #pragma unroll
-    for (int i = 0; i < PER; ++i) v[i] = (v[i] + half) >> sh;
-    return emax - 1084 + sh;
+    for (int i = 0; i < 8; ++i) v[i] = int_sample(u, v[i]);
+    *ex = int_unit_exponent(u);
+    if (bad) u.emax = -1;
+    return u;
 }
 
 // ---- template table -----------------------------------------------------------
@@ -418,36 +428,40 @@ __device__ __forceinline__ double int_inv_den(unsigned __int128 V, int ex, doubl
     return scale * __longlong_as_double(yb);
 }
 
-// One CTA per (tile of T samples, group).  MULTI false (one template length):
-// the channel's row den[c][k].  MULTI true: for every template of the group,
-// its own rows, written where the coefficients go (the correlator reads each
-// value before it stores the coefficient in its place).
+// One CTA per (block, group), on the correlator's blocks and integers.  MULTI
+// false (one template length): the channel's row den[c][k].  MULTI true: for
+// every template of the group, its own rows, written where the coefficients go
+// (the correlator reads each value before it stores the coefficient in its
+// place).
 //
-// The tile's prefix sums (24 bytes per sample) give any window of any length
-// in two loads each of S1 and S2: about 90 integer instructions and one FP64
+// The block's prefix sums (24 bytes per sample, 98 KB: two CTAs of 512 threads
+// per SM, whose loads, scans and lags overlap) give any window of any length in
+// two loads each of S1 and S2: about 90 integer instructions and one FP64
 // product per lag, against some 27 FP64 operations (16 clocks per SM) of the
-// running FP64 form.  T = 4096 (98 KB, two CTAs of 512 threads per SM, whose
-// loads, scans and lags overlap) for templates of up to 1,024 samples, where
-// the windows' overlap costs at most a third; T = 8192 above (64 x 360,000, L
-// = 500: 308 us, in tiles of 8192 346; 8 x 360,000, 160 templates of 200 ..
-// 2,000: 424 us, in tiles of 4096 444).
-// Bound by the integer pipes (ALU 61 %, issue 59 %).  Before the sums in three
-// words, the integer normalisation of V and the square roots of L taken out of
-// the threads: 396 and 562 us in tiles of 8192.
+// running FP64 form.  64 x 360,000, L = 500: 335 us; 8 x 360,000, 160 templates of
+// 200 .. 2,000: 450 us; bound by the integer pipes.  The block's unit is found
+// here and read by the correlator, whose own reductions for it took 80 and 60 us
+// of the same cases.  Tiles and integers of its own (50 bits; tiles of 8,192
+// samples above L = 1,024) took 308 and 424 us, but a loud sample outside a
+// block then took digits from that block's coefficients (a sample 1e6 times the
+// signal, L = 200: 3e-11, now below 1e-15).  Where a block leaves few lags they
+// were cheaper, too: one template of 4,065 on each of 8 channels x 120,000, 32
+// lags per block: 3.10 -> 3.57 ms (of 3,500: 242 -> 249 us; of 2,500: 131 -> 119).
 __device__ __forceinline__ int int_pswz(int i) { return i ^ ((i >> 3) & 15); }
-__host__ __device__ constexpr size_t int_den_bytes(int T) { return 3 * sizeof(long long) * (size_t) (T + 16); }
+__host__ __device__ constexpr size_t int_den_bytes() { return 3 * sizeof(long long) * (size_t) (kIntN + 16); }
 
-// sums of x and of x^2 as al^2 + 2^26 ah al + 2^50 ah^2, |x| = 2^25 ah + al <=
-// 2^50: three multiplies and no carries (the sums of 8,192 stay below 2^63)
+// sums of x and of x^2 as al^2 + 2^28 ah al + 2^54 ah^2, |x| = 2^27 ah + al <=
+// 2^55, over at most 256 samples: three multiplies and no carries (al^2 sums to
+// 2^62, ah al to 2^63; ah^2 to 2^63.2, as windows of two samples or more stay
+// below 2^55.1); x itself modulo 2^64
 struct IntSums
 {
-    long long s;
-    unsigned long long a, b, c;
+    unsigned long long s, a, b, c;
     __device__ __forceinline__ void add(long long v)
     {
-        s += v;
+        s += (unsigned long long) v;
         const unsigned long long m = v < 0 ? -v : v;
-        const unsigned l = (unsigned) m & ((1u << 25) - 1), h = (unsigned) (m >> 25);
+        const unsigned l = (unsigned) m & ((1u << 27) - 1), h = (unsigned) (m >> 27);
         a += (unsigned long long) l * l;
         b += (unsigned long long) h * l;
         c += (unsigned long long) h * h;
@@ -464,28 +478,25 @@ struct IntSums
         return IntSums{__shfl_up_sync(0xffffffffu, s, d), __shfl_up_sync(0xffffffffu, a, d),
                        __shfl_up_sync(0xffffffffu, b, d), __shfl_up_sync(0xffffffffu, c, d)};
     }
-    __device__ __forceinline__ void squares(unsigned long long &lo, unsigned long long &hi) const
+    __device__ __forceinline__ unsigned __int128 squares() const
     {
-        const unsigned __int128 q = ((unsigned __int128) c << 50) + ((unsigned __int128) b << 26) + a;
-        lo = (unsigned long long) q;
-        hi = (unsigned long long) (q >> 64);
+        return ((unsigned __int128) c << 54) + ((unsigned __int128) b << 28) + a;
     }
 };
 
-template <bool MULTI, int T> __global__ void __launch_bounds__(T / 8, T == 4096 ? 2 : 1) int_den_kernel(IntDenParams p)
+template <bool MULTI> __global__ void __launch_bounds__(kIntDenThreads, 2) int_den_kernel(IntDenParams p)
 {
     extern __shared__ __align__(16) unsigned char smem_id[];
-    __shared__ long long lred[32];
-    __shared__ IntSums wsum[32];
+    constexpr int NTH = kIntDenThreads, PER = 8, NW = NTH / 32;  // PER consecutive samples per thread, 256 per warp
+    constexpr int NP = kIntN + 16;  // prefixes 0 .. N, swizzled in groups of 16
+    __shared__ __align__(16) long long lred[64];
+    __shared__ unsigned long long ws[NW], wl[NW], wh[NW];  // sums up to and with each warp: x, x^2 (low, high)
     __shared__ int ired[32];
-    constexpr int PER = 8, NTH = T / PER;  // consecutive samples per thread
-    constexpr int NP = T + 16;             // prefixes 0 .. T, swizzled in groups of 16
-    long long *P1 = reinterpret_cast<long long *>(smem_id);
-    unsigned long long *PL = reinterpret_cast<unsigned long long *>(P1 + NP), *PH = PL + NP;
+    unsigned long long *P1 = reinterpret_cast<unsigned long long *>(smem_id), *PL = P1 + NP, *PH = PL + NP;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, g = blockIdx.y;
     const int c = MULTI ? p.grp_chan[g] : g;
     if (p.dead[c]) return;
-    const long k0 = (long) blockIdx.x * p.lags;
+    const long k0 = (long) blockIdx.x * p.S;
     const long long *x = reinterpret_cast<const long long *>(p.x + (long) c * p.ldx);
     long long v[PER];
     const long long first = x[k0];
@@ -493,15 +504,17 @@ template <bool MULTI, int T> __global__ void __launch_bounds__(T / 8, T == 4096 
     for (int i = 0; i < PER; i += 2)
     {
         // rows are 16-byte aligned and hold an even count of at least n; past
-        // the data the tile's first sample (as in the correlator)
+        // the data the block's first sample (as in the correlator)
         const long k = k0 + PER * tid + i;
         longlong2 d = make_longlong2(first, first);
         if (k < p.n) d = *reinterpret_cast<const longlong2 *>(x + k);
         v[i] = d.x;
         v[i + 1] = k + 1 < p.n ? d.y : first;
     }
-    bool bad;
-    const int ex = int_quantise<NTH, PER, false>(v, ired, lred, 0, &bad);
+    int ex;
+    const IntUnit unit = int_quantise(v, ired, lred, p.Lmax, &ex);
+    // (the groups of a channel write the same)
+    if (tid == 0) p.unit[(long) c * gridDim.x + blockIdx.x] = unit;
     // ---- prefix sums: thread, warp, block
     IntSums inc{0, 0, 0, 0};
 #pragma unroll
@@ -515,46 +528,65 @@ template <bool MULTI, int T> __global__ void __launch_bounds__(T / 8, T == 4096 
         const IntSums u = inc.shfl_up(o);
         if (lane >= o) inc.add(u);
     }
-    if (lane == 31) wsum[w] = inc;
+    if (lane == 31)
+    {
+        const unsigned __int128 q = inc.squares();
+        ws[w] = inc.s;
+        wl[w] = (unsigned long long) q;
+        wh[w] = (unsigned long long) (q >> 64);
+    }
     __syncthreads();
     if (w == 0)
     {
-        IntSums t = lane < NTH / 32 ? wsum[lane] : IntSums{0, 0, 0, 0};
+        unsigned long long s1 = lane < NW ? ws[lane] : 0;
+        unsigned __int128 s2 = lane < NW ? ((unsigned __int128) wh[lane] << 64) | wl[lane] : 0;
 #pragma unroll
-        for (int o = 1; o < NTH / 32; o <<= 1)
+        for (int o = 1; o < NW; o <<= 1)
         {
-            const IntSums u = t.shfl_up(o);
-            if (lane >= o) t.add(u);
+            const unsigned long long u1 = __shfl_up_sync(0xffffffffu, s1, o);
+            const unsigned long long ul = __shfl_up_sync(0xffffffffu, (unsigned long long) s2, o);
+            const unsigned long long uh = __shfl_up_sync(0xffffffffu, (unsigned long long) (s2 >> 64), o);
+            if (lane >= o)
+            {
+                s1 += u1;
+                s2 += ((unsigned __int128) uh << 64) | ul;
+            }
         }
-        if (lane < NTH / 32) wsum[lane] = t;
+        if (lane < NW)
+        {
+            ws[lane] = s1;
+            wl[lane] = (unsigned long long) s2;
+            wh[lane] = (unsigned long long) (s2 >> 64);
+        }
     }
     __syncthreads();
     IntSums ex_ = inc.shfl_up(1);
     if (lane == 0) ex_ = IntSums{0, 0, 0, 0};
-    if (w > 0) ex_.add(wsum[w - 1]);
+    const unsigned long long s0 = w > 0 ? ws[w - 1] : 0;
+    const unsigned __int128 q0 = w > 0 ? ((unsigned __int128) wh[w - 1] << 64) | wl[w - 1] : 0;
+    auto put = [&](int at) {
+        const unsigned __int128 q = q0 + ex_.squares();
+        const int k = int_pswz(at);
+        P1[k] = s0 + ex_.s;
+        PL[k] = (unsigned long long) q;
+        PH[k] = (unsigned long long) (q >> 64);
+    };
 #pragma unroll
     for (int i = 0; i < PER; ++i)
     {
-        const int k = int_pswz(PER * tid + i);
-        P1[k] = ex_.s;
-        ex_.squares(PL[k], PH[k]);
+        put(PER * tid + i);
         ex_.add(v[i]);
     }
-    if (tid == NTH - 1)
-    {
-        const int k = int_pswz(T);
-        P1[k] = ex_.s;
-        ex_.squares(PL[k], PH[k]);
-    }
+    if (tid == NTH - 1) put(kIntN);
     __syncthreads();
     const unsigned __int128 vtol = int_tol(p.tol * p.tol, ex);
     // sqrtL: sqrt(L) times the factor of the correlator's numerators
     auto lags_of = [&](int L, long nv, double *out, double sqrtL) {
-        const int n = (int) (nv - k0 < (long) p.lags ? nv - k0 : (long) p.lags);
+        const int n = (int) (nv - k0 < (long) p.S ? nv - k0 : (long) p.S);
         for (int k = tid; k < n; k += NTH)
         {
             const int a = int_pswz(k), b = int_pswz(k + L);
-            const long long S1 = P1[b] - P1[a];
+            const long long S1 = (long long) (P1[b] - P1[a]);  // below 2^61.1 by the window's norm
             const unsigned long long u = S1 < 0 ? 0ull - (unsigned long long) S1 : (unsigned long long) S1;
             const unsigned __int128 S2 = (((unsigned __int128) PH[b] << 64) | PL[b]) - (((unsigned __int128) PH[a] << 64) | PL[a]);
             const unsigned __int128 V = S2 * (unsigned) L - (unsigned __int128) u * u;
@@ -595,14 +627,13 @@ template <bool MULTI, int T> __global__ void __launch_bounds__(T / 8, T == 4096 
 //
 // Bound by the integer pipes (multiplier and ALU; issue 2 of 4 per clock).  160
 // templates of 200 .. 2,000 samples against 8 channels x 360,000: 8.35 ms (FP64
-// transforms with in-block normalisation) -> 1.71 ms + 0.42 ms normalisation;
+// transforms with in-block normalisation) -> 1.65 ms + 0.45 ms normalisation;
 // 64 channels x 360,000 with one template of 500 each: 2.69 + 1.15 (den_kernel)
-// -> 0.84 + 0.31 ms.  Signed words with centred residues took 2.14 and 0.98 ms.
+// -> 0.76 + 0.33 ms.  Signed words with centred residues took 2.14 and 0.98 ms.
 struct IntLayout
 {
-    static constexpr size_t off_red = 64;                    // after the barrier: reductions
-    static constexpr size_t off_mask = off_red + 640;        // two masks of 64 chunk bits
-    static constexpr size_t off_xh = 1024;
+    static constexpr size_t off_mask = 64;                   // after the barrier: two masks of 64 chunk bits
+    static constexpr size_t off_xh = 128;
     static constexpr size_t off_buf = off_xh + sizeof(int) * kIntPrimes * kIntN;
     static constexpr size_t off_tw = off_buf + sizeof(int) * kIntPrimes * kIntN;
     static constexpr size_t bytes = off_tw + sizeof(int) * kIntPrimes * kIntTw;
@@ -656,8 +687,6 @@ template <bool SHARED_DEN> __global__ void __launch_bounds__(kIntThreads, 1) int
 {
     extern __shared__ __align__(128) unsigned char smem_ix[];
     uint64_t *bar = reinterpret_cast<uint64_t *>(smem_ix);
-    long long *lred = reinterpret_cast<long long *>(smem_ix + IntLayout::off_red);
-    int *ired = reinterpret_cast<int *>(lred + 64);
     unsigned *Mk = reinterpret_cast<unsigned *>(smem_ix + IntLayout::off_mask);
     unsigned *xh = reinterpret_cast<unsigned *>(smem_ix + IntLayout::off_xh);
     unsigned *buf = reinterpret_cast<unsigned *>(smem_ix + IntLayout::off_buf);
@@ -696,31 +725,9 @@ template <bool SHARED_DEN> __global__ void __launch_bounds__(kIntThreads, 1) int
         }
     }
     __syncthreads();
+    const IntUnit unit = p.unit[(long) c * gridDim.x + bx];
     if (!xcorr_wait(bar, 0, x.err, x.test_skip_copy ? (1u << 12) : (1u << 24))) return;
-    bool bad;
-    int ex;
-    {
-        // samples in the first half of the exchange buffers, integers to the
-        // second half, reversed: X[(N - j) mod N] at j, so that transforms of
-        // one direction give the correlation
-        const long long *seg = reinterpret_cast<const long long *>(buf);
-        long long *xq = reinterpret_cast<long long *>(buf) + kIntN;
-        constexpr int PER = kIntN / kIntThreads;
-        long long v[PER];
-#pragma unroll
-        for (int i = 0; i < PER; ++i)
-        {
-            // past the data: the block's first sample instead of the zero
-            // tail, which would set the scale of a signal with an offset
-            const int j = tid + kIntThreads * i;
-            v[i] = seg[k0 + j < p.n ? j : 0];
-        }
-        ex = int_quantise<kIntThreads, PER, true>(v, ired, lred, p.Lmax, &bad);
-#pragma unroll
-        for (int i = 0; i < PER; ++i) xq[(kIntN - (tid + kIntThreads * i)) & (kIntN - 1)] = v[i];
-        __syncthreads();
-    }
-    if (bad)
+    if (unit.emax < 0)
     {
         // an infinity or NaN reaches every lag of an FP64 transform's block
         for (int ti = t_begin; ti < t_end; ++ti)
@@ -732,6 +739,23 @@ template <bool SHARED_DEN> __global__ void __launch_bounds__(kIntThreads, 1) int
                 if (k0 + k < nv) dst[k0 + k] = __longlong_as_double(0x7ff8000000000000ll);
         }
         return;
+    }
+    const int ex = int_unit_exponent(unit);
+    {
+        // samples in the first half of the exchange buffers, integers to the
+        // second half, reversed: X[(N - j) mod N] at j, so that transforms of
+        // one direction give the correlation
+        const long long *seg = reinterpret_cast<const long long *>(buf);
+        long long *xq = reinterpret_cast<long long *>(buf) + kIntN;
+#pragma unroll
+        for (int i = 0; i < kIntN / kIntThreads; ++i)
+        {
+            // past the data: the block's first sample instead of the zero
+            // tail, which would set the scale of a signal with an offset
+            const int j = tid + kIntThreads * i;
+            xq[(kIntN - j) & (kIntN - 1)] = int_sample(unit, int_fixed(seg[k0 + j < p.n ? j : 0], unit.emax));
+        }
+        __syncthreads();
     }
     // (the same for the warp, and known to be: the constants stay uniform)
     const int team = __shfl_sync(0xffffffffu, tid >> 8, 0), q = tid & 255, bar_id = 1 + team;

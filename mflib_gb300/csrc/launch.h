@@ -44,15 +44,16 @@ template <class T> cudaError_t launch_dead(const T *x, long ldx, int nch, long n
                                            T *pmax, int nchunks, cudaStream_t s, float *range = nullptr);
 // FP64 correlator in integer arithmetic (kernels_int.cuh): twiddles to upload,
 // template table (4 x kIntN words per template), normalisation (rows per
-// channel, or per template in rho), correlator over blocks of x.S lags
+// channel, or per template in rho; and the blocks' units), correlator over
+// blocks of x.S lags
 const std::vector<unsigned> &int_twiddles();
 // M 2^-64 2^-53: the numerators' unit (IntDenParams::scale)
 double int_numerator_scale();
 cudaError_t launch_int_bank(const double *tmpl, const long *toff, const int *tlen, int nt, const unsigned *tw, unsigned *B,
                             cudaStream_t s);
-cudaError_t launch_int_den(const IntDenParams &p, bool multi, int tile, int ntiles, int ngroups, cudaStream_t s);
-cudaError_t launch_int_xcorr(const XcorrParams<double> &x, bool shared_den, const unsigned *B, const unsigned *tw, int Lmax, long n,
-                             int nblocks, int ngroups, cudaStream_t s);
+cudaError_t launch_int_den(const IntDenParams &p, bool multi, int nblocks, int ngroups, cudaStream_t s);
+cudaError_t launch_int_xcorr(const XcorrParams<double> &x, bool shared_den, const unsigned *B, const unsigned *tw,
+                             const IntUnit *unit, long n, int nblocks, int ngroups, cudaStream_t s);
 // tensor-core correlator (FP32, one template length): shared memory per CTA,
 // the template bank in MMA layout (ngroups * Gp slots), the persistent launch
 size_t tc_smem_bytes(int Kp, int Gp);

@@ -115,25 +115,21 @@ cudaError_t launch_int_bank(const double *tmpl, const long *toff, const int *tle
     return cudaGetLastError();
 }
 
-template <bool MULTI, int T> static cudaError_t go_den(const IntDenParams &p, int ntiles, int ngroups, cudaStream_t s)
+cudaError_t launch_int_den(const IntDenParams &p, bool multi, int nblocks, int ngroups, cudaStream_t s)
 {
-    static SmemCap cap;
-    cudaError_t e = raise_smem_cap(int_den_kernel<MULTI, T>, int_den_bytes(T), cap);
+    static SmemCap caps, capm;
+    cudaError_t e = multi ? raise_smem_cap(int_den_kernel<true>, int_den_bytes(), capm)
+                          : raise_smem_cap(int_den_kernel<false>, int_den_bytes(), caps);
     if (e != cudaSuccess) return e;
-    int_den_kernel<MULTI, T><<<dim3(ntiles, ngroups), T / 8, int_den_bytes(T), s>>>(p);
+    if (multi) int_den_kernel<true><<<dim3(nblocks, ngroups), kIntDenThreads, int_den_bytes(), s>>>(p);
+    else int_den_kernel<false><<<dim3(nblocks, ngroups), kIntDenThreads, int_den_bytes(), s>>>(p);
     return cudaGetLastError();
 }
 
-cudaError_t launch_int_den(const IntDenParams &p, bool multi, int tile, int ntiles, int ngroups, cudaStream_t s)
+cudaError_t launch_int_xcorr(const XcorrParams<double> &x, bool shared_den, const unsigned *B, const unsigned *tw,
+                             const IntUnit *unit, long n, int nblocks, int ngroups, cudaStream_t s)
 {
-    if (tile == 4096) return multi ? go_den<true, 4096>(p, ntiles, ngroups, s) : go_den<false, 4096>(p, ntiles, ngroups, s);
-    return multi ? go_den<true, 8192>(p, ntiles, ngroups, s) : go_den<false, 8192>(p, ntiles, ngroups, s);
-}
-
-cudaError_t launch_int_xcorr(const XcorrParams<double> &x, bool shared_den, const unsigned *B, const unsigned *tw, int Lmax, long n,
-                             int nblocks, int ngroups, cudaStream_t s)
-{
-    IntParams p{x, B, tw, Lmax, n, tables().c};
+    IntParams p{x, B, tw, unit, n, tables().c};
     static SmemCap caps, capm;
     cudaError_t e = shared_den ? raise_smem_cap(int_xcorr_kernel<true>, IntLayout::bytes, caps)
                                : raise_smem_cap(int_xcorr_kernel<false>, IntLayout::bytes, capm);
