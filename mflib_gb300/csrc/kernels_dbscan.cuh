@@ -414,7 +414,12 @@ static __global__ void db_count_kernel(int nseg, const int *seg_off, const long 
 // numbered by their lowest point index.  One launch between one upload and
 // one read-back, where the sort on the host, nine uploads, nine launches and
 // the scans took 465 of the 535 us of an association (9,500 points in 8
-// segments; now 106 us in all).  Larger segments keep the launches above.
+// segments; now 106 us in all).  A segment's size is limited by the sort in
+// shared memory (20 bytes for each of a power of two of points: 164 KB); up to
+// there this form was the faster one wherever it was measured (one segment,
+// spread or in one neighbourhood, with and without weights: 1,024 points 65 ..
+// 117 us against 109 .. 134, 8,192 points 0.31 .. 0.49 ms against 0.53 .. 0.74).
+// Larger segments keep the launches above.
 constexpr int kDb1Cap = 8192, kDb1Threads = 1024;
 __host__ __device__ constexpr size_t db1_bytes(int n2) { return (sizeof(double) + 3 * sizeof(int)) * (size_t) n2; }
 
@@ -447,6 +452,39 @@ template <bool MAX> __device__ __forceinline__ int db1_scan(int v, int *sh, int 
     return MAX ? max(before, e) : before + e;
 }
 
+// exclusive scan over the CTA of one weight sum per thread; total and the total
+// of the magnitudes in every thread
+static __device__ __forceinline__ void db1_scan_weights(double own, double mag, double &before, double &total,
+                                                        double &mags)
+{
+    __shared__ double sw[kDb1Threads / 32], sm[kDb1Threads / 32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    double x = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1)
+    {
+        const double y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mag += __shfl_xor_sync(0xffffffffu, mag, o);
+    if (lane == 31)
+    {
+        sw[w] = x;
+        sm[w] = mag;
+    }
+    __syncthreads();
+    before = total = mags = 0;
+    for (int i = 0; i < kDb1Threads / 32; ++i)
+    {
+        if (i < w) before += sw[i];
+        total += sw[i];
+        mags += sm[i];
+    }
+    double e = __shfl_up_sync(0xffffffffu, x, 1);
+    if (lane > 0) before += e;
+}
+
 static __global__ void __launch_bounds__(kDb1Threads) db1_segment_kernel(const double *X, const double *wt,
                                                                         const int *seg_off, int n2max, double eps,
                                                                         double min_obs, int *labels, int *n_clusters)
@@ -455,9 +493,10 @@ static __global__ void __launch_bounds__(kDb1Threads) db1_segment_kernel(const d
     __shared__ int sh[33];
     unsigned long long *key = reinterpret_cast<unsigned long long *>(smem_db);
     double *xs = reinterpret_cast<double *>(smem_db);  // the sorted values, over the keys
-    int *idx = reinterpret_cast<int *>(key + n2max);   // point of each position
-    int *run = idx + n2max;                            // run of each position (-1: not core)
+    int *run = reinterpret_cast<int *>(key + n2max);   // run of each position (-1: not core)
     int *aux = run + n2max;                            // per run, then per point
+    int *idx = aux + n2max;                            // point of each position
+    double *ps = reinterpret_cast<double *>(run);      // prefix sums of the weights, over run and aux
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, s = blockIdx.x;
     const int b = seg_off[s], n = seg_off[s + 1] - b;
     if (n <= 0)
@@ -514,7 +553,7 @@ static __global__ void __launch_bounds__(kDb1Threads) db1_segment_kernel(const d
     int nv;
     db1_scan<false>(mine, sh, &nv);
     __syncthreads();
-    // ---- core points (weights summed as db1_core_kernel does)
+    // ---- core points
     if (!wt)
     {
         for (int r = tid; r < nv; r += kDb1Threads)
@@ -526,10 +565,56 @@ static __global__ void __launch_bounds__(kDb1Threads) db1_segment_kernel(const d
     }
     else
     {
+        // A neighbourhood's weight from prefix sums, where it is further from
+        // min_obs than both this sum and db1_core_kernel's can be off (less
+        // than 360 roundings of the weights' magnitudes together); the others
+        // (and weights that are no numbers) are summed as that kernel does, so
+        // that the decision is its own.  (8,192 points in one neighbourhood:
+        // 0.38 ms, without weights 0.31; a warp summing each neighbourhood took
+        // 24 ms on the one SM, the general launches take 0.74.)
+        const int per = (nv + kDb1Threads - 1) / kDb1Threads, r0 = min(nv, tid * per), r1 = min(nv, r0 + per);
+        double own = 0, mag = 0;
+        for (int r = r0; r < r1; ++r)
+        {
+            const double v = wt[b + idx[r]];
+            own += v;
+            mag += fabs(v);
+        }
+        double before, total, mags;
+        db1_scan_weights(own, mag, before, total, mags);
+        for (int r = r0; r < r1; ++r)
+        {
+            ps[r] = before;
+            before += wt[b + idx[r]];
+        }
+        __syncthreads();
+        const double margin = mags * 0x1p-42;
+        int core[kDb1Cap / kDb1Threads];
+#pragma unroll
+        for (int u = 0; u < kDb1Cap / kDb1Threads; ++u)
+        {
+            const int r = tid + u * kDb1Threads;
+            core[u] = -1;
+            if (r < nv)
+            {
+                int lo, hi;
+                db1_range(xs, 0, nv, xs[r], eps, lo, hi);
+                const double d = (hi > lo ? (hi < nv ? ps[hi] : total) - ps[lo] : 0.0) - min_obs;
+                core[u] = d > margin ? 0 : d < -margin ? -1 : -2;
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < kDb1Cap / kDb1Threads; ++u)
+            if (tid + u * kDb1Threads < nv) run[tid + u * kDb1Threads] = core[u];
+        __syncthreads();
         for (int r = w; r < nv; r += kDb1Threads / 32)
         {
-            int lo, hi;
-            db1_range(xs, 0, nv, xs[r], eps, lo, hi);
+            if (run[r] != -2) continue;  // uniform across the warp
+            int lo = 0, hi = 0;
+            if (lane == 0) db1_range(xs, 0, nv, xs[r], eps, lo, hi);
+            lo = __shfl_sync(0xffffffffu, lo, 0);
+            hi = __shfl_sync(0xffffffffu, hi, 0);
             double acc = 0;
             for (int i = lo + lane; i < hi; i += 32) acc += wt[b + idx[i]];
 #pragma unroll

@@ -1,0 +1,57 @@
+"""DBSCAN of one feature with weights: the one-CTA form against the general
+launches (taken by every segment of a call that holds one of more than 8,192
+points), and its time in dense segments."""
+import time
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+BIG = 8193
+
+
+def _both(gpu, eps, mo, x, off, w):
+    """Labels and cluster counts by the two forms."""
+    db = gpu.DBSCAN()
+    db.initialize(eps, mo)
+    labels, ncl = db.cluster_segments(x, off, w)
+    more = np.linspace(0.0, 1e9, BIG)
+    xg, wg = np.concatenate([x, more]), None if w is None else np.concatenate([w, np.ones(BIG)])
+    lg, ng = db.cluster_segments(xg, np.concatenate([off, [xg.size]]).astype(np.int32), wg)
+    return (np.asarray(labels), np.asarray(ncl)), (np.asarray(lg)[:x.size], np.asarray(ng)[:-1])
+
+
+# weights that are no binary fractions (a neighbourhood's sum depends on its
+# order where it meets min_obs), equal ones, magnitudes far apart, infinities and
+# values that are no numbers
+@pytest.mark.parametrize("kind", ["tenths", "thirds", "wide", "special"])
+@pytest.mark.parametrize("span", [0.02, 0.3, 3.0])
+def test_forms_agree(gpu, rng, kind, span):
+    sizes = (1, 2, 33, 1023, 1025, 8192)
+    off = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int32)
+    x = np.concatenate([np.round(rng.uniform(0, span * m, m) * 8) / 8 for m in sizes])
+    w = {"tenths": lambda: rng.integers(1, 12, x.size) / 10.0,
+         "thirds": lambda: np.full(x.size, 1.0 / 3.0),
+         "wide": lambda: 10.0 ** rng.uniform(-12, 6, x.size),
+         "special": lambda: np.where(rng.random(x.size) < 0.01, np.nan, np.where(rng.random(x.size) < 0.01, np.inf, 0.7))}[kind]()
+    for eps, mo in ((0.25, 1), (1.0, 3), (5.0, 40)):
+        (l1, n1), (l2, n2) = _both(gpu, eps, mo, x, off, w)
+        np.testing.assert_array_equal(n1, n2)
+        np.testing.assert_array_equal(l1, l2)
+
+
+def test_a_dense_segment_takes_no_longer_with_weights(gpu, rng):
+    """8,192 points in one neighbourhood: within five times the time without
+    weights (the same number of neighbourhood sums, each from two loads)."""
+    x, off = np.round(rng.uniform(0, 40.0, 8192)), np.array([0, 8192], np.int32)
+    db = gpu.DBSCAN()
+    db.initialize(50.0, 3)
+    best = {}
+    for name, w in (("none", None), ("weights", rng.uniform(0.5, 2.0, 8192))):
+        best[name] = 1e9
+        for _ in range(6):
+            t = time.perf_counter()
+            db.cluster_segments(x, off, w)
+            best[name] = min(best[name], time.perf_counter() - t)
+    assert best["weights"] < 5 * best["none"], best
