@@ -613,15 +613,18 @@ __global__ void __launch_bounds__(32 * kFixListWarps) fix_list_kernel(FixParams<
             __syncwarp();
             if (q + kFixListWarps < np) fetch(q + kFixListWarps, nx);
             float v[32], s = 0.f;
-            // past the longest window (its coefficients are zero) samples count
-            // as zero, also an infinity; such a piece is in no window's statistics
-            const int nin = Lb - 32 * q;
 #pragma unroll
             for (int i = 0; i < 32; ++i)
             {
-                v[i] = i < nin ? ys[lane + 32 * q + i] - Rl : 0.f;
+                v[i] = ys[lane + 32 * q + i] - Rl;
                 s += v[i];
             }
+            // past the longest window (its coefficients are zero) samples count
+            // as zero, also an infinity; such a piece is in no window's statistics
+            if (Lb < 32 * q + 32)
+#pragma unroll
+                for (int i = 1; i < 32; ++i)
+                    if (32 * q + i >= Lb) v[i] = 0.f;
             const float mu = s * (1.f / 32.f);
             float a = 0.f, b = 0.f;
 #pragma unroll
