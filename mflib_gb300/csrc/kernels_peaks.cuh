@@ -302,12 +302,24 @@ static __global__ void peak_compact_kernel(const long long *ncand_p, long long c
 }
 
 // per-trace peak offsets: peak_off[t] = pos[trace_beg[t]]
+// The traces' peak offsets; res[ntr + 1 ..]: candidates, whether the search is
+// dense, the object's device status word, candidates left undecided, overflow
+// (read back in one copy).
 static __global__ void peak_trace_offsets_kernel(int ntr, const long long *trace_beg, const long long *pos,
-                                                 long long *peak_off)
+                                                 const long long *ncand, const int *flags, const int *err,
+                                                 const int *counter, long long *res)
 {
     int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t == 0)
+    {
+        res[ntr + 1] = *ncand;
+        res[ntr + 2] = flags[0];
+        res[ntr + 3] = err ? *err : 0;
+        res[ntr + 4] = counter[0];
+        res[ntr + 5] = counter[1];
+    }
     if (t > ntr) return;
-    peak_off[t] = pos[trace_beg[t]];
+    res[t] = pos[trace_beg[t]];
 }
 
 // trace_beg[t] = min(offs[t * nchunks], cap): candidate offsets of each trace

@@ -59,7 +59,7 @@ int run_peaks(const T *x, long ldx, const int *host_rows, int ntr, int len, doub
         if (ws.row.p != old) ws.rows_on_device.clear();  // a new buffer holds no rows
     }
     MF_TRY(ws.trace_beg.ensure(sizeof(long long) * (ntr + 1)));
-    MF_TRY(ws.peak_off.ensure(sizeof(long long) * (ntr + 4)));
+    MF_TRY(ws.peak_off.ensure(sizeof(long long) * (ntr + 6)));
     MF_TRY(ws.counts.ensure(sizeof(int) * nslots));
     if (fused) MF_TRY(ws.ht.ensure(nslots));
     else
@@ -113,13 +113,14 @@ int run_peaks(const T *x, long ldx, const int *host_rows, int ntr, int len, doub
     // attempt that fails costs two launches and a wait.  The form below renews
     // the flag from the counts of its own traces.
     const PeakSearch search{thr, ntr, len, dist, fused != nullptr};
+    long long *res = ws.peak_off.as<long long>();
+    std::vector<long long> got(ntr + 6);
     while (!(ws.dense && ws.dense_search == search))
     {
         const long long cap = ws.cand_cap;
         MF_TRY(ws.nacc.ensure(sizeof(int) * ntr));
         MF_TRY(ws.cidx.ensure(sizeof(int) * cap));
         MF_TRY(ws.peaks.ensure(sizeof(int) * cap));
-        long long *res = ws.peak_off.as<long long>();
         const size_t bytes = pk_prune_bytes<T>();
         static SmemCap capf, caps;
         if (fused)
@@ -140,7 +141,6 @@ int run_peaks(const T *x, long ldx, const int *host_rows, int ntr, int len, doub
                                             ws.peaks.as<int>());
         *launches += 2;
         MF_TRY(cudaGetLastError());
-        std::vector<long long> got(ntr + 4);
         MF_TRY(cudaMemcpyAsync(got.data(), res, sizeof(long long) * (ntr + 4), cudaMemcpyDeviceToHost, s));
         MF_TRY(cudaStreamSynchronize(s));
         if (host_err) *host_err = (int) got[ntr + 3];
@@ -197,9 +197,8 @@ int run_peaks(const T *x, long ldx, const int *host_rows, int ntr, int len, doub
         // Pruning rounds, checked in batches: every round accepts at least
         // the highest-priority undecided candidate of each trace.
         long long rounds_done = 0;
-        int left = 0;
         long long ncand = 0;
-        int ovf = 0, dense = 0;
+        bool left = false, ovf = false, dense = false;
         for (;;)
         {
             if (prune)
@@ -227,22 +226,19 @@ int run_peaks(const T *x, long ldx, const int *host_rows, int ntr, int len, doub
             peak_compact_kernel<<<gblocks, kPkThreads, 0, s>>>(ncand_dev, cap, ws.flags.as<int>(),
                                                                ws.pos.as<long long>(), ws.cidx.as<int>(),
                                                                ws.peaks.as<int>());
-            peak_trace_offsets_kernel<<<(ntr + 1 + 127) / 128, 128, 0, s>>>(ntr, ws.trace_beg.as<long long>(),
-                                                                            ws.pos.as<long long>(),
-                                                                            ws.peak_off.as<long long>());
+            peak_trace_offsets_kernel<<<(ntr + 1 + 127) / 128, 128, 0, s>>>(
+                ntr, ws.trace_beg.as<long long>(), ws.pos.as<long long>(), ncand_dev, tick + 2, dev_err, undecided, res);
             *launches += 2;
             MF_TRY(cudaGetLastError());
-            MF_TRY(cudaMemcpyAsync(host_peak_off, ws.peak_off.p, sizeof(long long) * (ntr + 1),
-                                   cudaMemcpyDeviceToHost, s));
-            MF_TRY(cudaMemcpyAsync(&ncand, ncand_dev, sizeof(long long), cudaMemcpyDeviceToHost, s));
-            MF_TRY(cudaMemcpyAsync(&left, undecided, sizeof(int), cudaMemcpyDeviceToHost, s));
-            MF_TRY(cudaMemcpyAsync(&ovf, overflow, sizeof(int), cudaMemcpyDeviceToHost, s));
-            MF_TRY(cudaMemcpyAsync(&dense, tick + 2, sizeof(int), cudaMemcpyDeviceToHost, s));
-            if (dev_err && host_err)
-                MF_TRY(cudaMemcpyAsync(host_err, dev_err, sizeof(int), cudaMemcpyDeviceToHost, s));
+            MF_TRY(cudaMemcpyAsync(got.data(), res, sizeof(long long) * (ntr + 6), cudaMemcpyDeviceToHost, s));
             MF_TRY(cudaStreamSynchronize(s));
+            ncand = got[ntr + 1];
+            dense = got[ntr + 2] != 0;
+            if (host_err) *host_err = (int) got[ntr + 3];
+            left = got[ntr + 4] != 0;
+            ovf = got[ntr + 5] != 0;
             if (ovf || ncand > cap) break;
-            if (!prune || left == 0) break;
+            if (!prune || !left) break;
             if (rounds_done > ncand + 16)
             {
                 err = "peak pruning did not converge";
@@ -254,8 +250,9 @@ int run_peaks(const T *x, long ldx, const int *host_rows, int ntr, int len, doub
             ws.cand_cap = std::max<long long>(2 * cap, ncand + ncand / 4 + 1024);
             continue;
         }
+        std::copy(got.begin(), got.begin() + ntr + 1, host_peak_off);
         ws.npeaks = host_peak_off[ntr];
-        ws.dense = dense != 0;
+        ws.dense = dense;
         return 0;
     }
     err = "peak candidate capacity could not be sized";
