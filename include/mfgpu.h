@@ -223,7 +223,8 @@ mfgpu_status mfgpu_mf_get_plan(const mfgpu_mf *mf, int *fft_length, int *lags_pe
 /* Correlator organisation chosen at initialize, numbered like
  * correlator_variant (1-3, 5 and 6 FFT organisations, 4 tensor cores), or 7 for
  * the integer transforms that FP64 data take unless an FFT length, an
- * organisation or several buckets are asked for; for the tensor-core path also the templates per group and the padded K, else 0.
+ * organisation or several buckets are asked for; for the tensor-core path also
+ * the templates per group and the padded K, else 0.
  * Extension: the reference has one CPU correlator and no such query. */
 mfgpu_status mfgpu_mf_get_correlator(const mfgpu_mf *mf, int *variant, int *tc_group, int *tc_k);
 /* Length buckets chosen at initialize: their number, and for each (up to

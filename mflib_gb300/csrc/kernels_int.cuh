@@ -28,13 +28,14 @@
 // The remaining errors are the two roundings of the inputs and three roundings
 // to FP64 at the end.  A sample's is at most half a unit of its block, so a
 // coefficient whose window has the 2-norm W about its mean, in a block whose
-// loudest window has the norm A, errs by less than 2^-53 sqrt(L) A / W, about
-// 2^-56 A / W as a rule, besides some 1e-16; no sample outside the block counts.  An FP64 transform's rounding is 2^-53 of the block's norm spread over its
-// lags, and running FP64 sums of squares lose (A / W)^2 2^-53 after the loud
-// part.  Against exact sums, windows of 200 .. 2,000 samples of noise: 0.8e-16 ..
-// 1.1e-16 here, 0.6e-16 .. 3.9e-16 by the transform and its in-block sums;
-// quiet windows of a block with a part 1e3 (1e6) times louder: 0.5e-15 .. 6e-14
-// (0.5e-12 .. 8e-11) here, 0.4e-15 .. 2e-10 (1e-12 .. 3e-4) by the others.
+// loudest window has the norm A, errs by less than 2^-53 sqrt(L) A / W besides
+// the roundings at the end (about 2^-56 A / W as a rule); no sample outside the
+// block counts.  An FP64 transform's rounding is 2^-53 of the block's norm spread
+// over its lags, and its in-block sums of squares lose (A / W)^2 2^-53 of a
+// window after a loud part.  Errors against sums in 64 bits (whose own rounding
+// is in them) in the workloads of perf/cases.py: 1.2e-15 (three templates of
+// 1,001), 4.0e-16 (64 of 500) and 1.1e-15 (160 of 200 .. 2,000), by FP64
+// transforms 1.3e-15, 6.7e-16 and 1.2e-15.
 //
 // Arithmetic modulo p: Montgomery products with R = 2^32 on unsigned words
 // (wide multiply, low multiply, wide multiply-add; the signed forms cost two
@@ -439,8 +440,9 @@ __device__ __forceinline__ double int_inv_den(unsigned __int128 V, int ex, doubl
 // two loads each of S1 and S2: about 90 integer instructions and one FP64
 // product per lag, against some 27 FP64 operations (16 clocks per SM) of the
 // running FP64 form.  64 x 360,000, L = 500: 335 us; 8 x 360,000, 160 templates of
-// 200 .. 2,000: 450 us; bound by the integer pipes.  The block's unit is found
-// here and read by the correlator, whose own reductions for it took 80 and 60 us
+// 200 .. 2,000: 450 us; bound by the ALU pipe (65 % busy, issue 63 %) and, with
+// several lengths, by the FP64 product per lag (its pipe 63 %).  The block's unit
+// is found here and read by the correlator, whose own reductions for it took 80 and 60 us
 // of the same cases.  Tiles and integers of its own (50 bits; tiles of 8,192
 // samples above L = 1,024) took 308 and 424 us, but a loud sample outside a
 // block then took digits from that block's coefficients (a sample 1e6 times the
@@ -625,7 +627,8 @@ template <bool MULTI> __global__ void __launch_bounds__(kIntDenThreads, 2) int_d
 // threads combine them, four lags each.  Shared memory: the block's four
 // spectra (64 KB), four exchange buffers (64 KB), the twiddles (65 KB).
 //
-// Bound by the integer pipes (multiplier and ALU; issue 2 of 4 per clock).  160
+// Bound by the multiplier (the largest stall is its throttle), then barriers and
+// spectra from L2; issue 2.0 of 4 per clock.  160
 // templates of 200 .. 2,000 samples against 8 channels x 360,000: 8.35 ms (FP64
 // transforms with in-block normalisation) -> 1.65 ms + 0.45 ms normalisation;
 // 64 channels x 360,000 with one template of 500 each: 2.69 + 1.15 (den_kernel)
