@@ -276,7 +276,10 @@ int run_dbscan(int n, int nf, const double *X, const double *w, double eps, int 
     }
     int most = 0;
     for (int sg = 0; sg < nseg; ++sg) most = std::max(most, seg_off_host[sg + 1] - seg_off_host[sg]);
-    if (nf == 1 && most <= kDb1Cap)
+    // (weights in data holding a NaN are summed in the points' order by the full
+    // scans below, whose rounding decides where a sum meets min_obs)
+    const bool points_order = w && std::any_of(X, X + (size_t) n * nf, [](double v) { return std::isnan(v); });
+    if (nf == 1 && most <= kDb1Cap && !points_order)
     {
         // one CTA per segment: points (and weights) up, labels and counts down
         int n2 = 1;

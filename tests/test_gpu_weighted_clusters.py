@@ -55,3 +55,37 @@ def test_a_dense_segment_takes_no_longer_with_weights(gpu, rng):
             db.cluster_segments(x, off, w)
             best[name] = min(best[name], time.perf_counter() - t)
     assert best["weights"] < 5 * best["none"], best
+
+
+def _lane_sums(values, places):
+    """Sums as a warp forms them: the value at place j by lane j mod 32, then a tree over the lanes."""
+    acc = np.zeros((len(values), 32))
+    for k in range(values.shape[1]):
+        acc[np.arange(len(values)), places[:, k] % 32] += values[:, k]
+    for o in (16, 8, 4, 2, 1):
+        acc = acc + acc[:, np.arange(32) ^ o]
+    return acc[:, 0]
+
+
+def test_weights_beside_a_nan_are_summed_in_the_points_order(gpu, rng):
+    """Data holding a NaN are scanned in the points' own order.  Groups of
+    points whose weights, sevenths, add up to min_obs but for rounding: each
+    decides as that sum does."""
+    groups, m, mo = 600, 12, 3
+    k = rng.integers(1, 3, (groups, m))
+    k[:, -1] = 7 * mo - k[:, :-1].sum(axis=1)
+    k = k[k[:, -1] > 0]
+    groups = len(k)
+    place = np.sort(rng.permutation(groups * m).reshape(groups, m), axis=1) + 1  # the points of each group
+    x, w = np.full(groups * m + 1, np.nan), np.ones(groups * m + 1)
+    x[place] = 100.0 * np.arange(groups)[:, None]
+    w[place] = k / 7.0
+    values = w[place]
+    core = _lane_sums(values, place) >= mo
+    by_value = _lane_sums(values, m * np.arange(groups)[:, None] + np.arange(m)) >= mo
+    assert np.any(core != by_value)
+    db = gpu.DBSCAN()
+    db.initialize(1.0, mo)
+    labels, ncl = db.cluster_segments(x, np.array([0, x.size], np.int32), w)
+    assert ncl[0] == core.sum()
+    np.testing.assert_array_equal(np.asarray(labels)[place] >= 0, core[:, None].repeat(m, 1))
