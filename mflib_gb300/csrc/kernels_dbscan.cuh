@@ -420,12 +420,19 @@ static __global__ void db_count_kernel(int nseg, const int *seg_off, const long 
 // spread or in one neighbourhood, with and without weights: 1,024 points 65 ..
 // 117 us against 109 .. 134, 8,192 points 0.31 .. 0.49 ms against 0.53 .. 0.74).
 // Larger segments keep the launches above.
-constexpr int kDb1Cap = 8192, kDb1Threads = 1024;
+//
+// A CTA of NT threads takes segments of up to 8 NT points: 1,024 threads, and
+// where there are more segments than the chip holds CTAs of that size (two per
+// SM), 32 or 128 if the largest segment allows.  (100,000 segments of two points:
+// in CTAs of 1,024 threads 3.9 .. 5.0 ms, of one warp 0.37, the launches above 1.9;
+// 5,000 of 100: 0.55 .. 0.69, 0.33 and 14.7 ms.)
+constexpr int kDb1Per = 8, kDb1Cap = 8192;
+constexpr int kDb1Resident = 2 * 152;
 __host__ __device__ constexpr size_t db1_bytes(int n2) { return (sizeof(double) + 3 * sizeof(int)) * (size_t) n2; }
 
 // exclusive scan over the CTA of one value per thread (sum or maximum);
 // sh: 33 ints; the total goes to *total
-template <bool MAX> __device__ __forceinline__ int db1_scan(int v, int *sh, int *total)
+template <bool MAX, int NT> __device__ __forceinline__ int db1_scan(int v, int *sh, int *total)
 {
     constexpr int none = MAX ? -1 : 0;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -440,7 +447,7 @@ template <bool MAX> __device__ __forceinline__ int db1_scan(int v, int *sh, int 
     if (lane == 31) sh[w] = x;
     __syncthreads();
     int before = none, all = none;
-    for (int i = 0; i < kDb1Threads / 32; ++i)
+    for (int i = 0; i < NT / 32; ++i)
     {
         const int t = sh[i];
         if (i < w) before = MAX ? max(before, t) : before + t;
@@ -454,10 +461,11 @@ template <bool MAX> __device__ __forceinline__ int db1_scan(int v, int *sh, int 
 
 // exclusive scan over the CTA of one weight sum per thread; total and the total
 // of the magnitudes in every thread
-static __device__ __forceinline__ void db1_scan_weights(double own, double mag, double &before, double &total,
-                                                        double &mags)
+template <int NT>
+__device__ __forceinline__ void db1_scan_weights(double own, double mag, double &before, double &total, double &mags)
 {
-    __shared__ double sw[kDb1Threads / 32], sm[kDb1Threads / 32];
+    constexpr int NW = NT / 32;
+    __shared__ double sw[NW], sm[NW], all[2];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     double x = own;
 #pragma unroll
@@ -474,20 +482,35 @@ static __device__ __forceinline__ void db1_scan_weights(double own, double mag, 
         sm[w] = mag;
     }
     __syncthreads();
-    before = total = mags = 0;
-    for (int i = 0; i < kDb1Threads / 32; ++i)
+    // the warps' sums by one warp: 32 warps adding 32 sums each would keep the
+    // FP64 pipe busy for 30 us
+    if (w == 0)
     {
-        if (i < w) before += sw[i];
-        total += sw[i];
-        mags += sm[i];
+        const double y = lane < NW ? sw[lane] : 0.0;
+        double t = y, m = lane < NW ? sm[lane] : 0.0;
+#pragma unroll
+        for (int o = 1; o < NW; o <<= 1)
+        {
+            const double u = __shfl_up_sync(0xffffffffu, t, o);
+            if (lane >= o) t += u;
+            m += __shfl_xor_sync(0xffffffffu, m, o);
+        }
+        const double e = __shfl_up_sync(0xffffffffu, t, 1);
+        if (lane < NW) sw[lane] = lane > 0 ? e : 0.0;
+        if (lane == NW - 1) all[0] = t;
+        if (lane == 0) all[1] = m;
     }
-    double e = __shfl_up_sync(0xffffffffu, x, 1);
-    if (lane > 0) before += e;
+    __syncthreads();
+    total = all[0];
+    mags = all[1];
+    const double e = __shfl_up_sync(0xffffffffu, x, 1);
+    before = sw[w] + (lane > 0 ? e : 0.0);
 }
 
-static __global__ void __launch_bounds__(kDb1Threads) db1_segment_kernel(const double *X, const double *wt,
-                                                                        const int *seg_off, int n2max, double eps,
-                                                                        double min_obs, int *labels, int *n_clusters)
+template <int NT>
+static __global__ void __launch_bounds__(NT) db1_segment_kernel(const double *X, const double *wt, const int *seg_off,
+                                                               int n2max, double eps, double min_obs, int *labels,
+                                                               int *n_clusters)
 {
     extern __shared__ __align__(16) unsigned char smem_db[];
     __shared__ int sh[33];
@@ -507,7 +530,7 @@ static __global__ void __launch_bounds__(kDb1Threads) db1_segment_kernel(const d
     int n2 = 1;
     while (n2 < n) n2 <<= 1;
     // ---- sort: order-preserving integer keys (-0 as +0), NaN and padding last
-    for (int i = tid; i < n2; i += kDb1Threads)
+    for (int i = tid; i < n2; i += NT)
     {
         unsigned long long k = ~0ull;
         if (i < n)
@@ -523,7 +546,7 @@ static __global__ void __launch_bounds__(kDb1Threads) db1_segment_kernel(const d
     for (int k = 2; k <= n2; k <<= 1)
         for (int j = k >> 1; j > 0; j >>= 1)
         {
-            for (int i = tid; i < n2 / 2; i += kDb1Threads)
+            for (int i = tid; i < n2 / 2; i += NT)
             {
                 const int p = 2 * i - (i & (j - 1)), q = p + j;
                 const unsigned long long ka = key[p], kb = key[q];
@@ -541,7 +564,7 @@ static __global__ void __launch_bounds__(kDb1Threads) db1_segment_kernel(const d
         }
     // ---- values in place; nv: points that are no NaN
     int mine = 0;
-    for (int i = tid; i < n; i += kDb1Threads)
+    for (int i = tid; i < n; i += NT)
     {
         const unsigned long long k = key[i];
         if (k != ~0ull)
@@ -551,12 +574,12 @@ static __global__ void __launch_bounds__(kDb1Threads) db1_segment_kernel(const d
         }
     }
     int nv;
-    db1_scan<false>(mine, sh, &nv);
+    db1_scan<false, NT>(mine, sh, &nv);
     __syncthreads();
     // ---- core points
     if (!wt)
     {
-        for (int r = tid; r < nv; r += kDb1Threads)
+        for (int r = tid; r < nv; r += NT)
         {
             int lo, hi;
             db1_range(xs, 0, nv, xs[r], eps, lo, hi);
@@ -570,9 +593,9 @@ static __global__ void __launch_bounds__(kDb1Threads) db1_segment_kernel(const d
         // than 360 roundings of the weights' magnitudes together); the others
         // (and weights that are no numbers) are summed as that kernel does, so
         // that the decision is its own.  (8,192 points in one neighbourhood:
-        // 0.38 ms, without weights 0.31; a warp summing each neighbourhood took
+        // 0.36 ms, without weights 0.31; a warp summing each neighbourhood took
         // 24 ms on the one SM, the general launches take 0.74.)
-        const int per = (nv + kDb1Threads - 1) / kDb1Threads, r0 = min(nv, tid * per), r1 = min(nv, r0 + per);
+        const int per = (nv + NT - 1) / NT, r0 = min(nv, tid * per), r1 = min(nv, r0 + per);
         double own = 0, mag = 0;
         for (int r = r0; r < r1; ++r)
         {
@@ -581,7 +604,7 @@ static __global__ void __launch_bounds__(kDb1Threads) db1_segment_kernel(const d
             mag += fabs(v);
         }
         double before, total, mags;
-        db1_scan_weights(own, mag, before, total, mags);
+        db1_scan_weights<NT>(own, mag, before, total, mags);
         for (int r = r0; r < r1; ++r)
         {
             ps[r] = before;
@@ -589,11 +612,11 @@ static __global__ void __launch_bounds__(kDb1Threads) db1_segment_kernel(const d
         }
         __syncthreads();
         const double margin = mags * 0x1p-42;
-        int core[kDb1Cap / kDb1Threads];
+        int core[kDb1Per];
 #pragma unroll
-        for (int u = 0; u < kDb1Cap / kDb1Threads; ++u)
+        for (int u = 0; u < kDb1Per; ++u)
         {
-            const int r = tid + u * kDb1Threads;
+            const int r = tid + u * NT;
             core[u] = -1;
             if (r < nv)
             {
@@ -605,10 +628,10 @@ static __global__ void __launch_bounds__(kDb1Threads) db1_segment_kernel(const d
         }
         __syncthreads();
 #pragma unroll
-        for (int u = 0; u < kDb1Cap / kDb1Threads; ++u)
-            if (tid + u * kDb1Threads < nv) run[tid + u * kDb1Threads] = core[u];
+        for (int u = 0; u < kDb1Per; ++u)
+            if (tid + u * NT < nv) run[tid + u * NT] = core[u];
         __syncthreads();
-        for (int r = w; r < nv; r += kDb1Threads / 32)
+        for (int r = w; r < nv; r += NT / 32)
         {
             if (run[r] != -2) continue;  // uniform across the warp
             int lo = 0, hi = 0;
@@ -624,11 +647,11 @@ static __global__ void __launch_bounds__(kDb1Threads) db1_segment_kernel(const d
     }
     __syncthreads();
     // ---- runs: each thread a piece of consecutive positions
-    const int per = (nv + kDb1Threads - 1) / kDb1Threads, r0 = min(nv, tid * per), r1 = min(nv, r0 + per);
+    const int per = (nv + NT - 1) / NT, r0 = min(nv, tid * per), r1 = min(nv, r0 + per);
     int last = -1, tot;
     for (int r = r0; r < r1; ++r)
         if (run[r] == 0) last = r;
-    int prev = db1_scan<true>(last, sh, &tot);  // nearest core position before the piece
+    int prev = db1_scan<true, NT>(last, sh, &tot);  // nearest core position before the piece
     const int prev0 = prev;
     int starts = 0;
     for (int r = r0; r < r1; ++r)
@@ -638,7 +661,7 @@ static __global__ void __launch_bounds__(kDb1Threads) db1_segment_kernel(const d
             prev = r;
         }
     int nrun;
-    int id = db1_scan<false>(starts, sh, &nrun) - 1;  // the run the piece begins in
+    int id = db1_scan<false, NT>(starts, sh, &nrun) - 1;  // the run the piece begins in
     prev = prev0;
     for (int r = r0; r < r1; ++r)
         if (run[r] == 0)
@@ -647,31 +670,31 @@ static __global__ void __launch_bounds__(kDb1Threads) db1_segment_kernel(const d
             prev = r;
             run[r] = id;
         }
-    for (int i = tid; i < nrun; i += kDb1Threads) aux[i] = n;
+    for (int i = tid; i < nrun; i += NT) aux[i] = n;
     __syncthreads();
-    for (int r = tid; r < nv; r += kDb1Threads)
+    for (int r = tid; r < nv; r += NT)
         if (run[r] >= 0) atomicMin(aux + run[r], idx[r]);
     __syncthreads();
     // ---- cluster number of a run: how many runs have a lower first point.
     // The first points in index order, by a scan over marks
-    int root[kDb1Cap / kDb1Threads];
+    int root[kDb1Per];
 #pragma unroll
-    for (int u = 0; u < kDb1Cap / kDb1Threads; ++u)
+    for (int u = 0; u < kDb1Per; ++u)
     {
-        const int i = tid + u * kDb1Threads;
+        const int i = tid + u * NT;
         root[u] = i < nrun ? aux[i] : -1;
     }
     __syncthreads();
-    for (int i = tid; i < n; i += kDb1Threads) aux[i] = 0;
+    for (int i = tid; i < n; i += NT) aux[i] = 0;
     __syncthreads();
 #pragma unroll
-    for (int u = 0; u < kDb1Cap / kDb1Threads; ++u)
+    for (int u = 0; u < kDb1Per; ++u)
         if (root[u] >= 0) aux[root[u]] = 1;
     __syncthreads();
-    const int pern = (n + kDb1Threads - 1) / kDb1Threads, i0 = min(n, tid * pern), i1 = min(n, i0 + pern);
+    const int pern = (n + NT - 1) / NT, i0 = min(n, tid * pern), i1 = min(n, i0 + pern);
     int marks = 0;
     for (int i = i0; i < i1; ++i) marks += aux[i];
-    int base = db1_scan<false>(marks, sh, &tot);
+    int base = db1_scan<false, NT>(marks, sh, &tot);
     for (int i = i0; i < i1; ++i)
     {
         const int m = aux[i];
@@ -679,16 +702,16 @@ static __global__ void __launch_bounds__(kDb1Threads) db1_segment_kernel(const d
         base += m;
     }
     __syncthreads();
-    int num[kDb1Cap / kDb1Threads];
+    int num[kDb1Per];
 #pragma unroll
-    for (int u = 0; u < kDb1Cap / kDb1Threads; ++u) num[u] = root[u] >= 0 ? aux[root[u]] : 0;
+    for (int u = 0; u < kDb1Per; ++u) num[u] = root[u] >= 0 ? aux[root[u]] : 0;
     __syncthreads();
 #pragma unroll
-    for (int u = 0; u < kDb1Cap / kDb1Threads; ++u)
-        if (root[u] >= 0) aux[tid + u * kDb1Threads] = num[u];
+    for (int u = 0; u < kDb1Per; ++u)
+        if (root[u] >= 0) aux[tid + u * NT] = num[u];
     __syncthreads();
     // ---- labels: a core point's run; else the lowest cluster among the core neighbours
-    for (int r = tid; r < n; r += kDb1Threads)
+    for (int r = tid; r < n; r += NT)
     {
         int lab = -1;
         if (r < nv)

@@ -278,8 +278,13 @@ int run_dbscan(int n, int nf, const double *X, const double *w, double eps, int 
     for (int sg = 0; sg < nseg; ++sg) most = std::max(most, seg_off_host[sg + 1] - seg_off_host[sg]);
     // (weights in data holding a NaN are summed in the points' order by the full
     // scans below, whose rounding decides where a sum meets min_obs)
-    const bool points_order = w && std::any_of(X, X + (size_t) n * nf, [](double v) { return std::isnan(v); });
-    if (nf == 1 && most <= kDb1Cap && !points_order)
+    const bool points_order = nf == 1 && w && std::any_of(X, X + n, [](double v) { return std::isnan(v); });
+    // threads per segment; segments of a few points beside one that needs the
+    // large CTA are left to the general launches (39 ns each in such CTAs, 10 ns
+    // per point there)
+    const int nt1 = nseg <= kDb1Resident || most > kDb1Per * 128 ? 1024 : most > kDb1Per * 32 ? 128 : 32;
+    const bool few = nt1 == 1024 && nseg > kDb1Resident && n < 4 * (long) nseg;
+    if (nf == 1 && most <= kDb1Cap && !points_order && !few)
     {
         // one CTA per segment: points (and weights) up, labels and counts down
         int n2 = 1;
@@ -292,12 +297,17 @@ int run_dbscan(int n, int nf, const double *X, const double *w, double eps, int 
         MF_TRY(cudaMemcpyAsync(ws.X.p, X, sizeof(double) * (size_t) n, cudaMemcpyHostToDevice, s));
         if (w) MF_TRY(cudaMemcpyAsync(wd, w, sizeof(double) * (size_t) n, cudaMemcpyHostToDevice, s));
         MF_TRY(cudaMemcpyAsync(ws.seg_off.p, seg_off_host, sizeof(int) * (size_t) (nseg + 1), cudaMemcpyHostToDevice, s));
-        static SmemCap cap;
-        MF_TRY(raise_smem_cap(db1_segment_kernel, db1_bytes(n2), cap));
-        db1_segment_kernel<<<nseg, kDb1Threads, db1_bytes(n2), s>>>(ws.X.as<double>(), wd, ws.seg_off.as<int>(), n2, eps,
-                                                                  (double) min_obs, lab, lab + n);
+        auto launch = [&](auto kernel, SmemCap &cap) {
+            const cudaError_t e = raise_smem_cap(kernel, db1_bytes(n2), cap);
+            if (e != cudaSuccess) return e;
+            kernel<<<nseg, nt1, db1_bytes(n2), s>>>(ws.X.as<double>(), wd, ws.seg_off.as<int>(), n2, eps, (double) min_obs,
+                                                   lab, lab + n);
+            return cudaGetLastError();
+        };
+        static SmemCap caps[3];
+        MF_TRY(nt1 == 1024 ? launch(db1_segment_kernel<1024>, caps[0])
+                           : nt1 == 128 ? launch(db1_segment_kernel<128>, caps[1]) : launch(db1_segment_kernel<32>, caps[2]));
         ++*launches;
-        MF_TRY(cudaGetLastError());
         std::vector<int> got((size_t) n + nseg);
         MF_TRY(cudaMemcpyAsync(got.data(), lab, sizeof(int) * got.size(), cudaMemcpyDeviceToHost, s));
         MF_TRY(cudaStreamSynchronize(s));

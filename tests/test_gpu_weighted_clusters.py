@@ -89,3 +89,39 @@ def test_weights_beside_a_nan_are_summed_in_the_points_order(gpu, rng):
     labels, ncl = db.cluster_segments(x, np.array([0, x.size], np.int32), w)
     assert ncl[0] == core.sum()
     np.testing.assert_array_equal(np.asarray(labels)[place] >= 0, core[:, None].repeat(m, 1))
+
+
+# more segments than the chip holds large CTAs: small CTAs, by the largest
+# segment (their limits are 256 and 1,024 points), empty segments and segments
+# of one point among them; few points beside one large segment
+@pytest.mark.parametrize("largest,few", [(3, False), (256, False), (257, False), (1024, False), (1025, False), (1025, True)])
+@pytest.mark.parametrize("weighted", [False, True])
+def test_many_segments(gpu, rng, largest, few, weighted):
+    sizes = rng.integers(0, 3 if few else min(largest, 40) + 1, 400)
+    sizes[[7, 123, 399]] = largest, 0, 1
+    off = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int32)
+    x = np.concatenate([np.round(rng.uniform(0, 0.5 * m, m) * 8) / 8 for m in sizes])
+    x[::97], x[1::89], x[2::83] = np.nan, np.inf, -0.0
+    w = rng.integers(1, 12, x.size) / 10.0 if weighted else None
+    for eps, mo in ((0.25, 1), (1.0, 3)):
+        (l1, n1), (l2, n2) = _both(gpu, eps, mo, x, off, w)
+        np.testing.assert_array_equal(n1, n2)
+        np.testing.assert_array_equal(l1, l2)
+
+
+def test_many_small_segments_take_no_longer_than_the_general_form(gpu, rng):
+    """100,000 segments of two points, in one call and beside a segment that
+    sends them all to the general launches."""
+    db = gpu.DBSCAN()
+    db.initialize(50.0, 3)
+    nseg = 100_000
+    x, off = np.round(rng.uniform(0, 500, 2 * nseg)), (2 * np.arange(nseg + 1)).astype(np.int32)
+    xg, og = np.concatenate([x, np.zeros(BIG)]), np.concatenate([off, [2 * nseg + BIG]]).astype(np.int32)
+    best = {}
+    for name, a, o in (("small", x, off), ("general", xg, og)):
+        best[name] = 1e9
+        for _ in range(6):
+            t = time.perf_counter()
+            db.cluster_segments(a, o, None)
+            best[name] = min(best[name], time.perf_counter() - t)
+    assert best["small"] < best["general"], best
