@@ -516,7 +516,7 @@ static __global__ void __launch_bounds__(NT) db1_segment_kernel(const double *X,
     __shared__ int sh[33];
     unsigned long long *key = reinterpret_cast<unsigned long long *>(smem_db);
     double *xs = reinterpret_cast<double *>(smem_db);  // the sorted values, over the keys
-    int *run = reinterpret_cast<int *>(key + n2max);   // run of each position (-1: not core)
+    int *run = reinterpret_cast<int *>(key + n2max);   // run of each position; not core: -2 - the core position before (-1: none)
     int *aux = run + n2max;                            // per run, then per point
     int *idx = aux + n2max;                            // point of each position
     double *ps = reinterpret_cast<double *>(run);      // prefix sums of the weights, over run and aux
@@ -664,12 +664,16 @@ static __global__ void __launch_bounds__(NT) db1_segment_kernel(const double *X,
     int id = db1_scan<false, NT>(starts, sh, &nrun) - 1;  // the run the piece begins in
     prev = prev0;
     for (int r = r0; r < r1; ++r)
+    {
         if (run[r] == 0)
         {
             if (prev < 0 || !(xs[r] - xs[prev] <= eps)) ++id;
             prev = r;
             run[r] = id;
         }
+        else
+            run[r] = -2 - prev;
+    }
     for (int i = tid; i < nrun; i += NT) aux[i] = n;
     __syncthreads();
     for (int r = tid; r < nv; r += NT)
@@ -710,20 +714,29 @@ static __global__ void __launch_bounds__(NT) db1_segment_kernel(const double *X,
     for (int u = 0; u < kDb1Per; ++u)
         if (root[u] >= 0) aux[tid + u * NT] = num[u];
     __syncthreads();
-    // ---- labels: a core point's run; else the lowest cluster among the core neighbours
+    // ---- labels: a core point's run; else the lowest cluster among the core
+    // neighbours.  Those before it lie within eps of each other, so they are of
+    // the nearest one's run, and so are those after it
     for (int r = tid; r < n; r += NT)
     {
         int lab = -1;
         if (r < nv)
         {
             if (run[r] >= 0) lab = aux[run[r]];
-            else
+            else if (nrun > 0)
             {
                 int lo, hi;
                 db1_range(xs, 0, nv, xs[r], eps, lo, hi);
-                int best = n;
-                for (int i = nrun > 0 ? lo : hi; i < hi; ++i)
-                    if (run[i] >= 0) best = min(best, aux[run[i]]);
+                const int p = -2 - run[r];
+                int best = p >= lo ? aux[run[p]] : n;
+                int q = r + 1;  // the first core position after r
+                for (int e = hi; q < e;)
+                {
+                    const int m = (q + e) >> 1, v = run[m];
+                    if ((v >= 0 ? m : -2 - v) > p) e = m;
+                    else q = m + 1;
+                }
+                if (q < hi) best = min(best, aux[run[q]]);
                 if (best < n) lab = best;
             }
         }

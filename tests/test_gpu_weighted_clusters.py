@@ -125,3 +125,22 @@ def test_many_small_segments_take_no_longer_than_the_general_form(gpu, rng):
             db.cluster_segments(a, o, None)
             best[name] = min(best[name], time.perf_counter() - t)
     assert best["small"] < best["general"], best
+
+
+# many points that are not core, with core neighbours of one or two clusters far
+# from them in order
+@pytest.mark.parametrize("weighted", [False, True])
+def test_border_points(gpu, oracle, rng, weighted):
+    n = 3000
+    x = np.concatenate([rng.uniform(0, 4000, n - 40), rng.uniform(4600, 4700, 20), rng.uniform(5200, 5300, 20)]).round()
+    x = x[rng.permutation(n)]
+    w = rng.integers(1, 5, n) / 2.0 if weighted else None
+    db = gpu.DBSCAN()
+    for eps, share in ((1000.0, 0.45), (1000.0, 0.3), (700.0, 0.3), (50.0, 0.0245)):
+        mo = int(share * n * (1.25 if weighted else 1.0))
+        db.initialize(eps, mo)
+        labels, ncl = db.cluster_segments(x, np.array([0, n], np.int32), w)
+        n_ref, ref = oracle.dbscan(x, eps, mo, w)
+        assert ncl[0] == n_ref
+        np.testing.assert_array_equal(np.asarray(labels), ref)
+    assert n_ref > 1
