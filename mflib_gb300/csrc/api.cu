@@ -503,6 +503,22 @@ catch (...)
     return mfgpu::status_of_exception();
 }
 
+// whether every template's samples are finite, and sums of them
+static bool sums_are_finite(const std::vector<double> &x, const std::vector<long> &off, const std::vector<int> &len)
+{
+    for (size_t t = 0; t < len.size(); ++t)
+    {
+        double s[4] = {0, 0, 0, 0};
+        const double *b = x.data() + off[t];
+        int i = 0;
+        for (; i + 4 <= len[t]; i += 4)
+            for (int k = 0; k < 4; ++k) s[k] += std::fabs(b[i + k]);
+        for (; i < len[t]; ++i) s[0] += std::fabs(b[i]);
+        if (!std::isfinite((s[0] + s[1]) + (s[2] + s[3]))) return false;
+    }
+    return true;
+}
+
 // twiddles and resident template spectra of one plan (every template's
 // spectrum at the plan's FFT length; the plan reads its bucket's rows)
 template <class T>
@@ -813,8 +829,11 @@ try
     // lengths in buckets of its own lags per block costs the transforms less.
     // A (template, block) takes 76 ns against 302 for the FP64 transforms (160
     // templates of 200 .. 2,000 samples, 8 channels x 360,000), so that takes
-    // a few templates much longer than the others.
-    mf->intx = mf->prec == 8 && ntf > 0 && v == 0 && p->fft_length == 0 && !bucket_forced && p->length_buckets <= 1;
+    // a few templates much longer than the others.  A template holding an
+    // infinity or NaN (or whose mean overflows) has no integers: the transforms
+    // give NaN for it.
+    mf->intx = mf->prec == 8 && ntf > 0 && v == 0 && p->fft_length == 0 && !bucket_forced && p->length_buckets <= 1 &&
+               sums_are_finite(mf->tmpl, mf->toff, mf->lens);
     const int int_S = ((kIntN - maxLen + 1) / 32) * 32;
     if (!all_equal && p->fft_length == 0 && (forced_mode <= 1 || forced_mode == 4) && maxb > 1)
     {
