@@ -44,11 +44,13 @@ struct IntBankParams
 };
 
 // A block's integers: v = (f - level) 2^-sh, f the sample in units of 2^(emax -
-// 1084); emax -1: the block holds an infinity or NaN
+// 1084).  bad: the block holds an infinity or NaN, which count as f = 0 (the
+// windows that hold one are marked in the normalisation)
 struct IntUnit
 {
     long long level;
     int emax, sh;
+    int bad;
 };
 
 struct IntDenParams

@@ -288,21 +288,20 @@ __device__ __forceinline__ int int_unit_exponent(const IntUnit &u) { return u.em
 
 // Quantises a block's samples, sample 8 tid + i in v[i]: the finest unit at which
 // the 2-norm of every window of at most L samples stays below 2^kIntNormBits, at
-// most 55 bits.  An infinity or NaN counts as 0 and sets emax to -1 (the others
-// keep their integers).  lred: 64 words.
-__device__ __forceinline__ IntUnit int_quantise(long long (&v)[8], int *ired, long long *lred, int L, int *ex)
+// most 55 bits.  Infinities and NaN count as 0; nf: their bits.  lred: 64 words.
+__device__ __forceinline__ IntUnit int_quantise(long long (&v)[8], int *ired, long long *lred, int L, unsigned &nf)
 {
     constexpr int LOG2N = 12, NTH = kIntDenThreads;
     static_assert(kIntN == 1 << LOG2N, "the level is a sum shifted by log2 N");
     int em = 1;
-    bool nf = false;
+    nf = 0;
 #pragma unroll
     for (int i = 0; i < 8; ++i)
     {
         const int e = int_expo(v[i]);
         if (e == 2047)
         {
-            nf = true;
+            nf |= 1u << i;
             v[i] = 0;
         }
         else
@@ -311,9 +310,9 @@ __device__ __forceinline__ IntUnit int_quantise(long long (&v)[8], int *ired, lo
     const int emx = int_block_max<NTH>(em | (nf ? 1 << 12 : 0), ired);
     // (with a non-finite sample the largest exponent of the others is found
     // again: rare)
-    const bool bad = (emx >> 12) != 0;
     IntUnit u;
-    u.emax = bad ? int_block_max<NTH>(em, ired) : emx;
+    u.bad = emx >> 12;
+    u.emax = u.bad ? int_block_max<NTH>(em, ired) : emx;
     long long s = 0;
 #pragma unroll
     for (int i = 0; i < 8; ++i)
@@ -335,8 +334,6 @@ __device__ __forceinline__ IntUnit int_quantise(long long (&v)[8], int *ired, lo
     u.sh = max(max(0, nb - 55), (int) ceilf(0.5f * n2 - kIntNormBits));
 #pragma unroll
     for (int i = 0; i < 8; ++i) v[i] = int_sample(u, v[i]);
-    *ex = int_unit_exponent(u);
-    if (bad) u.emax = -1;
     return u;
 }
 
@@ -494,6 +491,7 @@ template <bool MULTI> __global__ void __launch_bounds__(kIntDenThreads, 2) int_d
     __shared__ __align__(16) long long lred[64];
     __shared__ unsigned long long ws[NW], wl[NW], wh[NW];  // sums up to and with each warp: x, x^2 (low, high)
     __shared__ int ired[32];
+    __shared__ __align__(4) unsigned char bad_bytes[NTH];  // a bit per sample that is an infinity or NaN
     unsigned long long *P1 = reinterpret_cast<unsigned long long *>(smem_id), *PL = P1 + NP, *PH = PL + NP;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, g = blockIdx.y;
     const int c = MULTI ? p.grp_chan[g] : g;
@@ -513,8 +511,10 @@ template <bool MULTI> __global__ void __launch_bounds__(kIntDenThreads, 2) int_d
         v[i] = d.x;
         v[i + 1] = k + 1 < p.n ? d.y : first;
     }
-    int ex;
-    const IntUnit unit = int_quantise(v, ired, lred, p.Lmax, &ex);
+    unsigned nf;
+    const IntUnit unit = int_quantise(v, ired, lred, p.Lmax, nf);
+    const int ex = int_unit_exponent(unit);
+    if (unit.bad) bad_bytes[tid] = (unsigned char) nf;
     // (the groups of a channel write the same)
     if (tid == 0) p.unit[(long) c * gridDim.x + blockIdx.x] = unit;
     // ---- prefix sums: thread, warp, block
@@ -595,6 +595,20 @@ template <bool MULTI> __global__ void __launch_bounds__(kIntDenThreads, 2) int_d
             // 0 for a constant window, sqrt(L) / tol where the deviation is
             // at most tol, as DenOps<double>::out
             out[k0 + k] = V < vtol ? (V == 0 ? 0.0 : sqrtL / p.tol) : int_inv_den(V, ex, sqrtL);
+        }
+        if (unit.bad)
+        {
+            // a window that holds an infinity or NaN has no coefficient (rare:
+            // each lag scans its window's words)
+            const unsigned *bits = reinterpret_cast<const unsigned *>(bad_bytes);
+            for (int k = tid; k < n; k += NTH)
+            {
+                const int a = k >> 5, b = (k + L - 1) >> 5;
+                unsigned any = 0;
+                for (int j = a; j <= b; ++j)
+                    any |= bits[j] & (j == a ? ~0u << (k & 31) : ~0u) & (j == b ? ~0u >> (31 - ((k + L - 1) & 31)) : ~0u);
+                if (any) out[k0 + k] = __longlong_as_double(0x7ff8000000000000ll);
+            }
         }
     };
     if constexpr (MULTI)
@@ -730,19 +744,6 @@ template <bool SHARED_DEN> __global__ void __launch_bounds__(kIntThreads, 1) int
     __syncthreads();
     const IntUnit unit = p.unit[(long) c * gridDim.x + bx];
     if (!xcorr_wait(bar, 0, x.err, x.test_skip_copy ? (1u << 12) : (1u << 24))) return;
-    if (unit.emax < 0)
-    {
-        // an infinity or NaN reaches every lag of an FP64 transform's block
-        for (int ti = t_begin; ti < t_end; ++ti)
-        {
-            const int t = x.tids[ti];
-            const long nv = x.nvalid[t];
-            double *dst = x.rho + (long) t * x.ldr;
-            for (int k = tid; k < S; k += kIntThreads)
-                if (k0 + k < nv) dst[k0 + k] = __longlong_as_double(0x7ff8000000000000ll);
-        }
-        return;
-    }
     const int ex = int_unit_exponent(unit);
     {
         // samples in the first half of the exchange buffers, integers to the
@@ -756,7 +757,9 @@ template <bool SHARED_DEN> __global__ void __launch_bounds__(kIntThreads, 1) int
             // past the data: the block's first sample instead of the zero
             // tail, which would set the scale of a signal with an offset
             const int j = tid + kIntThreads * i;
-            xq[(kIntN - j) & (kIntN - 1)] = int_sample(unit, int_fixed(seg[k0 + j < p.n ? j : 0], unit.emax));
+            long long b = seg[k0 + j < p.n ? j : 0];
+            if (unit.bad && int_expo(b) == 2047) b = 0;
+            xq[(kIntN - j) & (kIntN - 1)] = int_sample(unit, int_fixed(b, unit.emax));
         }
         __syncthreads();
     }
