@@ -786,7 +786,8 @@ def run_uneven_day(args, ctx):
                and not fp64)
     roof = {"bound": "hbm", "achieved": alg / (x_ms * 1e-3) / 1e9, "peak": peak, "unit": "GB/s",
             "frac": alg / (x_ms * 1e-3) / 1e9 / peak, "traffic": traffic if default else None,
-            "kernel": "xcorr_kernel<%s,%d,per-template normalisation>" % ("double" if fp64 else "float", P),
+            "kernel": "int_xcorr_kernel" if plan["correlator"] == 7 else
+                      "xcorr_kernel<%s,%d,per-template normalisation>" % ("double" if fp64 else "float", P),
             "kernel_ms": x_ms,
             "algorithmic_bytes": alg, "peak_source": kind}
     line = {"metric": METRIC, "value": ctx.world * lags / (el / args.steps), "unit": METRIC, "n_gpus": ctx.world,

@@ -417,8 +417,8 @@ static __global__ void db_count_kernel(int nseg, const int *seg_off, const long 
 // segments; now 106 us in all).  A segment's size is limited by the sort in
 // shared memory (20 bytes for each of a power of two of points: 164 KB); up to
 // there this form was the faster one wherever it was measured (one segment,
-// spread or in one neighbourhood, with and without weights: 1,024 points 65 ..
-// 117 us against 109 .. 134, 8,192 points 0.31 .. 0.49 ms against 0.53 .. 0.74).
+// spread or in one neighbourhood, with and without weights: 1,024 points 64 .. 87
+// us against 106 .. 137, 8,192 points 0.31 .. 0.46 ms against 0.53 .. 0.75).
 // Larger segments keep the launches above.
 //
 // A CTA of NT threads takes segments of up to 8 NT points: 1,024 threads, and
@@ -576,6 +576,11 @@ static __global__ void __launch_bounds__(NT) db1_segment_kernel(const double *X,
     int nv;
     db1_scan<false, NT>(mine, sh, &nv);
     __syncthreads();
+    if (wt && nv < n)
+    {
+        if (tid == 0) n_clusters[s] = -1;  // weights beside a NaN: left to the full scans
+        return;
+    }
     // ---- core points
     if (!wt)
     {

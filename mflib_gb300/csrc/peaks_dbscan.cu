@@ -276,15 +276,12 @@ int run_dbscan(int n, int nf, const double *X, const double *w, double eps, int 
     }
     int most = 0;
     for (int sg = 0; sg < nseg; ++sg) most = std::max(most, seg_off_host[sg + 1] - seg_off_host[sg]);
-    // (weights in data holding a NaN are summed in the points' order by the full
-    // scans below, whose rounding decides where a sum meets min_obs)
-    const bool points_order = nf == 1 && w && std::any_of(X, X + n, [](double v) { return std::isnan(v); });
     // threads per segment; segments of a few points beside one that needs the
     // large CTA are left to the general launches (39 ns each in such CTAs, 10 ns
     // per point there)
     const int nt1 = nseg <= kDb1Resident || most > kDb1Per * 128 ? 1024 : most > kDb1Per * 32 ? 128 : 32;
     const bool few = nt1 == 1024 && nseg > kDb1Resident && n < 4 * (long) nseg;
-    if (nf == 1 && most <= kDb1Cap && !points_order && !few)
+    if (nf == 1 && most <= kDb1Cap && !few)
     {
         // one CTA per segment: points (and weights) up, labels and counts down
         int n2 = 1;
@@ -311,9 +308,14 @@ int run_dbscan(int n, int nf, const double *X, const double *w, double eps, int 
         std::vector<int> got((size_t) n + nseg);
         MF_TRY(cudaMemcpyAsync(got.data(), lab, sizeof(int) * got.size(), cudaMemcpyDeviceToHost, s));
         MF_TRY(cudaStreamSynchronize(s));
-        std::copy(got.begin(), got.begin() + n, labels_host);
-        std::copy(got.begin() + n, got.end(), nclusters_host);
-        return 0;
+        // (weights in data holding a NaN are summed in the points' order by the
+        // full scans below, whose rounding decides where a sum meets min_obs)
+        if (*std::min_element(got.begin() + n, got.end()) >= 0)
+        {
+            std::copy(got.begin(), got.begin() + n, labels_host);
+            std::copy(got.begin() + n, got.end(), nclusters_host);
+            return 0;
+        }
     }
     MF_TRY(ws.X.ensure(sizeof(double) * (size_t) n * nf));
     MF_TRY(ws.w.ensure(sizeof(double) * (size_t) n));
