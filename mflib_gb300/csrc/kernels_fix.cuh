@@ -584,8 +584,14 @@ __global__ void __launch_bounds__(32 * kFixListWarps) fix_list_kernel(FixParams<
         const int L0 = __shfl_sync(0xffffffffu, myL, 0);
         const float *xc = p.x + (long) c * p.ldx;
         const long lag0 = 32L * r;
-        for (int i = tid; i < Lb + 64; i += 32 * kFixListWarps) ys[i] = i < Lb + 31 ? xc[lag0 + i] : 0.f;
-        const int np = (Lb + 31) / 32;
+        bool inf = false;  // a sample past the first window is an infinity or NaN
+        for (int i = tid; i < Lb + 64; i += 32 * kFixListWarps)
+        {
+            const float v = i < Lb + 31 ? xc[lag0 + i] : 0.f;
+            ys[i] = v;
+            inf |= i >= Lb && !isfinite(v);
+        }
+        int np = (Lb + 31) / 32;
         const float4 *co = reinterpret_cast<const float4 *>(p.bco + p.boff[B]);
         float4 *cw = reinterpret_cast<float4 *>(csh + (size_t) w * kFixBatch * 32);
         // coefficients of piece q: 128 float4, four per lane; zero past Lb
@@ -602,10 +608,30 @@ __global__ void __launch_bounds__(32 * kFixListWarps) fix_list_kernel(FixParams<
         for (int q = 0; q < kFixBatch / 2; ++q) acc[q] = f2_make(0.f, 0.f);
         float4 nx[4];
         if (w < np) fetch(w, nx);
-        __syncthreads();  // samples staged
+        inf = __syncthreads_or(inf);  // samples staged
         // each lag's own reference, a sample of its shortest window: a run
         // that straddles an amplitude step holds loud and quiet windows
         const float Rl = ys[lane + L0 / 2];
+        if (inf)
+        {
+            // a last piece that is not whole reaches past the windows with zero
+            // coefficients, which such a sample would make NaN: its samples one by
+            // one instead (no window reads its statistics)
+            if (w == 0)
+                for (int i = Lb & ~31; i < Lb; ++i)
+                {
+                    const ulonglong2 *cf = reinterpret_cast<const ulonglong2 *>(co + 4 * i);
+                    const f2 yy = f2_dup(ys[lane + i] - Rl);
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                    {
+                        const ulonglong2 cc = cf[u];
+                        acc[2 * u] = fma2(f2{cc.x}, yy, acc[2 * u]);
+                        acc[2 * u + 1] = fma2(f2{cc.y}, yy, acc[2 * u + 1]);
+                    }
+                }
+            np = Lb >> 5;
+        }
         for (int q = w; q < np; q += kFixListWarps)
         {
 #pragma unroll
@@ -619,12 +645,6 @@ __global__ void __launch_bounds__(32 * kFixListWarps) fix_list_kernel(FixParams<
                 v[i] = ys[lane + 32 * q + i] - Rl;
                 s += v[i];
             }
-            // past the longest window (its coefficients are zero) samples count
-            // as zero, also an infinity; such a piece is in no window's statistics
-            if (Lb < 32 * q + 32)
-#pragma unroll
-                for (int i = 1; i < 32; ++i)
-                    if (32 * q + i >= Lb) v[i] = 0.f;
             const float mu = s * (1.f / 32.f);
             float a = 0.f, b = 0.f;
 #pragma unroll
