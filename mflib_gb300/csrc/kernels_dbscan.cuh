@@ -516,7 +516,8 @@ static __global__ void __launch_bounds__(NT) db1_segment_kernel(const double *X,
     __shared__ int sh[33];
     unsigned long long *key = reinterpret_cast<unsigned long long *>(smem_db);
     double *xs = reinterpret_cast<double *>(smem_db);  // the sorted values, over the keys
-    int *run = reinterpret_cast<int *>(key + n2max);   // run of each position; not core: -2 - the core position before (-1: none)
+    // run of each position; not core: -2 - the core position before (-1: none)
+    int *run = reinterpret_cast<int *>(key + n2max);
     int *aux = run + n2max;                            // per run, then per point
     int *idx = aux + n2max;                            // point of each position
     double *ps = reinterpret_cast<double *>(run);      // prefix sums of the weights, over run and aux
